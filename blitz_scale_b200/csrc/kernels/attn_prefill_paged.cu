@@ -265,7 +265,7 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     if (!ok && lane == 0 && p.status) atomicCAS(p.status, 0, kStatusTimeoutProducer);
   } else if (warp == 8) {
     // ------------------------------------------------------------ MMA warp: one thread issues
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       auto issue_S = [&](int t, int stage) {
         const uint32_t a = ptx::smem_u32(sQ + t * TB), bb = ptx::smem_u32(sK + stage * TB);
 #pragma unroll

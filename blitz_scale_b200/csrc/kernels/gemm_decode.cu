@@ -55,6 +55,7 @@ struct DecGemmParams {
   int split;         // CTAs per tile = cluster size
   int kb_per_split;  // K blocks per CTA of a cluster
   int slice;         // tokens each cluster rank reduces and stores (multiple of 32: TMEM is read 32 columns at a time)
+  int slabs;         // the weights' columns come in whole slabs of 64, and tmap_w loads a tile of them at once
   int static_w;      // weights do not depend on earlier kernels of the stream
   float alpha;       // axpy; soft cap; limit of the clamped unit
   float beta;        // clamped unit (R: its biases)
@@ -207,11 +208,16 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       const uint32_t tx_bytes = static_cast<uint32_t>(p.x_box_rows) * kDecBK * 2 + kWBytes;
       auto load_w = [&](int stage, int tile, int kb) {
         uint8_t* sw = smem_w + stage * kWBytes;
         const int n0 = tile * kDecTile;
+        if (p.slabs) {  // (tmap_w: both slabs of the tile in one load)
+          ptx::tma_load_3d(sw, &tmap_w, &full_bar[stage], 0, kb * kDecBK, n0 >> 6);
+          if (epi_gated(EPI)) ptx::tma_load_3d(sw + 16384, &tmap_w, &full_bar[stage], 0, kb * kDecBK, (p.up_col_off + n0) >> 6);
+          return;
+        }
         ptx::tma_load_2d(sw, &tmap_w, &full_bar[stage], n0, kb * kDecBK);
         ptx::tma_load_2d(sw + 8192, &tmap_w, &full_bar[stage], n0 + 64, kb * kDecBK);
         if (epi_gated(EPI)) {
@@ -270,7 +276,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
   } else if (warp == 1) {
     // ------------------------------------------------------------ UMMA issuer
     ptx::griddep_wait();
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -580,7 +586,10 @@ int blitz_gemm_decode(const void* X, int64_t lda, const void* W, int64_t ldb, vo
   CUtensorMap tx, tw;
   if (!get_tmap_2d(&tx, X, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, kDecBK, (uint32_t)p.x_box_rows)) return -2;
   const int w_cols = epi_gated(epilogue) ? up_col_off + N : N;
-  if (!get_tmap_2d(&tw, W, (uint64_t)w_cols, (uint64_t)K, (uint64_t)ldb * 2, 64, kDecBK)) return -2;
+  p.slabs = w_cols % 64 == 0 && (!epi_gated(epilogue) || up_col_off % 64 == 0);
+  if (!(p.slabs ? get_tmap_slabs(&tw, W, (uint64_t)w_cols, (uint64_t)K, (uint64_t)ldb * 2, kDecBK, kDecTile / 64)
+                : get_tmap_2d(&tw, W, (uint64_t)w_cols, (uint64_t)K, (uint64_t)ldb * 2, 64, kDecBK)))
+    return -2;
 
   cudaError_t e;
   if (dtype == 1) {

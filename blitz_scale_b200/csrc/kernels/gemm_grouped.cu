@@ -36,6 +36,7 @@ struct GroupedTcParams {
   int box;         // rows per box of A: 32, or 128 where tiles are mostly full
   int src_rows;    // rows of A (bound of src)
   int sh_tiles, tn, tn_shared;
+  int slabs;       // the matrices' columns come in whole slabs of 64: one load per K block
   int* status;
 };
 
@@ -168,29 +169,36 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const uint32_t tx = static_cast<uint32_t>(pieces) * (gather ? 512u : p.box * 128u) + Cfg::kBBytes;
       const int row0 = FETCH == kGgGather4 ? it.t.row0 - p.g.shared_row0 : it.t.row0;  // of the boxes
       for (int kb = 0; kb < num_kb; ++kb) {
-        int good = 1;
-        if (lane == 0) {
-          good = ptx::bounded_mbar_wait(&empty_bar[g.stage], g.phase ^ 1u, abort_flag) ? 1 : 0;
-          if (good) ptx::mbar_expect_tx(&full_bar[g.stage], tx);
-          else if (p.status) atomicCAS(p.status, 0, kStatusTimeoutProducer);
+        // every lane waits (the warp stays converged), one lane issues what is one load; the rows' pieces of a gather come from as
+        // many lanes
+        ok = ptx::bounded_mbar_wait(&empty_bar[g.stage], g.phase ^ 1u, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+          if (p.status && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutProducer);
+          break;
         }
-        ok = __shfl_sync(0xffffffffu, good, 0) != 0;
-        if (!ok) break;
-        if (lane < BN / 64)  // slabs of 64 columns x 64 K rows
-          ptx::tma_load_2d(smem_b + g.stage * Cfg::kBBytes + lane * 8192, tb, &full_bar[g.stage], n0 + lane * 64, it.t.b_row + kb * kGgK);
-        if (lane < pieces) {
-          uint8_t* sa = smem_a + g.stage * a_stage;
-          if (gather)
-            ptx::tma_gather4(sa + lane * 512, ta, &full_bar[g.stage], kb * kGgK, idx[0], idx[1], idx[2], idx[3]);
-          else
-            ptx::tma_load_2d(sa + lane * (p.box * 128), ta, &full_bar[g.stage], kb * kGgK, row0 + lane * p.box);
+        uint8_t* sa = smem_a + g.stage * a_stage;
+        uint8_t* sb = smem_b + g.stage * Cfg::kBBytes;
+        if (ptx::elect_one()) {
+          ptx::mbar_expect_tx(&full_bar[g.stage], tx);
+          if (p.slabs) {
+            ptx::tma_load_3d(sb, tb, &full_bar[g.stage], 0, it.t.b_row + kb * kGgK, n0 >> 6);
+          } else {  // slabs of 64 columns x 64 K rows
+#pragma unroll
+            for (int s = 0; s < BN / 64; ++s) ptx::tma_load_2d(sb + s * 8192, tb, &full_bar[g.stage], n0 + s * 64, it.t.b_row + kb * kGgK);
+          }
+          if (!gather)
+            for (int s = 0; s < pieces; ++s) ptx::tma_load_2d(sa + s * (p.box * 128), ta, &full_bar[g.stage], kb * kGgK, row0 + s * p.box);
         }
+        __syncwarp();
+        if (gather && lane < pieces)
+          ptx::tma_gather4(sa + lane * 512, ta, &full_bar[g.stage], kb * kGgK, idx[0], idx[1], idx[2], idx[3]);
         g.next();
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ UMMA issuer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       Ring g{0, 0u, S};
       int acc = 0;
       uint32_t acc_phase = 0;
@@ -423,9 +431,13 @@ int blitz_gemm_grouped(const void* A, int64_t lda, int a_rows, const int* src, c
     tas = ta;
     if (B_shared && !get_tmap_2d(&tas, A, (uint64_t)K_shared, (uint64_t)a_rows, (uint64_t)lda * 2, kGgK, (uint32_t)p.box)) return -2;
   }
-  if (!get_tmap_2d(&tb, B, (uint64_t)N, (uint64_t)experts * K, (uint64_t)N * 2, 64, kGgK)) return -2;
+  p.slabs = N % 64 == 0 && (!B_shared || N_shared % 64 == 0);
+  auto weights = [&](CUtensorMap* m, const void* w, uint64_t cols, uint64_t rows) {
+    return p.slabs ? get_tmap_slabs(m, w, cols, rows, cols * 2, kGgK, (uint32_t)bn / 64) : get_tmap_2d(m, w, cols, rows, cols * 2, 64, kGgK);
+  };
+  if (!weights(&tb, B, (uint64_t)N, (uint64_t)experts * K)) return -2;
   tbs = tb;
-  if (B_shared && !get_tmap_2d(&tbs, B_shared, (uint64_t)N_shared, (uint64_t)K_shared, (uint64_t)N_shared * 2, 64, kGgK)) return -2;
+  if (B_shared && !weights(&tbs, B_shared, (uint64_t)N_shared, (uint64_t)K_shared)) return -2;
   const int64_t most = (int64_t)p.sh_tiles * p.tn_shared + (int64_t)max_tiles * p.tn;
   const int grid = (int)(most < sms ? most : sms);
   if (grid <= 0) return 0;

@@ -37,7 +37,7 @@
 #include "launch.cuh"
 #include "ptx.cuh"
 #include "tmap.cuh"
-#include "gemm_gate.cuh"
+#include "gemm_pair.cuh"
 #include <cstdlib>
 #include <type_traits>
 
@@ -68,6 +68,7 @@ struct PairParams {
   int upp;         // units (super tile x K block) per CTA pair
   int split;       // 0 = stream-K; 2..4 = every tile is cut into that many equal K parts, one pair each (nacc = 1)
   int total_units;
+  int slabs;       // W's columns come in whole slabs of 64, and tmap_b loads half a tile of them at once
   int static_b;    // W is not written by kernels still running in this stream
   float* ws;       // partials: [pair][cta rank][accumulator][bnf / 4][128 rows][4] fp32
   uint32_t* flags; // [tile][cta rank][4]: contributions landed (stream-K: word 0; split mode: one word per part); zero between launches
@@ -96,60 +97,6 @@ struct PairCfg {
   // accumulator buffers in TMEM: two sets (epilogue of one piece of work overlaps the UMMAs of the next) when they fit
   __host__ __device__ static int acc_bufs(int bnf, int nacc) { return 2 * nacc * bnf <= 512 ? 2 : 1; }
 };
-
-template <typename T>
-__device__ __forceinline__ uint32_t pair_pack2(float a, float b);
-template <>
-__device__ __forceinline__ uint32_t pair_pack2<__nv_bfloat16>(float a, float b) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-template <>
-__device__ __forceinline__ uint32_t pair_pack2<__half>(float a, float b) {
-  __half2 v = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-template <typename T>
-__device__ __forceinline__ float2 pair_unpack2(uint32_t u);
-template <>
-__device__ __forceinline__ float2 pair_unpack2<__nv_bfloat16>(uint32_t u) {
-  return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
-}
-template <>
-__device__ __forceinline__ float2 pair_unpack2<__half>(uint32_t u) {
-  return __half22float2(*reinterpret_cast<__half2*>(&u));
-}
-// fast-math sigmoid: the epilogue after the last UMMA is exposed time, and an IEEE division per element is a long
-// dependent chain on a handful of warps
-__device__ __forceinline__ float pair_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
-
-// 32 consecutive output columns of one row -> four 16-byte chunks.  EPI: 0 store, 1 add residual (its 32 values
-// come in `res`, read before the accumulator was waited for), 2 silu(g) * u.
-template <typename T, int EPI>
-__device__ __forceinline__ void pair_convert32(const float (&g)[32], const float (&u)[32], const uint4 (&res)[4],
-                                               uint4 (&out4)[4]) {
-  uint32_t out[16];
-  if (EPI == 2) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-      out[i] = pair_pack2<T>(pair_silu(g[2 * i]) * u[2 * i], pair_silu(g[2 * i + 1]) * u[2 * i + 1]);
-  } else if (EPI == 1) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t rr[4] = {res[j].x, res[j].y, res[j].z, res[j].w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 f = pair_unpack2<T>(rr[i]);
-        out[j * 4 + i] = pair_pack2<T>(g[j * 8 + 2 * i] + f.x, g[j * 8 + 2 * i + 1] + f.y);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) out[i] = pair_pack2<T>(g[2 * i], g[2 * i + 1]);
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) out4[j] = make_uint4(out[4 * j], out[4 * j + 1], out[4 * j + 2], out[4 * j + 3]);
-}
 
 template <typename T, int EPI>
 __global__ void __launch_bounds__(kPairThreads, 1)
@@ -220,7 +167,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs, own halves)
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       const uint32_t full0 = ptx::mapa_shared(ptx::smem_u32(full_bar), 0u);  // the even CTA's full barriers
       const uint32_t tx_bytes = 2u * static_cast<uint32_t>(stage_bytes);
       auto load_b = [&](int stage, int st, int kb) {
@@ -231,6 +178,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           int col;
           if (epi_gated(EPI)) col = (rank == 0 ? 0 : p.up_col_off) + nt * half;
           else col = nt * bnf + static_cast<int>(rank) * half;
+          if (p.slabs) {  // (tmap_b: all slabs of the half in one load)
+            ptx::tma_load_3d_pair(sb, &tmap_b, full0 + 8u * stage, 0, kb * kPairBK, col >> 6);
+            continue;
+          }
           for (int s = 0; s < half / 64; ++s)
             ptx::tma_load_2d_pair(sb + s * 8192, &tmap_b, full0 + 8u * stage, col + s * 64, kb * kPairBK);
         }
@@ -287,7 +238,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   } else if (warp == 1) {
     // ------------------------------------------------------------ UMMA issuer (even CTA only)
     ptx::griddep_wait();
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int buf = 0;
@@ -847,7 +798,10 @@ int blitz_gemm_pair(const void* A, int64_t lda, const void* W, int64_t ldb, void
   CUtensorMap ta, tb, tc;
   if (!get_tmap_2d(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, kPairBK, kPairRows)) return -2;
   const int w_cols = epi_gated(epilogue) ? up_col_off + N : N;
-  if (!get_tmap_2d(&tb, W, (uint64_t)w_cols, (uint64_t)K, (uint64_t)ldb * 2, 64, kPairBK)) return -2;
+  p.slabs = w_cols % 64 == 0 && (!epi_gated(epilogue) || up_col_off % 64 == 0);
+  if (!(p.slabs ? get_tmap_slabs(&tb, W, (uint64_t)w_cols, (uint64_t)K, (uint64_t)ldb * 2, kPairBK, (uint32_t)bnf / 128)
+                : get_tmap_2d(&tb, W, (uint64_t)w_cols, (uint64_t)K, (uint64_t)ldb * 2, 64, kPairBK)))
+    return -2;
   if (epi_f32(epilogue)) {
     tc = ta;  // fp32 outputs are stored without TMA; the map is not used
   } else if (!get_tmap_2d(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc * 2, 64, 32)) {

@@ -126,6 +126,13 @@ inline bool get_tmap_3d(CUtensorMap* out, const void* ptr, uint64_t d0, uint64_t
   return true;
 }
 
+// A "k rows of n columns" matrix as slabs of 64 columns (x, row, slab), so that one load fetches `slabs` of them one behind the
+// other, 64 x `rows` each: the layout of an N-major UMMA operand.  For columns in whole slabs.
+inline bool get_tmap_slabs(CUtensorMap* out, const void* ptr, uint64_t cols, uint64_t rows_total, uint64_t ld_bytes, uint32_t rows,
+                           uint32_t slabs) {
+  return get_tmap_3d(out, ptr, 64, rows_total, cols / 64, ld_bytes, 128, 64, rows, slabs);
+}
+
 // Number of SMs of the calling thread's current device (cached per device).
 inline int device_sm_count() {
   static std::atomic<int> cache[64];
