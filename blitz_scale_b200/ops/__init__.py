@@ -162,7 +162,7 @@ def _tensor_core_operands(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, N
 def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *, residual=None,
          epilogue: str = "store", alpha: float = 1.0, beta: float = 1.0, bias: Optional[torch.Tensor] = None, groups: int = 1, a_step: int = 0, out_step: int = 0, b_layout: str = "kn", bn: int = 0, split_k: int = 0, static_b: bool = False,
          decode_path: Optional[bool] = None, decode_split: int = 0, pair_path: Optional[bool] = None,
-         pair_bnf: int = 0, pair_upp: int = 0, pair_nacc: int = 0) -> torch.Tensor:
+         pair_bnf: int = 0, pair_upp: int = 0, pair_nacc: int = 0, wide_path: Optional[bool] = None) -> torch.Tensor:
     """``out = a @ b`` on tcgen05 with a fused epilogue.
 
     a: [M, K].  b: [K, N] when ``b_layout == 'kn'`` (weights stored in,out) or [N, K] for ``'nk'``.
@@ -179,6 +179,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     129..256 rows with 'kn' weights go to the paired-SM kernel (two CTAs issue one 256-row
     ``tcgen05.mma.cta_group::2``, stream-K over CTA pairs); ``pair_path`` forces (True) or forbids (False) it for
     any M, ``pair_bnf`` / ``pair_nacc`` / ``pair_upp`` override its tile width, tiles per pair and units per pair.
+
+    More rows with 'kn' weights go to the kernel whose CTA pairs walk 256 x 256 tiles; ``wide_path`` forces (True) or forbids
+    (False) it for any M.
 
     ``out`` may be fp32 with 16-bit operands (the accumulator is stored unrounded); epilogue 'axpy' adds
     ``alpha * (a @ b)`` to an fp32 ``out`` (residual streams kept in 32 bits); 'softcap' stores
@@ -240,6 +243,18 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     if pair_path is not None:
         assert not pair_path or pair_ok
         use_pair = pair_path
+    # fewer 128 x 128 tiles than half the SMs: cutting K over them (gemm_tcgen05.cu) is faster, and its sums are shorter
+    use_wide = M > PAIR_GEMM_MAX_M and bn == 0 and split_k == 0 and -(-M // 128) * -(-N // (64 if gated else 128)) * groups > 74 and \
+        bool(lib().blitz_gemm_wide_supported(M, N, K, 0 if b_layout == "kn" else 1, epi, groups))
+    if wide_path is not None:
+        assert not wide_path or lib().blitz_gemm_wide_supported(M, N, K, 0 if b_layout == "kn" else 1, epi, groups)
+        use_wide = wide_path
+    if use_wide:
+        rc = lib().blitz_gemm_wide(_p(a), a.stride(0), _p(b), b.stride(0), _p(out), out.stride(0), _p(extra), M, N, K, epi,
+                                   N if gated else 0, _dt(a), int(static_b), 0, 0, _p(status_word(a.device)), alpha, beta,
+                                   groups, a_step, out_step, _stream())
+        _check(rc, "blitz_gemm_wide")
+        return out
     if use_pair:
         pws, pflags = pair_gemm_workspace(a.device)
         rc = lib().blitz_gemm_pair(_p(a), a.stride(0), _p(b), b.stride(0), _p(out), out.stride(0), _p(extra), M, N,

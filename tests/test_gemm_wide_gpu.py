@@ -1,0 +1,55 @@
+"""The products of many rows (CTA pairs, 256 x 256 tiles) at the edges of their tiles against fp32 products of the same operands."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+# rows, columns, depth: below and behind a tile's edge, one K block and less, last rounds of halved and of whole tiles, columns that do
+# not come in slabs of 64
+SIZES = [(1, 64, 8), (257, 64, 64), (300, 136, 72), (512, 512, 512), (777, 1000, 1032), (1574, 6144, 256), (256, 14336, 256), (4999, 1032, 136)]
+
+
+@pytest.mark.parametrize("M,N,K", SIZES)
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_epilogues(M, N, K, dt):
+    from blitz_scale_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).to(dt)
+    a, w, r = rnd(M, K + 8)[:, :K], (rnd(K, N).float() * K ** -0.5).to(dt), rnd(M, N)
+    ref = a.float() @ w.float()
+    unit = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+
+    def near(got, want, rel):    # one rounding of the result, and 32-bit sums in another order
+        assert float(((got.float() - want).abs() - rel * want.abs()).max()) <= 2e-5 * K ** 0.5
+    run = lambda out, **kw: ops.gemm(a, w, out=out, wide_path=True, **kw)
+    near(run(torch.full((M, N), 7.0, dtype=dt, device=DEV)), ref, unit)
+    both = r.clone()
+    near(run(both, residual=both, epilogue="add"), ref + r.float(), unit)
+    near(run(torch.zeros(M, N, device=DEV)), ref, 1e-5)
+    near(run(torch.ones(M, N, device=DEV), epilogue="axpy", alpha=0.5), 1 + 0.5 * ref, 1e-5)
+    near(run(torch.zeros(M, N, device=DEV), epilogue="softcap", alpha=2.0), 2 * torch.tanh(ref / 2), 1e-5)
+    if N % 16 == 0 and N >= 128:
+        gate, up = ref[:, :N // 2], ref[:, N // 2:]
+        near(run(None, epilogue="silu_mul"), torch.nn.functional.silu(gate) * up, 2 * unit)
+        bias = rnd(N)
+        gb, ub = (gate + bias[:N // 2].float()).clamp(max=1.5), (up + bias[N // 2:].float()).clamp(-1.5, 1.5)
+        near(run(None, epilogue="clamp_glu", alpha=1.5, beta=1.7, bias=bias), gb * torch.sigmoid(1.7 * gb) * (ub + 1), 2 * unit)
+    ops.check_status()
+
+
+@pytest.mark.parametrize("M", [257, 700])
+@pytest.mark.parametrize("f32", [False, True])
+def test_diagonal_blocks(M, f32):
+    from blitz_scale_b200 import ops
+    G, K, N = 4, 192, 320
+    a = torch.randn(M, G * (K + 8), device=DEV).to(torch.bfloat16)
+    w = (torch.randn(G * K, N, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    out = torch.full((M, G * (N + 16)), 7.0, dtype=torch.float32 if f32 else torch.bfloat16, device=DEV)
+    ops.gemm(a, w, out=out, groups=G, a_step=K + 8, out_step=N + 16, wide_path=True)
+    ops.check_status()
+    for i in range(G):
+        want = a[:, i * (K + 8):i * (K + 8) + K].float() @ w[i * K:(i + 1) * K].float()
+        got = out[:, i * (N + 16):(i + 1) * (N + 16)]
+        assert float(((got[:, :N].float() - want).abs() - (1e-5 if f32 else 2.0 ** -8) * want.abs()).max()) <= 2e-5 * K ** 0.5
+        assert bool((got[:, N:] == 7.0).all())
