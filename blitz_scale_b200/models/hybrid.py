@@ -96,7 +96,7 @@ class HybridRunner:
                 self._freqs[self._rot_key(m)] = ops.rope_freqs(m.rot_dims, m.rot_base, dev, stretch)
             elif m.kind == "latent":
                 self._freqs[(m.rot_dim, m.rot_base, None)] = ops.rope_freqs(m.rot_dim, m.rot_base, dev)
-        self._ws: Optional[torch.Tensor] = None
+        self._ws: Dict[bool, torch.Tensor] = {}
         self._ws_old: List[Optional[torch.Tensor]] = []
 
     @staticmethod
@@ -335,20 +335,22 @@ class HybridRunner:
         ns = m.singles if m.is_prefill else m.batch
         if ns:
             ops.attn_decode(p["q"][:ns], kv, m.page_indices, m.page_indptr[:ns + 1], m.last_page_len[:ns],
-                            num_splits=m.num_splits, workspace=self._workspace(ns, mx, m.num_splits), out=mid[:ns],
+                            num_splits=m.num_splits, workspace=self._workspace(ns, mx, m.num_splits), out=mid[:ns], static_table=True,
                             gate=gate[:ns] if gate is not None else None, **args)
         if m.batch > ns:
             ops.attn_prefill_paged(p["q"], kv, m.page_indices, m.prefill_work, out=mid, gate=gate, **args)
 
     def _workspace(self, B: int, mx: AttentionMixer, splits: int) -> Optional[torch.Tensor]:
-        if splits <= 1:
+        if splits == 1:
             return None
         n = ops.attn_decode_workspace_bytes(B, mx.heads, mx.vdim, splits)
-        if self._ws is None or self._ws.numel() < n:
+        key = splits == 0               # shares of all keys: the kernel's tickets in it stay zero
+        ws = self._ws.get(key)
+        if ws is None or ws.numel() < n:
             # an earlier buffer may be named by captured graphs: keep it
-            self._ws_old.append(self._ws)
-            self._ws = torch.empty(n, dtype=torch.uint8, device=self.res.device)
-        return self._ws
+            self._ws_old.append(ws)
+            ws = self._ws[key] = torch.zeros(n, dtype=torch.uint8, device=self.res.device)
+        return ws
 
     def _latent(self, r: int, l: int, mx: LatentAttentionMixer, p: Dict[str, torch.Tensor], mid: torch.Tensor, m: StepMeta) -> None:
         T, H, R, W, kv = m.num_tokens, mx.heads, mx.kv_rank, mx.width, self.cache.runs[r].kv

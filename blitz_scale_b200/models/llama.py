@@ -110,13 +110,14 @@ class LlamaRunner:
             self.comm.all_reduce_(self.res[:T])
 
     def _workspace(self, B: int, splits: int) -> Optional[torch.Tensor]:
-        if splits <= 1:
+        if splits == 1:
             return None
         n = ops.attn_decode_workspace_bytes(B, self.qh, self.hd, splits)
-        ws = self._ws.get("dec")
+        key = splits == 0               # shares of all keys: the kernel's tickets in it stay zero
+        ws = self._ws.get(key)
         if ws is None or ws.numel() < n:
-            ws = torch.empty(n, dtype=torch.uint8, device=self.res.device)
-            self._ws["dec"] = ws
+            ws = torch.zeros(n, dtype=torch.uint8, device=self.res.device)
+            self._ws[key] = ws
         return ws
 
     def attention_block(self, l: int, m: StepMeta) -> None:
@@ -130,7 +131,7 @@ class LlamaRunner:
         else:
             ops.attn_decode(self.qkv[:T], self.kv[l], m.page_indices, m.page_indptr, m.last_page_len,
                             q_heads=self.qh, kv_heads=self.kvh, head_dim=self.hd, page_size=self.page_size,
-                            num_splits=m.num_splits, workspace=self._workspace(m.batch, m.num_splits),
+                            num_splits=m.num_splits, workspace=self._workspace(m.batch, m.num_splits), static_table=True,
                             out=self.attn[:T])
         if self.tp == 1:
             ops.gemm(self.attn[:T], self._w(l, "o"), static_b=True, out=self.res[:T], residual=self.res[:T], epilogue="add")

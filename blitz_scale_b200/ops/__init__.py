@@ -366,6 +366,9 @@ def rope_kv_store(qkv: torch.Tensor, pos: torch.Tensor, slot: torch.Tensor, kv_l
 
 
 # ---------------------------------------------------------------------------------------------- attention
+ATTN_DECODE_SHARED_ROWS = 256
+
+
 def attn_decode_workspace_bytes(batch: int, q_heads: int, value_dim: int, num_splits: int) -> int:
     return int(lib().blitz_attn_decode_workspace_bytes(batch, q_heads, value_dim, num_splits))
 
@@ -375,26 +378,30 @@ def attn_decode(q: torch.Tensor, kv_layer: KVLayer, indices: torch.Tensor, indpt
                 num_splits: int = 1, workspace: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
                 sm_scale: Optional[float] = None, window: int = 0, keep_first: int = 0, softcap: float = 0.0,
                 sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
-                bias: Optional[torch.Tensor] = None, chunked: bool = False, sigmoid: bool = False) -> torch.Tensor:
-    """q: [batch, >= q_heads*head_dim] (row pitch free, e.g. a view of the fused qkv buffer).  ``window`` > 0: only the
+                bias: Optional[torch.Tensor] = None, chunked: bool = False, sigmoid: bool = False, static_table: bool = False) -> torch.Tensor:
+    """q: [batch, >= q_heads*head_dim] (row pitch free, e.g. a view of the fused qkv buffer).  ``num_splits``: parts that every
+    sequence's keys are cut into; 0: equal shares of all sequences' keys, whatever their lengths (up to
+    `ATTN_DECODE_SHARED_ROWS` sequences); ``workspace`` has to be zero-filled before its first use then, and serves one call at a
+    time.  ``window`` > 0: only the
     last that many positions and the first ``keep_first`` are visible (and read); ``softcap`` > 0:
     scores are cap * tanh(score / cap); ``sink`` [q_heads]: a term e^sink in the softmax denominator; ``gate``
     [batch, q_heads]: a head's output is multiplied by its sigmoid; ``bias`` [q_heads, n]: added to the scaled scores by the
     key's distance, the last column for all longer ones.  ``chunked``: the window is a chunk counted from position 0, of which
-    the keys up to the position are visible; ``sigmoid``: the weights are sigmoids of the scores, not normalised.  Values may have a size of their own (KVPair)."""
+    the keys up to the position are visible; ``sigmoid``: the weights are sigmoids of the scores, not normalised.  Values may have a size of their own (KVPair).  ``static_table`` promises that ``indices``, ``indptr`` and
+    ``last_page_len`` are not written by kernels still running in this stream (the copy that brings a step's tables is no kernel)."""
     B = indptr.numel() - 1
     kp, vp, page_rows, pages, vdim = _kv(kv_layer)
     if out is None:
         out = torch.empty((B, q_heads * vdim), dtype=q.dtype, device=q.device)
-    if num_splits > 1 and workspace is None:
-        workspace = torch.empty(attn_decode_workspace_bytes(B, q_heads, vdim, num_splits), dtype=torch.uint8,
+    if num_splits != 1 and workspace is None:
+        workspace = torch.zeros(attn_decode_workspace_bytes(B, q_heads, vdim, num_splits), dtype=torch.uint8,
                                 device=q.device)
     if sm_scale is None:
         sm_scale = head_dim ** -0.5
     _check(lib().blitz_attn_decode(_p(q), q.stride(0), kp, vp, _p(indices), _p(indptr), _p(last_page_len),
                                    _p(out), out.stride(0), _p(workspace), B, q_heads, kv_heads, head_dim, vdim, page_size,
                                    page_rows, pages, num_splits, sm_scale, window, keep_first, int(chunked), int(sigmoid), softcap, _p(sink), *_bias(bias, q_heads), *_gate(gate),
-                                   _p(status_word(q.device)), _dt(q), _stream()), "blitz_attn_decode")
+                                   int(static_table), _p(status_word(q.device)), _dt(q), _stream()), "blitz_attn_decode")
     return out
 
 

@@ -134,13 +134,23 @@ class Engine:
             return None
         return b
 
-    def choose_splits(self, B: int, max_len: int) -> int:
+    def choose_splits(self, B: int, max_len: int, tokens: int = 0) -> int:
+        """How decode attention divides the keys of B sequences, the longest of max_len and `tokens` in all (0: not known).  0: equal
+        ranges of all of them, whatever the lengths.  Sequences of about one length need no ranges, whose pieces cost a fence, a ticket
+        and a merge inside the kernel: few of them are cut into as many parts as fill the SMs (16 x 1001 tokens, 8 KV heads: 15 us
+        instead of 20), many stay whole.  A batch has no more than two choices, so that it needs no more than two graphs."""
         if self.cfg.family == "hybrid":
             kv_heads, max_len = self.cfg.attention_work(max_len)
             if kv_heads == 0:
                 return 1
         else:
             kv_heads = self.cfg.kv_heads // self.tp
+        if B <= ops.ATTN_DECODE_SHARED_ROWS:
+            if 4 * B * max_len > 5 * tokens:
+                return 0
+            if B * kv_heads <= 148:
+                return 1 << min(4, (2 * 148 // (B * kv_heads)).bit_length() - 1)
+            return int(B * kv_heads >= 8 * 148)
         ctas = B * kv_heads
         if ctas >= 2 * 148 or max_len <= 256:
             return 1
@@ -229,7 +239,7 @@ class Engine:
             raise ValueError(f"decode batch of {B} sequences exceeds max_batch={self.max_batch}")
         Bp = _bucket(B) if self.use_graphs else B
         Bp = min(Bp, self.max_batch)
-        splits = self.choose_splits(Bp, batch.max_seq_len())
+        splits = self.choose_splits(Bp, batch.max_seq_len(), batch.num_pages() * self.page_size)
         P = batch.fill_decode(self.host_np, self.layout, Bp)
         self._h2d(self.layout.page_indices + P)
         if self.use_graphs:
@@ -290,7 +300,7 @@ class Engine:
         self._h2d(self.layout.page_indices + P)
         row_of = {b: r for r, b in enumerate(order)}
         if single:
-            splits = self.choose_splits(pad, max(kv_lens))
+            splits = self.choose_splits(pad, max(kv_lens), sum(kv_lens))
             if self.use_graphs:
                 (self._graphs.get((pad, splits)) or self._capture(pad, splits)).replay()
             else:
@@ -299,7 +309,7 @@ class Engine:
             if src:
                 got = self.runner.logits[torch.tensor([row_of[b] for b, _ in src], device=self.device)].float()
         else:
-            splits = self.choose_splits(singles, max(kv_lens[:singles])) if singles else 1
+            splits = self.choose_splits(singles, max(kv_lens[:singles]), sum(kv_lens[:singles])) if singles else 1
             m = self._views(T, rows, P, True, q_lens, splits=splits, kv_lens=kv_lens, singles=singles)
             with nvtx_range("step"):
                 self.runner.forward(m, with_head=False)
@@ -383,8 +393,8 @@ class Engine:
         for Bp in _BUCKETS:
             if Bp > limit:
                 break
-            for ctx in contexts:
-                splits = self.choose_splits(Bp, ctx)
+            for ctx, tokens in [(c, t) for c in contexts for t in (0, Bp * c)]:
+                splits = self.choose_splits(Bp, ctx, tokens)
                 if (Bp, splits) in self._graphs:
                     continue
                 P = empty.fill_decode(self.host_np, self.layout, Bp)      # Bp padded rows: no page, no cache write
