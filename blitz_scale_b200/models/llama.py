@@ -141,11 +141,19 @@ class LlamaRunner:
 
     def _prefill_attention(self, l: int, m: StepMeta) -> None:
         """The pass's rows against everything the cache holds for their sequences (rope_kv_store has just added the
-        rows' own keys and values): earlier chunks of a long prompt are simply a longer page list."""
-        T = m.num_tokens
+        rows' own keys and values): earlier chunks of a long prompt are simply a longer page list.  Leading rows of one token
+        (`m.singles`) are a decode batch: as tiles of 128 rows they would be padding (43 of them, 700 keys each, beside a portion
+        of 1531 tokens: 221 us with them among the tiles, 115 and 38 apart)."""
+        T, ns = m.num_tokens, m.singles
+        if ns:
+            ops.attn_decode(self.qkv[:ns], self.kv[l], m.page_indices, m.page_indptr[:ns + 1], m.last_page_len[:ns],
+                            q_heads=self.qh, kv_heads=self.kvh, head_dim=self.hd, page_size=self.page_size,
+                            num_splits=m.num_splits, workspace=self._workspace(ns, m.num_splits), static_table=True, out=self.attn[:ns])
+            if m.batch == ns:
+                return
         if m.prefill_work is None:      # a caller that built the step by hand
             m.prefill_work = ops.prefill_work_list(m.seq_lens_host, m.kv_lens_host or m.seq_lens_host, self.page_size,
-                                                   self.qkv.device)
+                                                   self.qkv.device, skip=ns)
         ops.attn_prefill_paged(self.qkv[:T], self.kv[l], m.page_indices, m.prefill_work, q_heads=self.qh,
                                kv_heads=self.kvh, head_dim=self.hd, page_size=self.page_size, out=self.attn[:T])
 

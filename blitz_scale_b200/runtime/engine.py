@@ -105,9 +105,8 @@ class Engine:
         L, d = self.layout, self.dev
         kv_lens = list(kv_lens) if kv_lens else list(seq_lens)
         if prefill and work is None:
-            # the hybrid runner takes the leading single tokens of a ragged step through its decode kernels
-            work = ops.prefill_work_list(seq_lens, kv_lens, self.page_size, self.device,
-                                         skip=singles if self.cfg.family == "hybrid" else 0)
+            # the leading single tokens of a ragged step go through the decode kernels
+            work = ops.prefill_work_list(seq_lens, kv_lens, self.page_size, self.device, skip=singles)
         return StepMeta(kv_lens_host=kv_lens, prefill_work=work,
                         ids=d[L.ids:L.ids + T], pos=d[L.pos:L.pos + T], slot=d[L.slot:L.slot + T],
                         page_indices=d[L.page_indices:L.page_indices + max(P, 1)],
