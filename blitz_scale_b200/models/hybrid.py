@@ -407,10 +407,15 @@ class HybridRunner:
         ps = self.page_size
         pages = [-(-kv_len // ps) for kv_len in m.kv_lens_host]
         first, total = sum(pages[:n]), sum(pages)
-        if not window:       # page i of the expanded pool is the i-th page of these sequences
-            return torch.arange(-first, total - first, dtype=torch.int32, device=dev), m.page_indices[first:total], total - first
         key = (n, window)
-        if self._expanded is None or self._expanded[0] is not m or key not in self._expanded[1]:
+        if self._expanded is not None and self._expanded[0] is m and key in self._expanded[1]:
+            return self._expanded[1][key]
+        if self._expanded is None or self._expanded[0] is not m:
+            self._expanded = (m, {})
+        if not window:       # page i of the expanded pool is the i-th page of these sequences
+            self._expanded[1][key] = (torch.arange(-first, total - first, dtype=torch.int32, device=dev), m.page_indices[first:total],
+                                      total - first)
+        else:
             index, need, at = [0] * first, [], first
             for s in range(n, len(pages)):
                 # (the attention kernel walks whole blocks of keys)
@@ -419,8 +424,6 @@ class HybridRunner:
                 need += range(at + lo, at + pages[s])
                 at += pages[s]
             both = torch.tensor(index + need, dtype=torch.int32).to(dev, non_blocking=True)
-            if self._expanded is None or self._expanded[0] is not m:
-                self._expanded = (m, {})
             self._expanded[1][key] = (both[:len(index)], m.page_indices.index_select(0, both[len(index):]), len(need))
         return self._expanded[1][key]
 

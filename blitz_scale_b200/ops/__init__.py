@@ -17,7 +17,9 @@ from ._lib import lib, available, KernelLibraryMissing  # noqa: F401
 
 _DT = {torch.float16: 0, torch.bfloat16: 1}
 _DT3 = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}
+_raw_stream, _raw_device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
 _status = {}
+_status_by_index = {}      # the same words by device number, for the launches
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -35,12 +37,12 @@ def _dt3(t: torch.Tensor) -> int:
         raise TypeError(f"kernel takes fp16/bf16/fp32 tensors, got {t.dtype}") from None
 
 
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    return _raw_stream(_raw_device())      # (torch.cuda.current_stream() makes a stream object first)
 
 
-def _p(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _p(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
 def _check(rc: int, what: str) -> None:
@@ -98,6 +100,15 @@ def status_word(device=None) -> torch.Tensor:
     return _status[key]
 
 
+def _status_ptr(t: torch.Tensor) -> int:
+    """Address of the status word of a tensor's device."""
+    index = t.get_device()
+    word = _status_by_index.get(index)
+    if word is None:
+        word = _status_by_index[index] = status_word(t.device)
+    return word.data_ptr()
+
+
 def check_status(device=None, reset: bool = True) -> int:
     """Read the status word (synchronises). Raises on a non-zero code."""
     w = status_word(device)
@@ -149,6 +160,26 @@ def pair_gemm_workspace(device=None):
         _pair_ws[key] = (torch.empty(n, dtype=torch.uint8, device=dev),
                          torch.zeros(PAIR_FLAGS, dtype=torch.int32, device=dev))
     return _pair_ws[key]
+
+
+class _GemmScratch(ctypes.Structure):
+    _fields_ = [("ws", ctypes.c_void_p), ("ws_bytes", ctypes.c_int64), ("tickets", ctypes.c_void_p), ("num_tickets", ctypes.c_int64),
+                ("pair_ws", ctypes.c_void_p), ("pair_bytes", ctypes.c_int64), ("pair_flags", ctypes.c_void_p),
+                ("num_pair_flags", ctypes.c_int64), ("status", ctypes.c_void_p)]
+
+
+_gemm_scratch = {}
+
+
+def _scratch_of(index: int) -> int:
+    """Address of the record of a device's product scratch (what blitz_gemm_any takes)."""
+    if index not in _gemm_scratch:
+        dev = torch.device("cuda", index)
+        (ws, tickets), (pair, flags) = gemm_workspace(dev), pair_gemm_workspace(dev)
+        record = _GemmScratch(ws.data_ptr(), ws.numel(), tickets.data_ptr(), tickets.numel(), pair.data_ptr(), pair.numel(), flags.data_ptr(),
+                              flags.numel(), status_word(dev).data_ptr())
+        _gemm_scratch[index] = (ctypes.addressof(record), record)
+    return _gemm_scratch[index][0]
 
 
 def _tensor_core_operands(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, N: int, K: int) -> bool:
@@ -230,28 +261,33 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     if epi == 1:
         assert residual is not None and residual.shape == (M, N) and residual.stride(0) == out.stride(0)
     extra = bias if epi == 7 else residual
-    ws, tickets = gemm_workspace(a.device)
-    # the decode kernel re-reads the activation tile with every weight tile, which the SM's load path cannot keep up
-    # with beyond ~128 rows; from there on the tiled kernel is faster
-    use_dec = groups == 1 and M <= DECODE_GEMM_MAX_M and bn == 0 and split_k == 0 and \
-        bool(lib().blitz_gemm_decode_supported(M, N, K, 0 if b_layout == "kn" else 1, epi))
+    if b_layout == "kn" and not (bn or split_k or decode_split or pair_bnf or pair_upp or pair_nacc) and \
+            decode_path is None and pair_path is None and wide_path is None:
+        rc = lib().blitz_gemm_any(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(), out.stride(0), _p(extra), M, N, K, epi,
+                                  N if gated else 0, _dt(a), int(static_b), _scratch_of(a.get_device()), alpha, beta, groups, a_step, out_step,
+                                  _stream())
+        _check(rc, "blitz_gemm")
+        return out
+    # the kernel that a hint asks for, or else the choice without hints
+    layout = 0 if b_layout == "kn" else 1
+    choice = lib().blitz_gemm_choice(M, N, K, epi, groups) if layout == 0 and bn == 0 and split_k == 0 else 0
+    use_dec, use_pair, use_wide = choice == 1, choice == 2, choice == 3
     if decode_path is not None:
-        assert not decode_path or lib().blitz_gemm_decode_supported(M, N, K, 0 if b_layout == "kn" else 1, epi)
+        assert not decode_path or lib().blitz_gemm_decode_supported(M, N, K, layout, epi)
         use_dec = decode_path
-    pair_ok = bool(lib().blitz_gemm_pair_supported(M, N, K, 0 if b_layout == "kn" else 1, epi))
-    use_pair = (groups == 1 and not use_dec and DECODE_GEMM_MAX_M < M <= PAIR_GEMM_MAX_M and bn == 0 and split_k == 0 and pair_ok)
     if pair_path is not None:
-        assert not pair_path or pair_ok
+        assert not pair_path or lib().blitz_gemm_pair_supported(M, N, K, layout, epi)
         use_pair = pair_path
-    # fewer 128 x 128 tiles than half the SMs: cutting K over them (gemm_tcgen05.cu) is faster, and its sums are shorter
-    use_wide = M > PAIR_GEMM_MAX_M and bn == 0 and split_k == 0 and -(-M // 128) * -(-N // (64 if gated else 128)) * groups > 74 and \
-        bool(lib().blitz_gemm_wide_supported(M, N, K, 0 if b_layout == "kn" else 1, epi, groups))
+    elif decode_path:
+        use_pair = False
     if wide_path is not None:
-        assert not wide_path or lib().blitz_gemm_wide_supported(M, N, K, 0 if b_layout == "kn" else 1, epi, groups)
+        assert not wide_path or lib().blitz_gemm_wide_supported(M, N, K, layout, epi, groups)
         use_wide = wide_path
+    elif decode_path or pair_path:
+        use_wide = False
     if use_wide:
         rc = lib().blitz_gemm_wide(_p(a), a.stride(0), _p(b), b.stride(0), _p(out), out.stride(0), _p(extra), M, N, K, epi,
-                                   N if gated else 0, _dt(a), int(static_b), 0, 0, _p(status_word(a.device)), alpha, beta,
+                                   N if gated else 0, _dt(a), int(static_b), 0, 0, _status_ptr(a), alpha, beta,
                                    groups, a_step, out_step, _stream())
         _check(rc, "blitz_gemm_wide")
         return out
@@ -259,19 +295,20 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
         pws, pflags = pair_gemm_workspace(a.device)
         rc = lib().blitz_gemm_pair(_p(a), a.stride(0), _p(b), b.stride(0), _p(out), out.stride(0), _p(extra), M, N,
                                    K, epi, N if gated else 0, _dt(a), int(static_b), pair_bnf, pair_nacc, pair_upp,
-                                   _p(pws), pws.numel(), _p(pflags), pflags.numel(), _p(status_word(a.device)),
+                                   _p(pws), pws.numel(), _p(pflags), pflags.numel(), _status_ptr(a),
                                    alpha, beta, _stream())
         _check(rc, "blitz_gemm_pair")
         return out
     if use_dec:
         rc = lib().blitz_gemm_decode(_p(a), a.stride(0), _p(b), b.stride(0), _p(out), out.stride(0), _p(extra), M, N,
                                      K, epi, N if gated else 0, _dt(a), int(static_b), decode_split,
-                                     _p(status_word(a.device)), alpha, beta, _stream())
+                                     _status_ptr(a), alpha, beta, _stream())
         _check(rc, "blitz_gemm_decode")
         return out
+    ws, tickets = gemm_workspace(a.device)
     rc = lib().blitz_gemm(_p(a), a.stride(0), _p(b), b.stride(0), _p(out), out.stride(0), _p(extra), M, N, K,
                           0 if b_layout == "kn" else 1, epi, N if gated else 0, _dt(a), bn, split_k,
-                          _p(ws), ws.numel(), _p(tickets), tickets.numel(), _p(status_word(a.device)), alpha, beta,
+                          _p(ws), ws.numel(), _p(tickets), tickets.numel(), _status_ptr(a), alpha, beta,
                           groups, a_step, out_step, _stream())
     _check(rc, "blitz_gemm")
     return out
@@ -361,7 +398,7 @@ def rope_kv_store(qkv: torch.Tensor, pos: torch.Tensor, slot: torch.Tensor, kv_l
     assert pos.dtype == torch.int32 and slot.dtype == torch.int32
     max_pages = kv_layer.shape[0]
     _check(lib().blitz_rope_kv_store(_p(qkv), _p(pos), _p(slot), _p(kv_layer), T, q_heads, kv_heads, head_dim,
-                                     page_size, max_pages, rope_theta, _p(status_word(qkv.device)), _dt(qkv),
+                                     page_size, max_pages, rope_theta, _status_ptr(qkv), _dt(qkv),
                                      _stream()), "blitz_rope_kv_store")
 
 
@@ -401,7 +438,7 @@ def attn_decode(q: torch.Tensor, kv_layer: KVLayer, indices: torch.Tensor, indpt
     _check(lib().blitz_attn_decode(_p(q), q.stride(0), kp, vp, _p(indices), _p(indptr), _p(last_page_len),
                                    _p(out), out.stride(0), _p(workspace), B, q_heads, kv_heads, head_dim, vdim, page_size,
                                    page_rows, pages, num_splits, sm_scale, window, keep_first, int(chunked), int(sigmoid), softcap, _p(sink), *_bias(bias, q_heads), *_gate(gate),
-                                   int(static_table), _p(status_word(q.device)), _dt(q), _stream()), "blitz_attn_decode")
+                                   int(static_table), _status_ptr(q), _dt(q), _stream()), "blitz_attn_decode")
     return out
 
 
@@ -458,7 +495,7 @@ def attn_prefill_paged(q: torch.Tensor, kv_layer: KVLayer, page_indices: torch.T
     _check(lib().blitz_attn_prefill_paged(_p(q), q.stride(0), kp, vp, _p(out), out.stride(0), _p(page_indices),
                                           _p(work), work.shape[0], T, q_heads, kv_heads, head_dim, vdim, page_size, page_rows,
                                           pages, sm_scale, 1 if poly_exp else 0, window, keep_first, int(chunked), int(sigmoid), softcap, _p(sink),
-                                          *_bias(bias, q_heads), *_gate(gate), _p(status_word(q.device)), _dt(q), _stream()), "blitz_attn_prefill_paged")
+                                          *_bias(bias, q_heads), *_gate(gate), _status_ptr(q), _dt(q), _stream()), "blitz_attn_prefill_paged")
     return out
 
 
@@ -485,7 +522,7 @@ def stream_norm(x: torch.Tensor, w: Optional[torch.Tensor], eps: float, out: Opt
     _check(lib().blitz_stream_norm(_p(ids), _p(embed), _p(step), _p(rows), row_offset, _p(x), _p(w), _p(out), _p(add), _p(add_rows),
                                    n_add, n,
                                    x.shape[1], embed.shape[0] if embed is not None else 0, int(init), int(add_embed),
-                                   eps, w_offset, _p(status_word(x.device)), _dt3(ref), _stream()), "blitz_stream_norm")
+                                   eps, w_offset, _status_ptr(x), _dt3(ref), _stream()), "blitz_stream_norm")
     return out
 
 
@@ -515,7 +552,7 @@ def rope_store(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[torch.Ten
     kp, vp, page_rows, pages, vdim = _kv(kv_layer)
     _check(lib().blitz_rope_store(_p(q), _p(k), _p(v), _p(q_b), _p(k_b), _p(v_b), q.stride(0), _p(q_w), _p(k_w), eps, _p(pos), _p(slot), kp, vp, _p(freqs),
                                   gain, T, q_heads, kv_heads, dim, vdim, rot_dims, int(interleaved), page_size, page_rows, pages,
-                                  _p(status_word(q.device)), _dt3(q), _stream()), "blitz_rope_store")
+                                  _status_ptr(q), _dt3(q), _stream()), "blitz_rope_store")
 
 
 def attn_ragged(q: torch.Tensor, kv_layer: KVLayer, pos: torch.Tensor, tok_indptr: Optional[torch.Tensor],
@@ -533,7 +570,7 @@ def attn_ragged(q: torch.Tensor, kv_layer: KVLayer, pos: torch.Tensor, tok_indpt
                                    _p(page_indptr), _p(page_indices), _p(sink), *_bias(bias, q_heads),
                                    kv_layer.pool.shape[3] if isinstance(kv_layer, LatentKV) else vdim, *_gate(gate), T, rows,
                                    q_heads, kv_heads, dim, vdim,
-                                   page_size, page_rows, pages, window, keep_first, int(chunked), int(sigmoid), scale, softcap, _p(status_word(q.device)),
+                                   page_size, page_rows, pages, window, keep_first, int(chunked), int(sigmoid), scale, softcap, _status_ptr(q),
                                    _dt3(q), _stream()), "blitz_attn_ragged")
     return out
 
@@ -561,7 +598,7 @@ def stream_mix(x: torch.Tensor, *, n: Optional[int] = None, ids: Optional[torch.
     _check(lib().blitz_stream_mix(_p(ids), _p(embed), embed.shape[0] if embed is not None else 0, int(embed is not None), _p(x), _p(pd.y),
                                   _p(pd.place), pd.place.shape[1] if pd.place is not None else 0, _p(pd.ident), _p(pd.prev), _p(pd.mix),
                                   _p(pd.out), _p(read), _p(alpha), _p(w), _p(b), _p(rows), row_offset, _p(out), _p(total), int(write),
-                                  n, H, S, _p(status_word(x.device)), _dt3(ref), _stream()), "blitz_stream_mix")
+                                  n, H, S, _status_ptr(x), _dt3(ref), _stream()), "blitz_stream_mix")
 
 
 class Pending(NamedTuple):
@@ -619,7 +656,7 @@ def stream_rms(x: torch.Tensor, *, eps: float, n: Optional[int] = None, ids: Opt
                                   pd.y.stride(0) if pd.y is not None else H, _p(pd.bias), _p(w0), _p(w1), _p(pd.mix), _p(pd.out), _p(read),
                                   _p(w), int(w is not None and w.numel() > 1), w_offset, eps, _p(rows), row_offset, _p(out), int(h32), _p(total),
                                   int(write), _p(ts.conv), taps, _p(ts.hist), _p(ts.mu), mixes, _p(ts.shift), _p(pos), _p(seq_slot),
-                                  0 if ts.hist is None else ts.hist.shape[0], n, H, S, _p(status_word(x.device)), _dt3(ref), _stream()),
+                                  0 if ts.hist is None else ts.hist.shape[0], n, H, S, _status_ptr(x), _dt3(ref), _stream()),
            "blitz_stream_rms")
 
 
@@ -637,7 +674,7 @@ def token_conv(x: torch.Tensor, conv: torch.Tensor, hist: torch.Tensor, out: tor
     assert conv.is_contiguous() and hist.is_contiguous() and out.shape[1] >= max(1, mixes) * width
     _check(lib().blitz_token_conv(_p(x), x.stride(0), _p(conv), _p(bias), _p(hist), _p(out), out.stride(0), int(silu), int(residual), int(x.dtype != out.dtype), _p(mu),
                                   mixes, _p(shift), _p(last), _p(pos), _p(tok_indptr), _p(seq_slot), x.shape[0], seq_slot.numel(), width,
-                                  keep + 1, slots, _p(status_word(x.device)), _dt3(out), _stream()), "blitz_token_conv")
+                                  keep + 1, slots, _status_ptr(x), _dt3(out), _stream()), "blitz_token_conv")
     return out
 
 
@@ -650,7 +687,7 @@ def norm_store(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, pos: torch.Ten
     assert all(x.stride(0) == q.stride(0) and x.stride(1) == 1 for x in (q, k, v))
     kp, vp, page_rows, pages, vdim = _kv(kv_layer)
     _check(lib().blitz_norm_store(_p(q), _p(k), _p(v), q.stride(0), _p(q_w), _p(k_w), eps, temp_coef, temp_every, _p(pos), _p(slot),
-                                  kp, vp, T, q_heads, kv_heads, dim, vdim, page_size, page_rows, pages, _p(status_word(q.device)),
+                                  kp, vp, T, q_heads, kv_heads, dim, vdim, page_size, page_rows, pages, _status_ptr(q),
                                   _dt3(q), _stream()), "blitz_norm_store")
 
 
@@ -664,7 +701,7 @@ def latent_store(cq: Optional[torch.Tensor], ckv: torch.Tensor, pos: torch.Tenso
     assert ckv.shape[1] == width and ckv.stride(1) == 1 and (cq is None or (cq.stride(0) == ckv.stride(0) and cq.stride(1) == 1))
     _check(lib().blitz_latent_store(_p(cq), _p(ckv), ckv.stride(0), _p(cq_w), _p(ckv_w), _p(pos), _p(slot), _p(kv.pool), _p(freqs), eps,
                                     T, cq.shape[1] if cq is not None else 0, kv.rank, width - kv.rank, int(interleaved), page, pages,
-                                    _p(status_word(ckv.device)), _dt3(ckv), _stream()), "blitz_latent_store")
+                                    _status_ptr(ckv), _dt3(ckv), _stream()), "blitz_latent_store")
 
 
 def latent_rotate(q: torch.Tensor, out: torch.Tensor, pos: torch.Tensor, freqs: torch.Tensor, *, heads: int, dim: int, rot: int,
@@ -681,7 +718,7 @@ def latent_gather(kv: LatentKV, pages: torch.Tensor, out: torch.Tensor) -> torch
     n, page, width = pages.numel(), kv.pool.shape[1], kv.pool.shape[3]
     assert out.is_contiguous() and out.shape == (n * page, width) and pages.dtype == torch.int32
     _check(lib().blitz_latent_gather(_p(kv.pool), _p(pages), _p(out), n, page * width * out.element_size(), kv.pool.shape[0],
-                                     _p(status_word(out.device)), _stream()), "blitz_latent_gather")
+                                     _status_ptr(out), _stream()), "blitz_latent_gather")
     return out
 
 
@@ -727,7 +764,7 @@ def _attn_latent(q, kv, indices, indptr, last_page_len, heads, scale, workspace,
     assert q.shape == (B, heads * width) and out.shape == (B, heads * kv.rank) and q.stride(1) == 1 and out.stride(1) == 1
     assert workspace.numel() >= int(lib().blitz_attn_latent_workspace_bytes(heads, kv.rank))
     _check(lib().blitz_attn_latent(_p(q), q.stride(0), _p(kv.pool), _p(indices), _p(indptr), _p(last_page_len), _p(pos),
-                                   _p(tok_indptr), rows, first, _p(out), out.stride(0), _p(workspace), B, heads, width, kv.rank, page, pages, scale, window, _p(sink), *_gate(gate), keys, int(static_table), _p(status_word(q.device)),
+                                   _p(tok_indptr), rows, first, _p(out), out.stride(0), _p(workspace), B, heads, width, kv.rank, page, pages, scale, window, _p(sink), *_gate(gate), keys, int(static_table), _status_ptr(q),
                                    _dt(q), _stream()), "blitz_attn_latent")
 
 
@@ -785,7 +822,7 @@ def moe_route(logits: torch.Tensor, plan: ExpertPlan, *, weight_on_input: bool =
                                  int(renormalize), plan.identity, int(softmax), groups, keep, _p(correction),
                                  0 if correction is None else _dt3(correction), _p(plan._ident), tile_rows, plan.tiles_at_most(T, tile_rows), _p(plan.pairs), _p(plan.counters),
                                  _p(plan.src), _p(plan.factors), _p(plan._place), _p(plan._tiles), _p(plan.num_tiles),
-                                 _p(status_word(logits.device)), _stream()), "blitz_moe_route")
+                                 _status_ptr(logits), _stream()), "blitz_moe_route")
     return plan
 
 
@@ -823,7 +860,7 @@ def gemm_grouped(a: torch.Tensor, b: torch.Tensor, plan: ExpertPlan, out: torch.
     _check(lib().blitz_gemm_grouped(_p(a), a.stride(0), plan.tokens if gather else plan.rows, _p(src), _p(b), E, N, K, _p(shared), Ns,
                                     Ks, _p(out), out.stride(0), _p(fac), _p(plan._tiles), _p(plan.num_tiles), most,
                                     *plan.tiles_usually(), row0, shared_rows, plan.tokens, _ACT[act], bn, fetch,
-                                    _p(status_word(a.device)), _dt(a), _stream()), "blitz_gemm_grouped")
+                                    _status_ptr(a), _dt(a), _stream()), "blitz_gemm_grouped")
     return out
 
 
@@ -842,7 +879,7 @@ def gla_recurrent(q, k, v, g, low, a2, a2_b, norm, state: torch.Tensor, out: tor
     _check(lib().blitz_gla_recurrent(_p(q), _p(k), _p(v), _p(g), _p(low), q.stride(0), _p(a2), _p(a2_b), _p(norm),
                                      _p(state), _p(out), out.stride(0), _p(pos), _p(tok_indptr), _p(seq_slot),
                                      seq_slot.numel(), heads, dim, vdim, rank, slots, dim ** -0.5, tau, eps,
-                                     int(tok_indptr is not None), _p(status_word(q.device)), _dt3(q), _stream()),
+                                     int(tok_indptr is not None), _status_ptr(q), _dt3(q), _stream()),
            "blitz_gla_recurrent")
     return out
 
@@ -852,7 +889,7 @@ def conv_causal(x, x_b, conv, conv_b, hist: torch.Tensor, u: torch.Tensor, pos, 
     slots, keep, width = hist.shape
     _check(lib().blitz_conv_causal(_p(x), x.stride(0), _p(x_b), _p(conv), _p(conv_b), _p(hist), _p(u), u.stride(0), _p(pos),
                                    _p(tok_indptr), _p(seq_slot), x.shape[0], seq_slot.numel(), width, keep + 1, slots,
-                                   _p(status_word(x.device)), _dt3(x), _stream()), "blitz_conv_causal")
+                                   _status_ptr(x), _dt3(x), _stream()), "blitz_conv_causal")
     return u
 
 
@@ -865,7 +902,7 @@ def rglru_scan(u, gates: torch.Tensor, gate_b, lam, y, x, y_b, state: torch.Tens
     _check(lib().blitz_rglru_scan(_p(u), u.stride(0), _p(gates), _p(gate_b), _p(lam), _p(y), _p(x), y.stride(0), _p(y_b),
                                   _p(state), _p(hist), _p(out), out.stride(0), _p(pos), _p(tok_indptr), _p(seq_slot),
                                   seq_slot.numel(), width, block, hist.shape[1] + 1, slots, int(tok_indptr is None),
-                                  _p(status_word(u.device)), _dt3(u), _stream()), "blitz_rglru_scan")
+                                  _status_ptr(u), _dt3(u), _stream()), "blitz_rglru_scan")
     return out
 
 
@@ -889,7 +926,7 @@ def gla(q, k, v, g, low, a2, a2_b, norm, state: torch.Tensor, out: torch.Tensor,
     assert cum.dtype == torch.float32 and cum.numel() >= n and state.dtype == torch.float32 and state.is_contiguous()
     _check(lib().blitz_gla_chunk(_p(q), _p(k), _p(v), _p(g), _p(low), q.stride(0), _p(a2), _p(a2_b), _p(norm), _p(cum),
                                  _p(state), _p(out), out.stride(0), _p(pos), _p(tok_indptr), _p(seq_slot), seq_slot.numel(),
-                                 longest, heads, dim, vdim, rank, slots, dim ** -0.5, tau, eps, _p(status_word(q.device)),
+                                 longest, heads, dim, vdim, rank, slots, dim ** -0.5, tau, eps, _status_ptr(q),
                                  _stream()), "blitz_gla_chunk")
     return out
 
@@ -907,7 +944,7 @@ def wkv(r, k, v, g, low: torch.Tensor, a2, a2_b, bonus, norm, state: torch.Tenso
     if (longest < GLA_CHUNK_MIN_LEN or r.dtype != torch.bfloat16 or not aligned or out.stride(0) % 2 or out.data_ptr() % 4
             or not lib().blitz_gla_chunk_supported(dim, vdim, rank)):
         _check(lib().blitz_wkv_recurrent(*args, _p(state), _p(out), out.stride(0), _p(pos), _p(tok_indptr), _p(seq_slot), seq_slot.numel(),
-                                         heads, dim, vdim, rank, slots, eps, int(tok_indptr is not None), _p(status_word(r.device)),
+                                         heads, dim, vdim, rank, slots, eps, int(tok_indptr is not None), _status_ptr(r),
                                          _dt3(r), _stream()), "blitz_wkv_recurrent")
         return out
     n = r.shape[0] * heads * dim
@@ -915,7 +952,7 @@ def wkv(r, k, v, g, low: torch.Tensor, a2, a2_b, bonus, norm, state: torch.Tenso
         cum = torch.empty(n, dtype=torch.float32, device=r.device)
     assert cum.dtype == torch.float32 and cum.numel() >= n
     _check(lib().blitz_wkv_chunk(*args, _p(cum), _p(state), _p(out), out.stride(0), _p(pos), _p(tok_indptr), _p(seq_slot), seq_slot.numel(),
-                                 longest, heads, dim, vdim, rank, slots, eps, _p(status_word(r.device)), _stream()), "blitz_wkv_chunk")
+                                 longest, heads, dim, vdim, rank, slots, eps, _status_ptr(r), _stream()), "blitz_wkv_chunk")
     return out
 
 
@@ -930,7 +967,7 @@ def ssd(x, B, C, z, dt, dt_bias, A_log, D, state: torch.Tensor, out: torch.Tenso
     assert state.dtype == torch.float32 and state.is_contiguous() and out.stride(1) == 1
     assert B.stride(0) == x.stride(0) == C.stride(0) and z.stride(0) == dt.stride(0)
     args = [_p(x), _p(B), _p(C), x.stride(0), _p(z), _p(dt), z.stride(0), _p(dt_bias), _p(A_log), _p(D), _p(state), _p(out), out.stride(0),
-            _p(pos), _p(tok_indptr), _p(seq_slot), seq_slot.numel(), heads, groups, dim, vdim, slots, _p(status_word(x.device))]
+            _p(pos), _p(tok_indptr), _p(seq_slot), seq_slot.numel(), heads, groups, dim, vdim, slots, _status_ptr(x)]
     longest = 1 if tok_indptr is None else max(row_lens)
     aligned = all(t.data_ptr() % 16 == 0 for t in (x, B, C)) and x.stride(0) % 8 == 0 and all(t.data_ptr() % 4 == 0 and t.stride(0) % 2 == 0 for t in (z, out))
     if longest < SSD_CHUNK_MIN_LEN or x.dtype != torch.bfloat16 or not aligned or not lib().blitz_ssd_chunk_supported(dim, vdim):

@@ -11,6 +11,7 @@ exactly one H2D copy (inputs + page table) and one D2H copy (sampled tokens) per
 from __future__ import annotations
 
 import time
+from itertools import accumulate
 from typing import Dict, List, Optional, Sequence
 
 import numpy as np
@@ -269,8 +270,11 @@ class Engine:
             raise ValueError(f"step over {batch.size} sequences exceeds max_batch={self.max_batch}")
         counts = list(counts)
         want = [list(w) for w in want] if len(want) else [[] for _ in counts]
-        first = [sum(len(w) for w in want[:i]) for i in range(len(want))]
         total = sum(len(w) for w in want)
+        if 0 < sum(counts) <= self.max_batch_tokens and all(0 <= p < c for w, c in zip(want, counts) for p in w):
+            # one pass, whose rows come in the order asked for
+            return self._step_pass(batch, counts, [(i, p) for i, w in enumerate(want) for p in w])
+        first = [sum(len(w) for w in want[:i]) for i in range(len(want))]
         out = torch.empty(total, self.cfg.vocab, dtype=torch.float32, device=self.device) if total else None
         done = [0] * len(counts)
         while any(d < c for d, c in zip(done, counts)):
@@ -306,19 +310,23 @@ class Engine:
                 self.runner.forward(self._views(pad, pad, self.num_pages, False, splits=splits))
             got = None
             if src:
-                got = self.runner.logits[torch.tensor([row_of[b] for b, _ in src], device=self.device)].float()
+                at = [row_of[b] for b, _ in src]
+                if at == list(range(len(at))):
+                    got = self.runner.logits[:len(at)].to(torch.float32, copy=True)
+                else:
+                    got = self.runner.logits[torch.tensor(at, device=self.device)].float()
         else:
             splits = self.choose_splits(singles, max(kv_lens[:singles]), sum(kv_lens[:singles])) if singles else 1
             m = self._views(T, rows, P, True, q_lens, splits=splits, kv_lens=kv_lens, singles=singles)
             with nvtx_range("step"):
                 self.runner.forward(m, with_head=False)
-                starts = [sum(q_lens[:r]) for r in range(rows)]
+                starts = [0, *accumulate(q_lens)]
                 flat = [starts[row_of[b]] + p for b, p in src]
                 parts = []
                 for i in range(0, len(flat), self.max_batch):
                     idx = torch.tensor(flat[i:i + self.max_batch], dtype=torch.int32, device=self.device)
-                    parts.append(self.runner.logits_of(idx.numel(), idx).float().clone())
-                got = torch.cat(parts) if parts else None
+                    parts.append(self.runner.logits_of(idx.numel(), idx).to(torch.float32, copy=True))
+                got = parts[0] if len(parts) == 1 else torch.cat(parts) if parts else None
         torch.cuda.current_stream().synchronize()       # the staging arrays are reused by the next pass
         batch.advance(counts)
         return got
