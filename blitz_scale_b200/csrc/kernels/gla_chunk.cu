@@ -42,6 +42,7 @@ constexpr int kGcB = 16;        // tokens per block
 constexpr int kGcV = 64;        // value columns per CTA: this many, or twice as many when that still fills the GPU
 constexpr int kGcThreads = 512;
 constexpr int kGcMaxCluster = 8;
+constexpr int kGcMaxSegments = 16;  // of a row: a segment reads what those before it left
 constexpr float kGcMaxDecay = 80.f;
 
 struct GlaChunkParams {
@@ -59,6 +60,32 @@ struct GlaChunkParams {
   int heads, dim, vdim, rank, num_slots;
   float q_scale, inv_tau, eps;
   int* status;
+  int rows;
+  int seg_chunks;        // chunks of a segment; 0: rows whole
+  float* seg_state;      // [segments][heads][dim][vdim], and
+  float* seg_decay;      // [segments][heads * dim]: see GcSegment
+};
+
+// One segment of a row: `seg_chunks` chunks, the last one what is left.  Entry 0 of a row that is cut: the state it starts with (unless
+// that is zero); entry j: what segment j - 1 adds to the state, and the sum of its log decays (the first one: the state behind it).
+struct GcSegment {
+  int row, seg, num, beg, len, t_row;  // beg, len: its tokens; t_row: the row's first
+  int64_t entry;                       // of entry 0: rows of n segments are n entries apart at least
+  __device__ GcSegment(const GlaChunkParams& p, int z) {
+    row = z % p.rows;
+    seg = z / p.rows;
+    t_row = beg = p.tok_indptr[row];
+    len = p.tok_indptr[row + 1] - beg;
+    num = 1;
+    entry = 0;
+    if (p.seg_chunks > 0) {
+      const int tokens = p.seg_chunks * kGcC;
+      num = (len + tokens - 1) / tokens;
+      entry = beg / tokens + row;
+      beg += seg * tokens;
+      len = min(tokens, len - seg * tokens);
+    }
+  }
 };
 
 // log(sigmoid(z)) = min(z, 0) - log(1 + e^-|z|) on the special-function unit; the series keeps the digits of a slow decay
@@ -168,6 +195,176 @@ __device__ __forceinline__ void gc_tile(int tile, int& i, int& j) {
   j = tile >= 6 ? i : (tile >= 3 ? tile - 3 : tile >= 1 ? tile - 1 : 0);
 }
 
+// This warp's part of the state that a segment starts with: the row's own, or what the segments before it leave.
+template <int NT>
+__device__ __forceinline__ void gc_load_state(const GlaChunkParams& p, const GcSegment& sg, int h, int v0, int nv, bool has_state, int rowS,
+                                              int cS, float (&S)[NT][4]) {
+  const int64_t size = static_cast<int64_t>(p.heads) * p.dim * p.vdim, head = static_cast<int64_t>(h) * p.dim * p.vdim + v0;
+  const bool fresh = p.pos[sg.t_row] == 0;
+  const int t4 = threadIdx.x & 3;
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) S[n][e] = 0.f;
+  if (!has_state || (sg.seg == 0 && fresh)) return;
+  for (int j = min(1, sg.seg); j <= sg.seg; ++j) {
+    const float* from = (sg.num == 1 ? p.state + p.seq_slot[sg.row] * size : p.seg_state + (sg.entry + j) * size) + head;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int c = rowS + half * 8;
+      if (c >= p.dim) continue;
+      const float d = j < 2 ? 0.f : __expf(p.seg_decay[(sg.entry + j) * p.heads * p.dim + h * p.dim + c]);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        const int col = cS + n * 8 + 2 * t4;
+        if (col >= nv) continue;
+        const float* x = from + static_cast<int64_t>(c) * p.vdim + col;
+        S[n][2 * half] = S[n][2 * half] * d + x[0];
+        S[n][2 * half + 1] = S[n][2 * half + 1] * d + x[1];
+      }
+    }
+  }
+}
+
+// What every segment but a row's last adds to the state: the part of the recurrence that has to run before the others.  Bound by the
+// loads of k, v and b (a chunk ahead) and by 16 x 64 x VB products a warp; two sets of operands, one barrier per chunk.
+template <int DK, int VB>
+struct GsSmem {
+  static constexpr int kK = DK + 8, kV = VB + 8;
+  struct Set {
+    __nv_bfloat16 kh[kGcC * kK], kl[kGcC * kK], v[kGcC * kV];  // k e^(b_end - b)
+    float fe[DK];                                              // e^(b_end)
+  } set[2];
+};
+template <int DK, int VB>
+__global__ void __launch_bounds__(kGcThreads, 1) gla_segment_kernel(const GlaChunkParams p) {
+  using bf = __nv_bfloat16;
+  using SM = GsSmem<DK, VB>;
+  constexpr int RB = DK / 16, CP = RB >= 4 ? 16 / RB : 4, NT = VB / CP / 8;  // as in gla_chunk_kernel
+  constexpr int kVecs = kGcC * DK / 8, NV = (kVecs + kGcThreads - 1) / kGcThreads;
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  SM& sm = *reinterpret_cast<SM*>(smem_raw);
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  const int mi = lane >> 3, mr = lane & 7;
+  const int h = blockIdx.y, v0 = blockIdx.x * VB, nv = min(VB, p.vdim - v0), hk = p.heads * p.dim;
+  const GcSegment sg(p, blockIdx.z);
+  const int slot = p.seq_slot[sg.row];
+  if (slot < 0 || slot >= p.num_slots || sg.seg >= sg.num - 1) return;
+  const bool has_state = warp < RB * CP;
+  const int rbS = warp % RB, cS = has_state ? (warp / RB) * (VB / CP) : 0, rowS = rbS * 16 + g;
+  const int64_t size = static_cast<int64_t>(p.heads) * p.dim * p.vdim, head = static_cast<int64_t>(h) * p.dim * p.vdim + v0;
+  float S[NT][4];
+  auto store = [&](int64_t entry) {
+    float* to = p.seg_state + entry * size + head;
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int c = rowS + half * 8, col = cS + n * 8 + 2 * t4;
+        if (has_state && c < p.dim && col < nv)
+          *reinterpret_cast<float2*>(to + static_cast<int64_t>(c) * p.vdim + col) = make_float2(S[n][2 * half], S[n][2 * half + 1]);
+      }
+  };
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) S[n][e] = 0.f;
+  if (sg.seg == 0 && p.pos[sg.t_row] != 0) {  // the row's last segment writes its new state: keep the old one for the first
+    const float* from = p.state + slot * size + head;
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int c = rowS + half * 8, col = cS + n * 8 + 2 * t4;
+        if (!has_state || c >= p.dim || col >= nv) continue;
+        S[n][2 * half] = from[static_cast<int64_t>(c) * p.vdim + col];
+        S[n][2 * half + 1] = from[static_cast<int64_t>(c) * p.vdim + col + 1];
+      }
+    store(sg.entry);
+  }
+
+  uint4 rk[NV], rv[VB / 64];
+  float rb[NV][8], re[NV][8], rend = 0.f, sum = 0.f;
+  auto request = [&](int chunk) {
+    const int64_t tok = sg.beg + chunk * kGcC;
+    const float* cum = p.cum + tok * hk + h * p.dim;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int e = tid + i * kGcThreads, t = e / (DK / 8), c = (e % (DK / 8)) * 8;
+      rk[i] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) rb[i][j] = re[i][j] = 0.f;
+      if (e < kVecs && c < p.dim) {
+        rk[i] = *reinterpret_cast<const uint4*>(p.k + (tok + t) * p.row + h * p.dim + c);
+        ldf8(cum + static_cast<int64_t>(t) * hk + c, rb[i]);
+        ldf8(cum + static_cast<int64_t>(kGcC - 1) * hk + c, re[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < VB / 64; ++i) {
+      const int t = tid / 8, c = (tid % 8) * 8 + i * 64;
+      rv[i] = make_uint4(0, 0, 0, 0);
+      if (c < nv) rv[i] = *reinterpret_cast<const uint4*>(p.v + (tok + t) * p.row + h * p.vdim + v0 + c);
+    }
+    if (tid < p.dim) rend = cum[static_cast<int64_t>(kGcC - 1) * hk + tid];
+  };
+  const int nchunks = sg.len / kGcC;  // whole chunks all of them
+  request(0);
+  for (int ch = 0; ch < nchunks; ++ch) {
+    auto& st = sm.set[ch & 1];  // (whoever still reads it has not passed the barrier of the chunk before)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int e = tid + i * kGcThreads, t = e / (DK / 8), c = (e % (DK / 8)) * 8;
+      if (e >= kVecs) continue;
+      float x[8];
+      unpack8<bf>(rk[i], x);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] *= __expf(re[i][j] - rb[i][j]);
+      uint4 hi, lo;
+      split2(x[0], x[1], hi.x, lo.x);
+      split2(x[2], x[3], hi.y, lo.y);
+      split2(x[4], x[5], hi.z, lo.z);
+      split2(x[6], x[7], hi.w, lo.w);
+      *reinterpret_cast<uint4*>(st.kh + t * SM::kK + c) = hi;
+      *reinterpret_cast<uint4*>(st.kl + t * SM::kK + c) = lo;
+    }
+#pragma unroll
+    for (int i = 0; i < VB / 64; ++i) *reinterpret_cast<uint4*>(st.v + (tid / 8) * SM::kV + (tid % 8) * 8 + i * 64) = rv[i];
+    if (tid < DK) st.fe[tid] = __expf(rend);
+    sum += rend;
+    if (ch + 1 < nchunks) request(ch + 1);
+    __syncthreads();
+    if (!has_state) continue;
+    const float d0 = st.fe[rowS], d1 = st.fe[rowS + 8];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      S[n][0] *= d0; S[n][1] *= d0;
+      S[n][2] *= d1; S[n][3] *= d1;
+    }
+#pragma unroll
+    for (int j = 0; j < kGcC / 16; ++j) {
+      const uint32_t off = static_cast<uint32_t>((j * 16 + (mi >> 1) * 8 + mr) * SM::kK + rbS * 16 + (mi & 1) * 8);
+      uint32_t ah[4], al[4];
+      ldmatrix_x4_trans(ptx::smem_u32(st.kh + off), ah[0], ah[1], ah[2], ah[3]);
+      ldmatrix_x4_trans(ptx::smem_u32(st.kl + off), al[0], al[1], al[2], al[3]);
+#pragma unroll
+      for (int m = 0; m < NT / 2; ++m) {
+        const uint32_t at = static_cast<uint32_t>((j * 16 + (mi & 1) * 8 + mr) * SM::kV + cS + m * 16 + (mi >> 1) * 8);
+        uint32_t b0, b1, b2, b3;
+        ldmatrix_x4_trans(ptx::smem_u32(st.v + at), b0, b1, b2, b3);
+        mma16816<bf>(S[2 * m], ah[0], ah[1], ah[2], ah[3], b0, b1);
+        mma16816<bf>(S[2 * m + 1], ah[0], ah[1], ah[2], ah[3], b2, b3);
+        mma16816<bf>(S[2 * m], al[0], al[1], al[2], al[3], b0, b1);
+        mma16816<bf>(S[2 * m + 1], al[0], al[1], al[2], al[3], b2, b3);
+      }
+    }
+  }
+  store(sg.entry + sg.seg + 1);
+  if (v0 == 0 && tid < p.dim) p.seg_decay[(sg.entry + sg.seg + 1) * hk + h * p.dim + tid] = sum;
+}
+
 template <int DK, int VB, bool WKV>
 __global__ void __launch_bounds__(kGcThreads, 1) gla_chunk_kernel(const GlaChunkParams p) {
   using bf = __nv_bfloat16;
@@ -185,12 +382,12 @@ __global__ void __launch_bounds__(kGcThreads, 1) gla_chunk_kernel(const GlaChunk
   ptx::griddep_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int mi = lane >> 3, mr = lane & 7;
-  const int h = blockIdx.y, r = blockIdx.z, nrank = gridDim.x, rank = blockIdx.x;
+  const int h = blockIdx.y, nrank = gridDim.x, rank = blockIdx.x;
   const int v0 = blockIdx.x * VB, nv = min(VB, p.vdim - v0);
-  const int slot = p.seq_slot[r];
-  const int t_beg = p.tok_indptr[r], len = p.tok_indptr[r + 1] - t_beg;
+  const GcSegment sg(p, blockIdx.z);
+  const int slot = p.seq_slot[sg.row], t_beg = sg.beg, len = sg.len;
   const int hk = p.heads * p.dim;
-  // the CTAs of a cluster have the same row: they take the same way out
+  // the CTAs of a cluster have the same segment: they take the same way out
   if (slot < 0 || slot >= p.num_slots || len <= 0) {
     if (slot >= p.num_slots && tid == 0 && p.status) atomicCAS(p.status, 0, kStatusBadIndex);
     return;
@@ -202,14 +399,7 @@ __global__ void __launch_bounds__(kGcThreads, 1) gla_chunk_kernel(const GlaChunk
   const int rowS = rbS * 16 + g;
   float* gstate = p.state + (static_cast<int64_t>(slot) * p.heads + h) * p.dim * p.vdim + v0;
   float S[NT][4];
-  const bool fresh = p.pos[t_beg] == 0;
-#pragma unroll
-  for (int n = 0; n < NT; ++n)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int c = rowS + (e >> 1) * 8, col = cS + n * 8 + 2 * t4 + (e & 1);
-      S[n][e] = (fresh || !has_state || c >= p.dim || col >= nv) ? 0.f : gstate[static_cast<int64_t>(c) * p.vdim + col];
-    }
+  gc_load_state<NT>(p, sg, h, v0, nv, has_state, rowS, cS, S);
   auto publish_state = [&] {
     if (!has_state) return;
 #pragma unroll
@@ -585,32 +775,66 @@ __global__ void __launch_bounds__(kGcThreads, 1) gla_chunk_kernel(const GlaChunk
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int c = rowS + (e >> 1) * 8, col = cS + n * 8 + 2 * t4 + (e & 1);
-      if (has_state && c < p.dim && col < nv) gstate[static_cast<int64_t>(c) * p.vdim + col] = S[n][e];
+      if (sg.seg == sg.num - 1 && has_state && c < p.dim && col < nv) gstate[static_cast<int64_t>(c) * p.vdim + col] = S[n][e];
     }
 }
 
+// Chunks of a segment, 0 to leave the rows whole.  Whole rows take as long as the longest one (a chunk: 8 to 13 us); cut, the chunks of
+// all rows and heads are dealt out over the SMs, for the price of another pass over k and v (a quarter of a chunk's time) and of a
+// segment's granularity.  Whole and cut: 593 and 397 us for rows of 455, 335, 1489 and 2720 tokens, 16 heads of 128 x 256; 177 and 97
+// for one of 1024, 656 and 313 for one of 4096; second form with 32 heads of 128 x 128, rows of 254, 315 and 2432: 1208 and 455, one of
+// 8192 with 16 heads: 1656 and 490.  One row of 512 tokens (99 and 91) is near the line, rows of equal length stay whole.
+static int gla_segment_chunks(int64_t tokens, int rows, int max_len, int heads, int vdim, int sms) {
+  const int64_t longest = (max_len + kGcC - 1) / kGcC, blocks = (int64_t)heads * ((vdim + 2 * kGcV - 1) / (2 * kGcV));
+  const int64_t share = ((tokens + kGcC - 1) / kGcC * blocks + sms - 1) / sms;  // chunks per SM
+  int64_t cut = share / 2;
+  if (cut < (longest + kGcMaxSegments - 1) / kGcMaxSegments) cut = (longest + kGcMaxSegments - 1) / kGcMaxSegments;
+  if (cut < 4) cut = 4;
+  return rows <= 65535 / kGcMaxSegments && 5 * share / 4 + cut < longest * 9 / 10 ? (int)cut : 0;
+}
+
 template <int DK, int VB, bool WKV>
-static cudaError_t launch_gla_chunk(const GlaChunkParams& p, int rows, cudaStream_t stream) {
+static cudaError_t launch_gla_chunk(const GlaChunkParams& p, int max_len, cudaStream_t stream) {
+  const unsigned vb = (p.vdim + VB - 1) / VB;
+  unsigned segments = 1;
+  if (p.seg_chunks > 0) {
+    segments = (max_len + p.seg_chunks * kGcC - 1) / (p.seg_chunks * kGcC);
+    auto kern = gla_segment_kernel<DK, VB>;
+    constexpr int smem = (int)sizeof(GsSmem<DK, VB>);
+    static PerDeviceOnce once;
+    cudaError_t e = once.run([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+    if (e == cudaSuccess && segments > 1)
+      e = launch_pdl(kern, dim3(vb, p.heads, p.rows * (segments - 1)), dim3(kGcThreads), (size_t)smem, stream, p);
+    if (e != cudaSuccess) return e;
+  }
   auto kern = gla_chunk_kernel<DK, VB, WKV>;
   constexpr int smem = (int)sizeof(GcSmem<DK, VB>);
   static_assert(smem <= 227 * 1024, "shared memory");
   static PerDeviceOnce once;
   cudaError_t e = once.run([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
   if (e != cudaSuccess) return e;
-  const unsigned vb = (p.vdim + VB - 1) / VB;
-  return launch_pdl_cluster(kern, dim3(vb, p.heads, rows), dim3(kGcThreads), (size_t)smem, vb, stream, p);
+  return launch_pdl_cluster(kern, dim3(vb, p.heads, p.rows * segments), dim3(kGcThreads), (size_t)smem, vb, stream, p);
 }
 
 // 128 value columns per block halve the work that every block of a head repeats (scaled operands, scores); 64 give twice
 // as many blocks, which is worth more while they do not fill the GPU.
 template <int DK, bool WKV>
-static cudaError_t launch_gla_width(const GlaChunkParams& p, int rows, int sms, cudaStream_t stream) {
-  const bool wide = p.vdim > kGcV && (int64_t)rows * p.heads * ((p.vdim + kGcV - 1) / kGcV) > sms;
-  return wide ? launch_gla_chunk<DK, 2 * kGcV, WKV>(p, rows, stream) : launch_gla_chunk<DK, kGcV, WKV>(p, rows, stream);
+static cudaError_t launch_gla_width(const GlaChunkParams& p, int max_len, int sms, cudaStream_t stream) {
+  const bool wide = p.vdim > kGcV && (p.seg_chunks > 0 || (int64_t)p.rows * p.heads * ((p.vdim + kGcV - 1) / kGcV) > sms);
+  return wide ? launch_gla_chunk<DK, 2 * kGcV, WKV>(p, max_len, stream) : launch_gla_chunk<DK, kGcV, WKV>(p, max_len, stream);
 }
 
 template <bool WKV>
-static int gla_chunk_any(const GlaChunkParams& p, int rows, int max_len, cudaStream_t stream) {
+static int gla_chunk_any(GlaChunkParams& p, int rows, int max_len, int64_t tokens, void* seg, cudaStream_t stream) {
+  const int sms = device_sm_count();
+  p.rows = rows;
+  if (seg != nullptr && (reinterpret_cast<uintptr_t>(seg) & 15) == 0) {
+    p.seg_chunks = gla_segment_chunks(tokens, rows, max_len, p.heads, p.vdim, sms);
+    if (p.seg_chunks > 0) {
+      p.seg_state = static_cast<float*>(seg);
+      p.seg_decay = p.seg_state + (tokens / (p.seg_chunks * kGcC) + rows) * p.heads * p.dim * p.vdim;
+    }
+  }
   if (p.heads > 65535 || rows > 65535 || (p.row & 7) || (p.out_stride & 1)) return -1;
   for (const void* x : {p.q, p.k, p.v})
     if (reinterpret_cast<uintptr_t>(x) & 15) return -1;
@@ -628,10 +852,9 @@ static int gla_chunk_any(const GlaChunkParams& p, int rows, int max_len, cudaStr
   e = launch_pdl(gla_decay_kernel<WKV>, dim3((hk + kGdThreads - 1) / kGdThreads, (max_len + kGcC - 1) / kGcC, rows),
                              dim3(kGdThreads), smem, stream, p);
   if (e != cudaSuccess) return (int)e;
-  const int sms = device_sm_count();
-  e = p.dim <= 32   ? launch_gla_width<32, WKV>(p, rows, sms, stream)
-      : p.dim <= 64 ? launch_gla_width<64, WKV>(p, rows, sms, stream)
-                    : launch_gla_width<128, WKV>(p, rows, sms, stream);
+  e = p.dim <= 32   ? launch_gla_width<32, WKV>(p, max_len, sms, stream)
+      : p.dim <= 64 ? launch_gla_width<64, WKV>(p, max_len, sms, stream)
+                    : launch_gla_width<128, WKV>(p, max_len, sms, stream);
   return (int)e;
 }
 
@@ -646,10 +869,16 @@ int blitz_gla_chunk_supported(int dim, int vdim, int rank) {
          rank <= kGdMaxRank;
 }
 
+// Bytes of the scratch `seg` for `tokens` tokens (16-byte aligned; tok_indptr ends at `tokens` at most); 0: the rows are not cut.
+int64_t blitz_gla_chunk_scratch(int64_t tokens, int rows, int max_len, int heads, int dim, int vdim) {
+  const int cut = gla_segment_chunks(tokens, rows, max_len, heads, vdim, device_sm_count());
+  return cut == 0 ? 0 : (tokens / (cut * kGcC) + rows) * heads * dim * (vdim + 1) * (int64_t)sizeof(float);
+}
+
 // Rows of at least one token each: tokens tok_indptr[r] .. tok_indptr[r + 1]; max_len: the longest row.  cum: fp32 scratch
-// [tokens][heads * dim], indexed by token number.  The pitch `row` and the five column pointers are multiples of 8 elements.
+// [tokens][heads * dim], indexed by token number.  seg: blitz_gla_chunk_scratch bytes for the same `tokens`, or null.  The pitch `row` and the five column pointers are multiples of 8 elements.
 int blitz_gla_chunk(const void* q, const void* k, const void* v, const void* g, const void* low, int64_t row, const void* a2,
-                    const void* a2_b, const void* norm, float* cum, float* state, void* out, int64_t out_stride,
+                    const void* a2_b, const void* norm, float* cum, void* seg, int64_t tokens, float* state, void* out, int64_t out_stride,
                     const int32_t* pos, const int32_t* tok_indptr, const int32_t* seq_slot, int rows, int max_len, int heads,
                     int dim, int vdim, int rank, int num_slots, float q_scale, float tau, float eps, int* status,
                     cudaStream_t stream) {
@@ -659,12 +888,12 @@ int blitz_gla_chunk(const void* q, const void* k, const void* v, const void* g, 
   GlaChunkParams p{(const bf*)q, (const bf*)k, (const bf*)v, (const bf*)g, (const bf*)low, row, nullptr, 0, (const bf*)a2,
                    (const bf*)a2_b, (const bf*)norm, nullptr, 0, cum, state, (bf*)out, out_stride, pos, tok_indptr, seq_slot,
                    heads, dim, vdim, rank, num_slots, q_scale, 1.f / tau, eps, status};
-  return gla_chunk_any<false>(p, rows, max_len, stream);
+  return gla_chunk_any<false>(p, rows, max_len, tokens, seg, stream);
 }
 
 // The second form (see blitz_wkv_recurrent for what differs); bonus 16-byte aligned, dim a multiple of 8.
 int blitz_wkv_chunk(const void* q, const void* k, const void* v, const void* g, int64_t row, const float* low, int64_t low_row,
-                    const void* a2, const void* a2_b, const void* bonus, const void* norm, float* cum, float* state, void* out,
+                    const void* a2, const void* a2_b, const void* bonus, const void* norm, float* cum, void* seg, int64_t tokens, float* state, void* out,
                     int64_t out_stride, const int32_t* pos, const int32_t* tok_indptr, const int32_t* seq_slot, int rows,
                     int max_len, int heads, int dim, int vdim, int rank, int num_slots, float eps, int* status, cudaStream_t stream) {
   using bf = __nv_bfloat16;
@@ -673,7 +902,7 @@ int blitz_wkv_chunk(const void* q, const void* k, const void* v, const void* g, 
   GlaChunkParams p{(const bf*)q, (const bf*)k, (const bf*)v, (const bf*)g, nullptr, row, low, low_row, (const bf*)a2,
                    (const bf*)a2_b, (const bf*)norm, (const bf*)bonus, vdim, cum, state, (bf*)out, out_stride, pos, tok_indptr, seq_slot,
                    heads, dim, vdim, rank, num_slots, 1.f, 1.f, eps, status};
-  return gla_chunk_any<true>(p, rows, max_len, stream);
+  return gla_chunk_any<true>(p, rows, max_len, tokens, seg, stream);
 }
 
 }  // extern "C"

@@ -201,7 +201,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     N_out = b_cols / 2 and returns silu(a@gate) * (a@up).  ``split_k``: 0 lets the kernel split K when the
     GEMM is too skinny to fill the GPU, 1 forbids it, n > 1 forces n splits.
 
-    Up to 256 rows of ``a`` with 'kn' weights go to the weight-streaming decode kernel (operands swapped on
+    Up to 128 rows of ``a`` with 'kn' weights go to the weight-streaming decode kernel (operands swapped on
     the tensor core, K split over a thread-block cluster with the reduction in distributed shared memory);
     ``decode_path`` forces (True) or forbids (False) that choice and ``decode_split`` caps its cluster size.  ``static_b=True`` promises that ``b`` is not written by kernels still
     running in this stream (model weights), so the decode kernel may start streaming it before its
@@ -909,6 +909,12 @@ def rglru_scan(u, gates: torch.Tensor, gate_b, lam, y, x, y_b, state: torch.Tens
 GLA_CHUNK_MIN_LEN = 16      # rows shorter than this are faster token by token
 
 
+def _segment_scratch(x: torch.Tensor, rows: int, longest: int, heads: int, dim: int, vdim: int) -> Optional[torch.Tensor]:
+    """States between the segments that the chunked kernel cuts long rows into (None: it takes them whole)."""
+    n = lib().blitz_gla_chunk_scratch(x.shape[0], rows, longest, heads, dim, vdim)
+    return torch.empty(n, dtype=torch.uint8, device=x.device) if n else None
+
+
 def gla(q, k, v, g, low, a2, a2_b, norm, state: torch.Tensor, out: torch.Tensor, pos, tok_indptr, seq_slot, *, rank: int,
         tau: float, eps: float, row_lens=None, cum: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Gated linear attention over the rows of a step; ``row_lens``: tokens per row (host), needed where rows are longer
@@ -924,8 +930,9 @@ def gla(q, k, v, g, low, a2, a2_b, norm, state: torch.Tensor, out: torch.Tensor,
     if cum is None:
         cum = torch.empty(n, dtype=torch.float32, device=q.device)
     assert cum.dtype == torch.float32 and cum.numel() >= n and state.dtype == torch.float32 and state.is_contiguous()
+    seg = _segment_scratch(q, seq_slot.numel(), longest, heads, dim, vdim)
     _check(lib().blitz_gla_chunk(_p(q), _p(k), _p(v), _p(g), _p(low), q.stride(0), _p(a2), _p(a2_b), _p(norm), _p(cum),
-                                 _p(state), _p(out), out.stride(0), _p(pos), _p(tok_indptr), _p(seq_slot), seq_slot.numel(),
+                                 _p(seg), q.shape[0], _p(state), _p(out), out.stride(0), _p(pos), _p(tok_indptr), _p(seq_slot), seq_slot.numel(),
                                  longest, heads, dim, vdim, rank, slots, dim ** -0.5, tau, eps, _status_ptr(q),
                                  _stream()), "blitz_gla_chunk")
     return out
@@ -951,7 +958,8 @@ def wkv(r, k, v, g, low: torch.Tensor, a2, a2_b, bonus, norm, state: torch.Tenso
     if cum is None:
         cum = torch.empty(n, dtype=torch.float32, device=r.device)
     assert cum.dtype == torch.float32 and cum.numel() >= n
-    _check(lib().blitz_wkv_chunk(*args, _p(cum), _p(state), _p(out), out.stride(0), _p(pos), _p(tok_indptr), _p(seq_slot), seq_slot.numel(),
+    seg = _segment_scratch(r, seq_slot.numel(), longest, heads, dim, vdim)
+    _check(lib().blitz_wkv_chunk(*args, _p(cum), _p(seg), r.shape[0], _p(state), _p(out), out.stride(0), _p(pos), _p(tok_indptr), _p(seq_slot), seq_slot.numel(),
                                  longest, heads, dim, vdim, rank, slots, eps, _status_ptr(r), _stream()), "blitz_wkv_chunk")
     return out
 

@@ -120,7 +120,8 @@ def _declare(L: ctypes.CDLL) -> None:
                                     c_p])
     sig("blitz_gla_recurrent", [c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_p, c_i, c_i,
                                 c_i, c_i, c_i, c_i, c_f, c_f, c_f, c_i, c_p, c_i, c_p])
-    sig("blitz_gla_chunk", [c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_p, c_i, c_i, c_i,
+    sig("blitz_gla_chunk_scratch", [c_i64, c_i, c_i, c_i, c_i, c_i], c_i64)
+    sig("blitz_gla_chunk", [c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_i64, c_p, c_p, c_p, c_i, c_i, c_i,
                             c_i, c_i, c_i, c_i, c_f, c_f, c_f, c_p, c_p])
     sig("blitz_gla_chunk_supported", [c_i, c_i, c_i], c_i)
     sig("blitz_conv_causal", [c_p, c_i64, c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_i, c_p, c_i,
@@ -133,7 +134,7 @@ def _declare(L: ctypes.CDLL) -> None:
                              c_p, c_i, c_p])
     sig("blitz_wkv_recurrent", [c_p, c_p, c_p, c_p, c_i64, c_p, c_i64, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_p, c_i, c_i, c_i,
                                 c_i, c_i, c_i, c_f, c_i, c_p, c_i, c_p])
-    sig("blitz_wkv_chunk", [c_p, c_p, c_p, c_p, c_i64, c_p, c_i64, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_p, c_i, c_i, c_i,
+    sig("blitz_wkv_chunk", [c_p, c_p, c_p, c_p, c_i64, c_p, c_i64, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_i64, c_p, c_p, c_p, c_i, c_i, c_i,
                             c_i, c_i, c_i, c_i, c_f, c_p, c_p])
     ssd = [c_p, c_p, c_p, c_i64, c_p, c_p, c_i64, c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_p]
     sig("blitz_ssd_recurrent", ssd + [c_i, c_p])
