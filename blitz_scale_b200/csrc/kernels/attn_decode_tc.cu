@@ -316,7 +316,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   if (warp >= 8) {
     // ------------------------------------------------------------ producer (a whole warp; one lane issues)
     // A TMA box can only be issued once its page id is known, and a page id read from global memory right before
-    // the issue costs one memory latency per chunk, which by itself caps the stream near 50 GB/s per SM.  So the
+    // the issue costs one memory latency per chunk, which by itself is more than HBM's time for the chunk.  So the
     // warp reads page ids 32 at a time (one coalesced load, lane l keeps entry l of the window), hands them out by
     // shuffle, and requests the next item's page-table window and lengths while the current item streams.
     const int ps = p.page_size;

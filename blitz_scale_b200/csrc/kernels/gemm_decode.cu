@@ -10,8 +10,9 @@
 //    the instruction's N (16..256, M rounded up to 16).  One instruction covers the whole batch, and a
 //    small batch costs a small instruction instead of a 128-row tile that is mostly padding.  The
 //    accumulator in TMEM holds C transposed: lane = output feature, column = token.
-//  * A single SM cannot pull more than ~50 GB/s through TMA (measured), so HBM is only saturated when
-//    ~128 or more SMs stream.  Matrices with fewer than that many 128-feature tiles therefore split K
+//  * HBM's 6.5 TB/s are 44 GB/s for each of 148 SMs, and one loading thread that fills a K block of 16 KB in
+//    about 440 cycles (elected by elect.sync; 640 behind `lane == 0`) reaches some 70, so HBM is only
+//    saturated when most SMs stream.  Matrices with fewer than that many 128-feature tiles therefore split K
 //    over a thread-block cluster: the `split` CTAs of a cluster work on the same tile, each on 1/split
 //    of K.  The reduction never touches global memory: after a cluster barrier every CTA stores its fp32
 //    accumulator, slice by slice, straight into the shared memory of the CTA that owns that slice of

@@ -5,9 +5,9 @@
 //
 // Why a pair.  At 129..256 rows a decode GEMM sits on the ridge of the roofline: the weight stream and the
 // tensor pipe take the same time, and every weight tile drags an activation tile of its own size out of L2.
-// Measured on B200, the sum of those two streams is what bounds such a GEMM (the L2 -> SM fabric delivers about
-// 10 TB/s to all SMs together, the weight stream alone could run at 6.5), and a single CTA is additionally bound
-// by shared-memory operand reads of a 128-row tcgen05.mma.  Two CTAs of a 2-wide cluster issue ONE
+// A loading thread needs about 440 cycles for a K block whatever its bytes, so what one CTA has to fetch per
+// product bounds such a GEMM, and a single CTA is additionally bound by shared-memory operand reads of a 128-row
+// tcgen05.mma.  Two CTAs of a 2-wide cluster issue ONE
 // `tcgen05.mma.cta_group::2` of 256 rows: each CTA keeps 128 rows of A and half of the N columns of the weight
 // tile, so per SM the operand reads and the activation re-read are halved.  With two accumulators per pair
 // (a "super tile" of 2 x 256 columns that shares every activation tile) the re-read halves again.
