@@ -70,7 +70,7 @@ struct GlaChunkParams {
 // that is zero); entry j: what segment j - 1 adds to the state, and the sum of its log decays (the first one: the state behind it).
 struct GcSegment {
   int row, seg, num, beg, len, t_row;  // beg, len: its tokens; t_row: the row's first
-  int64_t entry;                       // of entry 0: rows of n segments are n entries apart at least
+  int64_t entry;                       // of entry 0; two entries for every `tokens` tokens: enough for a row of more than one segment
   __device__ GcSegment(const GlaChunkParams& p, int z) {
     row = z % p.rows;
     seg = z / p.rows;
@@ -81,7 +81,7 @@ struct GcSegment {
     if (p.seg_chunks > 0) {
       const int tokens = p.seg_chunks * kGcC;
       num = (len + tokens - 1) / tokens;
-      entry = beg / tokens + row;
+      entry = 2 * static_cast<int64_t>(beg) / tokens;
       beg += seg * tokens;
       len = min(tokens, len - seg * tokens);
     }
@@ -832,7 +832,7 @@ static int gla_chunk_any(GlaChunkParams& p, int rows, int max_len, int64_t token
     p.seg_chunks = gla_segment_chunks(tokens, rows, max_len, p.heads, p.vdim, sms);
     if (p.seg_chunks > 0) {
       p.seg_state = static_cast<float*>(seg);
-      p.seg_decay = p.seg_state + (tokens / (p.seg_chunks * kGcC) + rows) * p.heads * p.dim * p.vdim;
+      p.seg_decay = p.seg_state + 2 * tokens / (p.seg_chunks * kGcC) * p.heads * p.dim * p.vdim;
     }
   }
   if (p.heads > 65535 || rows > 65535 || (p.row & 7) || (p.out_stride & 1)) return -1;
@@ -869,10 +869,11 @@ int blitz_gla_chunk_supported(int dim, int vdim, int rank) {
          rank <= kGdMaxRank;
 }
 
-// Bytes of the scratch `seg` for `tokens` tokens (16-byte aligned; tok_indptr ends at `tokens` at most); 0: the rows are not cut.
+// Bytes of the scratch `seg` for `tokens` tokens (16-byte aligned; tok_indptr ends at `tokens` at most), 45 MB at most; 0: the rows are
+// not cut.
 int64_t blitz_gla_chunk_scratch(int64_t tokens, int rows, int max_len, int heads, int dim, int vdim) {
   const int cut = gla_segment_chunks(tokens, rows, max_len, heads, vdim, device_sm_count());
-  return cut == 0 ? 0 : (tokens / (cut * kGcC) + rows) * heads * dim * (vdim + 1) * (int64_t)sizeof(float);
+  return cut == 0 ? 0 : 2 * tokens / (cut * kGcC) * heads * dim * (vdim + 1) * (int64_t)sizeof(float);
 }
 
 // Rows of at least one token each: tokens tok_indptr[r] .. tok_indptr[r + 1]; max_len: the longest row.  cum: fp32 scratch
