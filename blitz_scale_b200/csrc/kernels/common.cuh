@@ -90,6 +90,14 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   __syncthreads();
   return red[32];
 }
+// The same with a single barrier; `red` must not be in use by anything before that barrier.
+__device__ __forceinline__ float block_sum1(float v, float* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  v = warp_sum(v);
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  return warp_sum(lane < nw ? red[lane] : 0.f);
+}
 // The same for two numbers with a single barrier; `red` must not be in use by anything before that barrier.
 __device__ __forceinline__ float2 block_sum2(float a, float b, float2 (&red)[32]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
