@@ -96,6 +96,7 @@ class LlamaRunner:
         self.tokens = torch.empty(max_batch, dtype=torch.int32, device=dev)
         self.maxval = torch.empty(max_batch, dtype=torch.float32, device=dev)
         self._ws = {}
+        self._ws_old: List[Optional[torch.Tensor]] = []
 
     # ------------------------------------------------------------------ pieces
     def _w(self, l: int, name: str) -> torch.Tensor:
@@ -116,8 +117,10 @@ class LlamaRunner:
         key = splits == 0               # shares of all keys: the kernel's tickets in it stay zero
         ws = self._ws.get(key)
         if ws is None or ws.numel() < n:
-            ws = torch.zeros(n, dtype=torch.uint8, device=self.res.device)
-            self._ws[key] = ws
+            # an earlier buffer may be named by captured graphs: keep it (parts of a batch are a few hundred at most, 17 KB each for 32
+            # heads of 128)
+            self._ws_old.append(ws)
+            ws = self._ws[key] = torch.zeros(n, dtype=torch.uint8, device=self.res.device)
         return ws
 
     def attention_block(self, l: int, m: StepMeta) -> None:
