@@ -119,7 +119,7 @@ def measure_tp_replica(args, world, rank, barrier, owners):
         for _ in range(warmup):
             eng.decode(batch)
         Bp = min(b for b in _BUCKETS if b >= B)
-        splits = eng.choose_splits(Bp, batch.max_seq_len(), batch.num_pages() * eng.page_size)
+        splits = eng.choose_splits(B, batch.max_seq_len(), batch.num_pages() * eng.page_size)
         graph = eng._graphs.get((Bp, splits)) or eng._capture(Bp, splits)
         for _ in range(warmup):
             graph.replay()
@@ -299,7 +299,7 @@ def main():
 
     # ---------------- kernel-only: replay the captured step
     Bp = min(b for b in __import__("blitz_scale_b200.runtime.engine", fromlist=["_BUCKETS"])._BUCKETS if b >= B)
-    splits = eng.choose_splits(Bp, batch.max_seq_len(), batch.num_pages() * eng.page_size)
+    splits = eng.choose_splits(B, batch.max_seq_len(), batch.num_pages() * eng.page_size)
     graph = eng._graphs.get((Bp, splits)) or eng._capture(Bp, splits)
     for _ in range(args.warmup):
         graph.replay()

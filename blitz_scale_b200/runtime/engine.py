@@ -135,10 +135,11 @@ class Engine:
         return b
 
     def choose_splits(self, B: int, max_len: int, tokens: int = 0) -> int:
-        """How decode attention divides the keys of B sequences, the longest of max_len and `tokens` in all (0: not known).  0: equal
+        """How decode attention divides the keys of B sequences (rows of padding not counted), the longest of max_len and `tokens` in all
+        (0: not known).  0: equal
         ranges of all of them, whatever the lengths.  Sequences of about one length need no ranges, whose pieces cost a fence, a ticket
         and a merge inside the kernel: few of them are cut into as many parts as fill the SMs (16 x 1001 tokens, 8 KV heads: 15 us
-        instead of 20), many stay whole.  A batch has no more than two choices, so that it needs no more than two graphs."""
+        instead of 20), many stay whole."""
         if self.cfg.family == "hybrid":
             kv_heads, max_len = self.cfg.attention_work(max_len)
             if kv_heads == 0:
@@ -239,7 +240,7 @@ class Engine:
             raise ValueError(f"decode batch of {B} sequences exceeds max_batch={self.max_batch}")
         Bp = _bucket(B) if self.use_graphs else B
         Bp = min(Bp, self.max_batch)
-        splits = self.choose_splits(Bp, batch.max_seq_len(), batch.num_pages() * self.page_size)
+        splits = self.choose_splits(B, batch.max_seq_len(), batch.num_pages() * self.page_size)
         P = batch.fill_decode(self.host_np, self.layout, Bp)
         self._h2d(self.layout.page_indices + P)
         if self.use_graphs:
@@ -303,7 +304,7 @@ class Engine:
         self._h2d(self.layout.page_indices + P)
         row_of = {b: r for r, b in enumerate(order)}
         if single:
-            splits = self.choose_splits(pad, max(kv_lens), sum(kv_lens))
+            splits = self.choose_splits(rows_max, max(kv_lens), sum(kv_lens))
             if self.use_graphs:
                 (self._graphs.get((pad, splits)) or self._capture(pad, splits)).replay()
             else:
@@ -397,11 +398,11 @@ class Engine:
         limit = min(max_batch or self.max_batch, self.max_batch)
         empty = core.Batch((1 << 62), self.pool)
         n = 0
-        for Bp in _BUCKETS:
+        for below, Bp in zip([0] + _BUCKETS, _BUCKETS):
             if Bp > limit:
                 break
-            for ctx, tokens in [(c, t) for c in contexts for t in (0, Bp * c)]:
-                splits = self.choose_splits(Bp, ctx, tokens)
+            # every number of sequences that this bucket serves, of one length and as unequal as they can be
+            for splits in sorted({self.choose_splits(n, c, t) for n in range(below + 1, Bp + 1) for c in contexts for t in (n * c, c + n - 1)}):
                 if (Bp, splits) in self._graphs:
                     continue
                 P = empty.fill_decode(self.host_np, self.layout, Bp)      # Bp padded rows: no page, no cache write
