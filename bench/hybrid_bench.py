@@ -74,7 +74,7 @@ def bench_models(out, sizes=("h4096", "h2048"), configs=configs):
                 b.append_tokens(torch.randint(0, VOCAB, (B,), generator=g).tolist(), False)   # (they choose experts)
                 P = b.fill_decode(eng.host_np, eng.layout, _bucket(B))
                 eng._h2d(eng.layout.page_indices + P)
-                graph = eng._capture(_bucket(B), eng.choose_splits(_bucket(B), b.max_seq_len()))
+                graph = eng._capture(_bucket(B), eng.choose_splits(B, b.max_seq_len(), b.num_pages() * eng.page_size))
                 t = _median(graph.replay, n=15)
                 ops.check_status()
                 b.clear()

@@ -134,10 +134,9 @@ class Engine:
             return None
         return b
 
-    def choose_splits(self, B: int, max_len: int, tokens: int = 0) -> int:
-        """How decode attention divides the keys of B sequences (rows of padding not counted), the longest of max_len and `tokens` in all
-        (0: not known).  0: equal
-        ranges of all of them, whatever the lengths.  Sequences of about one length need no ranges, whose pieces cost a fence, a ticket
+    def choose_splits(self, B: int, max_len: int, tokens: int) -> int:
+        """How decode attention divides the keys of B sequences (rows of padding not counted), the longest of max_len and `tokens` in
+        all.  0: equal ranges of all of them, whatever the lengths.  Sequences of about one length need no ranges, whose pieces cost a fence, a ticket
         and a merge inside the kernel: few of them are cut into as many parts as fill the SMs (16 x 1001 tokens, 8 KV heads: 15 us
         instead of 20), many stay whole."""
         if self.cfg.family == "hybrid":

@@ -1,10 +1,13 @@
 """How a decode step divides its keys: the rule, and what the engine asks it (no GPU)."""
+import pathlib
 import types
 
 import pytest
 
 from blitz_scale_b200.models.config import get_config
 from blitz_scale_b200.runtime import engine as E
+
+ROOT = pathlib.Path(__file__).resolve().parents[1]
 
 
 def test_rows_of_padding_do_not_count():
@@ -45,3 +48,10 @@ def test_captures_cover_what_a_step_may_choose():
             for tokens in (n * length, length + n - 1):
                 assert (E._bucket(n), eng.choose_splits(n, length, tokens)) in eng._graphs
     assert max(sum(rows == b for rows, _ in eng._graphs) for b in E._BUCKETS) <= 4
+
+
+def test_every_caller_says_how_many_tokens():
+    with pytest.raises(TypeError):
+        E.Engine.choose_splits(E.Engine.__new__(E.Engine), 1, 1000)
+    calls = [line for f in (ROOT / "bench.py", *(ROOT / "bench").glob("*.py")) for line in f.read_text().splitlines() if "choose_splits(" in line]
+    assert calls and all("page_size" in line for line in calls)
