@@ -31,7 +31,7 @@ from __future__ import annotations
 
 import math
 from dataclasses import dataclass
-from typing import Dict, List, Optional, Tuple, Union
+from typing import Dict, List, Optional, Sequence, Tuple, Union
 
 import torch
 
@@ -654,10 +654,10 @@ class HybridConfig:
                 n += 4 * m.width + elem * (m.taps - 1) * m.width
         return n
 
-    def attention_work(self, length: int) -> Tuple[int, int]:
-        """(KV heads, positions) of the attention run with the fewest heads and of the one that looks furthest back, for a
-        sequence of `length` tokens: what the number of key splits is chosen from.  (0, 0) without attention."""
-        a = [m for m in self.run_parts() if m.kind in PAGED]
+    def attention_work(self, length: int, kinds: Sequence[str] = PAGED) -> Tuple[int, int]:
+        """(KV heads, positions) of the attention run (of these kinds) with the fewest heads and of the one that looks furthest
+        back, for a sequence of `length` tokens: what the number of key splits is chosen from.  (0, 0) without attention."""
+        a = [m for m in self.run_parts() if m.kind in kinds]
         if not a:
             return 0, 0
         span = max(min(length, m.window + getattr(m, "keep_first", 0)) if getattr(m, "window", 0) else length for m in a)

@@ -34,6 +34,38 @@ def _bucket(n: int) -> int:
     return n
 
 
+def decode_parts(rows: int, kv_heads: int, longest: int, tokens: int) -> int:
+    """How decode attention divides the keys of `rows` sequences, `tokens` in all, the longest of `longest`: 1: every sequence whole; n:
+    into n parts each; 0: equal ranges of all of them, whatever their lengths.
+
+    One of the 296 halves of the SMs takes a chunk of 64 keys in 0.7 us until they wait for HBM (all of them at work: 1.5 us).  Parts cost
+    a merge kernel, 2.8 us, so they have to save seven chunks, and more where they bring second halves of SMs to work: those start late
+    and share what their SM is given.  Ranges cost 7 us (pieces, tickets, merges), so they pay where the end of a launch would
+    otherwise leave most halves idle for longer than that.  Measured behind a small kernel, us, KV heads of 128, whole / parts / ranges
+    (* chosen):
+      8 heads, 1 sequence of 300, 500, 1000, 100k tokens:  7.8* / 9.2 (4) / 9.2,  9.9 / 8.7 (8)* / 9.2,  15.8 / 9.6 (16)* / 10.8,
+        1085 / 72 (32)* / 76;  1 head, 100k: 1084 / 44 (32)* / 55
+      8 heads, 3, 12, 18 and 25 of 1000:  16.1 / 11.8 (4)* / 15.0,  16.7* / 17.7 (2) / 23.0,  18.4* / 22.6 (2) / 26.5,  23.7* / - / 30.9
+      8 heads, 38, 150 and 256 of 1000:  41.8 / - / 37.7*,  109.3 / - / 107.7*,  168.7* / - / 172.3
+      8 heads, unequal, 5 up to 1000, 16 up to 16k:  15.9 / 13.6 (2)* / 20.1,  180 / 123 (2) / 105*;  61 up to 300, 600 and 4000:
+        17.9* / - / 24.2,  25.7* / - / 30.8,  102.7 / - / 92.2*"""
+    items, chunks = rows * kv_heads, -(-longest // 64)
+    shared = rows <= ops.ATTN_DECODE_SHARED_ROWS
+    equal = 4 * rows * longest <= 5 * tokens
+    for parts in (32, 16, 8, 4, 2):
+        n, part = items * parts, -(-chunks // parts)
+        fits = n <= 128 and (parts <= 16 or part > 1) or n <= 192 and part >= (16 if parts == 2 else 8) or n <= 256 and part >= 16
+        if fits and parts <= chunks and chunks - part >= 7:
+            return parts if equal or part <= 60 or not shared else 0
+    if items <= 296:         # (in chunks at the full rate of HBM: what the longest one takes beyond an equal share)
+        late = 174 * chunks - kv_heads * tokens // 64 > 2500
+    elif equal:              # how much of the last round has nothing to do
+        late = chunks * (136 - (items - 1) % 296) > 1200
+    else:
+        late = chunks > 20
+    return int(not (late and shared))
+
+
 class Engine:
     def __init__(self, model: str | ModelConfig, *, num_pages: int, page_size: int = 64, max_batch: int = 256,
                  max_batch_tokens: int = 8192, tp: int = 1, tp_rank: int = 0, dtype=torch.bfloat16,
@@ -134,32 +166,18 @@ class Engine:
             return None
         return b
 
-    def choose_splits(self, B: int, max_len: int, tokens: int) -> int:
-        """How decode attention divides the keys of B sequences (rows of padding not counted), the longest of max_len and `tokens` in
-        all.  0: equal ranges of all of them, whatever the lengths.  Sequences of about one length need no ranges, whose pieces cost a fence, a ticket
-        and a merge inside the kernel: few of them are cut into as many parts as fill the SMs (16 x 1001 tokens, 8 KV heads: 15 us
-        instead of 20), many stay whole."""
+    def choose_splits(self, rows: int, max_len: int, tokens: int) -> int:
+        """How decode attention divides the keys of `rows` sequences (rows of padding not counted), the longest of max_len and `tokens`
+        in all: see decode_parts."""
         if self.cfg.family == "hybrid":
-            kv_heads, max_len = self.cfg.attention_work(max_len)
+            # (latent attention divides its keys by itself)
+            kv_heads, max_len = self.cfg.attention_work(max_len, ("attention",))
             if kv_heads == 0:
                 return 1
+            tokens = min(tokens, rows * max_len)
         else:
             kv_heads = self.cfg.kv_heads // self.tp
-        if B <= ops.ATTN_DECODE_SHARED_ROWS:
-            if 4 * B * max_len > 5 * tokens:
-                return 0
-            if B * kv_heads <= 148:
-                return 1 << min(4, (2 * 148 // (B * kv_heads)).bit_length() - 1)
-            return int(B * kv_heads >= 8 * 148)
-        ctas = B * kv_heads
-        if ctas >= 2 * 148 or max_len <= 256:
-            return 1
-        want = (2 * 148 + ctas - 1) // ctas
-        cap = max(1, max_len // 256)
-        s = 1
-        while s * 2 <= min(want, cap, 32):
-            s *= 2
-        return s
+        return decode_parts(rows, kv_heads, max_len, tokens)
 
     # ------------------------------------------------------------------ steps
     @torch.no_grad()
@@ -386,7 +404,7 @@ class Engine:
         self._graphs[(Bp, splits)] = g
         return g
 
-    def precapture(self, max_batch: Optional[int] = None, contexts: Sequence[int] = (64, 1024, 4096, 16384)) -> int:
+    def precapture(self, max_batch: Optional[int] = None, contexts: Sequence[int] = (64, 512, 1024, 4096, 16384)) -> int:
         """Capture the decode graphs of every batch bucket up to `max_batch` (default: the engine's) and of the
         split-KV choices that contexts of the given lengths select, so that no request pays for a capture later.
         The captures run on padded rows only (an empty batch): graph topology and buffer addresses do not depend
