@@ -10,7 +10,7 @@
 // A K block of a whole tile takes 300 ns of UMMAs and, beside them, 240 ns of loads once one elected thread issues two loads (three
 // from a `lane == 0` branch: 345 ns).  Measured on the products of a Llama-3-8B layer, us (before: gemm_tcgen05.cu, also elected):
 //   M = 8192: 6144 x 4096 321 -> 265, 4096 x 4096 222 -> 197, gate and up 1623 -> 1373;  cuBLAS 316 / 227 / 1424 (without SiLU)
-//   M = 1574: 75 -> 64, 55 -> 46, 293 -> 257, 4096 x 14336 188 -> 165;  cuBLAS 55 / 36 / 267 / 118
+//   M = 1574: 75 -> 64, 55 -> 46, 293 -> 257 (before the division in SiLU was exact), 4096 x 14336 188 -> 165;  cuBLAS 55 / 36 / 267 / 118
 //
 // Tiles are handed out in rounds of one per pair, `group_m` row tiles by all column tiles at a time, so that the pairs working at
 // the same moment share rows and columns in L2.  The last, incomplete round is cut into tiles of half the columns where these fit
@@ -347,6 +347,13 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         if (EPI == kEpiClampGlu) {
           float y[32];
           clamp_glu32<T>(reinterpret_cast<const T*>(p.R), p.up_col_off, n + ch * 32, p.N, p.alpha, p.beta, g, up, y);
+          pair_convert32<T, 0>(y, up, res[s], o4);
+        } else if (EPI == 2) {
+          // divided as IEEE does: __fdividef is off by two units and answers zero for denominators beyond 2^126 (14336 x 4096 with it and
+          // so, us: 300 rows 84.5 and 88.3, 1574 rows 264.5 and 272.0, within the spread at 8192)
+          float y[32];
+#pragma unroll
+          for (int k = 0; k < 32; ++k) y[k] = g[k] / (1.f + __expf(-g[k])) * up[k];
           pair_convert32<T, 0>(y, up, res[s], o4);
         } else {
           pair_convert32<T, EPI>(g, up, res[s], o4);

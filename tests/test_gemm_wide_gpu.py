@@ -53,3 +53,20 @@ def test_diagonal_blocks(M, f32):
         got = out[:, i * (N + 16):(i + 1) * (N + 16)]
         assert float(((got[:, :N].float() - want).abs() - (1e-5 if f32 else 2.0 ** -8) * want.abs()).max()) <= 2e-5 * K ** 0.5
         assert bool((got[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M", [129, 300, 1574])
+def test_silu_of_large_negative_gates(M):
+    """Denominators beyond 2^126, where an approximate division answers zero."""
+    from blitz_scale_b200 import ops
+    N, K = 192, 64
+    gates = torch.cat([torch.linspace(-88.5, -80.0, 96), torch.linspace(-20.0, 20.0, 96)]).to(torch.bfloat16)
+    w = torch.zeros(K, 2 * N, dtype=torch.bfloat16, device=DEV)
+    w[0, :N], w[0, N:] = gates.to(DEV), 2.0 ** 100
+    a = torch.zeros(M, K, dtype=torch.bfloat16, device=DEV)
+    a[:, 0] = 1
+    got = ops.gemm(a, w, epilogue="silu_mul", wide_path=True).double()
+    g = gates.double().to(DEV)
+    want = (g / (1 + torch.exp(-g)) * 2.0 ** 100).expand(M, N)
+    # one rounding to bf16; the exponential of fp32 numbers is off by 2 + 1.16 |x| units of fp32
+    assert bool(((got - want).abs() <= want.abs() * (2.0 ** -8 + 110 * 2.0 ** -23)).all())
