@@ -9,6 +9,7 @@ cache ``[page][K|V][token][kv_head][head_dim]`` per layer.
 from __future__ import annotations
 
 import ctypes
+import threading
 from typing import NamedTuple, Optional, Sequence, Union
 
 import torch
@@ -91,21 +92,29 @@ def _gate(gate: Optional[torch.Tensor]):
     return _p(gate), 0 if gate is None else gate.stride(0)
 
 
+_first_use = threading.RLock()
+
+
+def _once(table: dict, key, make):
+    """table[key], made by the first thread that asks for it: kernels are handed its address, so there must be only one."""
+    if key not in table:
+        with _first_use:
+            if key not in table:
+                table[key] = make()
+    return table[key]
+
+
 def status_word(device=None) -> torch.Tensor:
     """Per-device int32 word the kernels write a non-zero code into when a bounded wait or an index check fails."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    key = (dev.type, dev.index)
-    if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32, device=dev)
-    return _status[key]
+    return _once(_status, (dev.type, dev.index), lambda: torch.zeros(1, dtype=torch.int32, device=dev))
 
 
 def _status_ptr(t: torch.Tensor) -> int:
     """Address of the status word of a tensor's device."""
-    index = t.get_device()
-    word = _status_by_index.get(index)
+    word = _status_by_index.get(t.get_device())
     if word is None:
-        word = _status_by_index[index] = status_word(t.device)
+        word = _once(_status_by_index, t.get_device(), lambda: status_word(t.device))
     return word.data_ptr()
 
 
@@ -142,24 +151,20 @@ PAIR_GEMM_MAX_M = 256
 def gemm_workspace(device=None):
     """Per-device scratch of the split-K path: (fp32 partials as bytes, zeroed uint32 tickets)."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    key = (dev.type, dev.index)
-    if key not in _gemm_ws:
-        n = int(lib().blitz_gemm_workspace_bytes(148))
-        _gemm_ws[key] = (torch.empty(n, dtype=torch.uint8, device=dev),
-                         torch.zeros(GEMM_TICKETS, dtype=torch.int32, device=dev))
-    return _gemm_ws[key]
+    return _once(_gemm_ws, (dev.type, dev.index),
+                 lambda: (torch.empty(int(lib().blitz_gemm_workspace_bytes(148)), dtype=torch.uint8, device=dev),
+                          torch.zeros(GEMM_TICKETS, dtype=torch.int32, device=dev)))
 
 
 def pair_gemm_workspace(device=None):
     """Per-device scratch of the paired-SM GEMM: (fp32 partials as bytes, zeroed uint32 counters, eight per tile)."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    key = (dev.type, dev.index)
-    if key not in _pair_ws:
+
+    def make():
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
-        n = int(lib().blitz_gemm_pair_workspace_bytes(sms))
-        _pair_ws[key] = (torch.empty(n, dtype=torch.uint8, device=dev),
-                         torch.zeros(PAIR_FLAGS, dtype=torch.int32, device=dev))
-    return _pair_ws[key]
+        return (torch.empty(int(lib().blitz_gemm_pair_workspace_bytes(sms)), dtype=torch.uint8, device=dev),
+                torch.zeros(PAIR_FLAGS, dtype=torch.int32, device=dev))
+    return _once(_pair_ws, (dev.type, dev.index), make)
 
 
 class _GemmScratch(ctypes.Structure):
@@ -173,13 +178,13 @@ _gemm_scratch = {}
 
 def _scratch_of(index: int) -> int:
     """Address of the record of a device's product scratch (what blitz_gemm_any takes)."""
-    if index not in _gemm_scratch:
+    def make():
         dev = torch.device("cuda", index)
         (ws, tickets), (pair, flags) = gemm_workspace(dev), pair_gemm_workspace(dev)
         record = _GemmScratch(ws.data_ptr(), ws.numel(), tickets.data_ptr(), tickets.numel(), pair.data_ptr(), pair.numel(), flags.data_ptr(),
                               flags.numel(), status_word(dev).data_ptr())
-        _gemm_scratch[index] = (ctypes.addressof(record), record)
-    return _gemm_scratch[index][0]
+        return ctypes.addressof(record), record
+    return (_gemm_scratch.get(index) or _once(_gemm_scratch, index, make))[0]
 
 
 def _tensor_core_operands(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, N: int, K: int) -> bool:
