@@ -184,6 +184,8 @@ class HybridRunner:
     def run_layer(self, r: int, m: StepMeta) -> None:
         """Layer run `r` (an index into the executions of a pass, not a layer number)."""
         run, T, c = self.runs[r], m.num_tokens, self.cfg
+        if r == 0:
+            self._expanded = None        # (the step's lengths and pages may be others than in a pass before)
         l = run.layer
         spec = c.layer_specs[l]
         if c.streams:
@@ -427,7 +429,7 @@ class HybridRunner:
             self._expanded[1][key] = (both[:len(index)], m.page_indices.index_select(0, both[len(index):]), len(need))
         return self._expanded[1][key]
 
-    _expanded: Optional[tuple] = None       # (step, tables) of the last prefill pass
+    _expanded: Optional[tuple] = None       # (step, tables) of the prefill pass that is running
     EXPANDED_BYTES = 1 << 30      # of expanded keys and values at a time
 
     def _room(self, name: str, shape: tuple, dt) -> torch.Tensor:
