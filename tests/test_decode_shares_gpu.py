@@ -90,3 +90,48 @@ def test_shares_of_all_keys(case, dt):
             got = out[b, h * dv:(h + 1) * dv].float()
             big = float(want.abs().max()) + float(v.abs().max()) * (0.1 if not kw.get("sigmoid") else 1.0)
             assert float((got - want).abs().max()) <= 3 * unit * big, (b, h)
+
+
+def test_one_workspace_for_all_launches():
+    """Launches of other batches, lengths and heads share a workspace, eagerly and in a graph: each leaves its tickets zero, and results
+    repeat bit for bit.  The page tables are read before the kernel in front has finished."""
+    from blitz_scale_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).to(torch.bfloat16)
+    calls, size = [], 0
+    for lens, H, G, d, page in [([978], 32, 8, 128, 64), ([3, 700, 64, 65, 0, 2049, 1], 16, 4, 128, 64), ([900, 130, 1], 8, 4, 64, 64),
+                                ([30 + 7 * i for i in range(256)], 4, 2, 64, 64), ([0, 0, 5, 0], 8, 2, 64, 16), ([600, 33, 1500], 12, 1, 64, 32)]:
+        used = [-(-n // page) for n in lens]
+        kv, q = rnd(sum(used) + 1, 2, page, G, d), rnd(len(lens), H * d)
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+        tables = (torch.randperm(sum(used) + 1, device=DEV, generator=g).to(torch.int32), i32([sum(used[:i]) for i in range(len(lens) + 1)]),
+                  i32([n - (u - 1) * page if n else 0 for n, u in zip(lens, used)]))
+        calls.append((q, kv, tables, dict(q_heads=H, kv_heads=G, head_dim=d, page_size=page, num_splits=0, static_table=True)))
+        size = max(size, ops.attn_decode_workspace_bytes(len(lens), H, d, 0))
+    want = [ops.attn_decode(q, kv, *t, **kw) for q, kv, t, kw in calls]              # (a fresh workspace each)
+    ws = torch.zeros(size, dtype=torch.uint8, device=DEV)
+    tickets = ws[:256 * 128 * 4]
+    outs = [torch.full_like(w, 7.0) for w in want]
+    norm_in, norm_w, norm_out = rnd(256, 4096), torch.ones(4096, dtype=torch.bfloat16, device=DEV), torch.empty(256, 4096, dtype=torch.bfloat16, device=DEV)
+
+    def body():
+        for (q, kv, t, kw), out in zip(calls, outs):
+            ops.rms_norm(norm_in, norm_w, 1e-5, out=norm_out)                         # a kernel to run beside
+            ops.attn_decode(q, kv, *t, workspace=ws, out=out, **kw)
+
+    def same():
+        ops.check_status()
+        assert not bool(tickets.any())
+        for out, w in zip(outs, want):
+            assert torch.equal(out, w)
+            out.fill_(7.0)
+    for _ in range(2):
+        body()
+        same()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        body()
+        body()
+    for _ in range(3):
+        graph.replay()
+        same()
