@@ -4,6 +4,7 @@
     python bench/ncu_case.py attn_decode B CTX            # 3 launches of the paged decode attention
     python bench/ncu_case.py experts T                    # 3 rounds of router, grouped up and grouped down product
     python bench/ncu_case.py latent B CTX                 # 3 launches of latent decode attention, and of stream_mix over B * CTX / 32 tokens
+    python bench/ncu_case.py linear_attention N ...       # 3 launches of chunked linear attention over rows of these lengths
     python bench/ncu_case.py attn_prefill_paged B N       # 3 launches of the paged prefill attention (64-token pages)
 """
 import os
@@ -75,6 +76,17 @@ def main():
         for _ in range(3):
             ops.attn_latent(q, kv, idx, indptr, last, heads=h, scale=W ** -0.5, workspace=ws, out=o, gate=gate)
             ops.stream_mix(x, pending=pending, read=norm[2][:S].contiguous(), norm=norm, out=hh, write=True)
+    elif kind == "linear_attention":
+        lens, heads, dim, vdim, rank = list(map(int, sys.argv[2:])), 16, 128, 256, 16
+        T, hk, hv = sum(lens), heads * dim, heads * vdim
+        rnd = lambda *s: torch.randn(*s, device="cuda", dtype=torch.bfloat16)
+        q, k, v, g, low = rnd(T, 2 * hk + 2 * hv + rank).split([hk, hk, hv, hv, rank], 1)
+        a2, a2_b, norm = rnd(rank, hk) * rank ** -0.5, rnd(hk), torch.ones(vdim, device="cuda", dtype=torch.bfloat16)
+        state, out = torch.zeros(len(lens), heads, dim, vdim, device="cuda"), rnd(T, hv)
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+        pos, ends, slots = i32([t for n in lens for t in range(n)]), i32([sum(lens[:i]) for i in range(len(lens) + 1)]), i32(range(len(lens)))
+        for _ in range(3):
+            ops.gla(q, k, v, g, low, a2, a2_b, norm, state, out, pos, ends, slots, rank=rank, tau=16.0, eps=1e-5, row_lens=lens)
     elif kind == "decode_step":
         # two eager decode steps of the full model (no CUDA graph), for a per-kernel launch list of one step:
         #   ncu --metrics gpu__time_duration.sum -k regex:"blitz|gemm|attn|rms|rope|argmax|embedding|sample" ...

@@ -14,8 +14,8 @@ int blitz_gemm_decode(const void*, int64_t, const void*, int64_t, void*, int64_t
                       float, float, cudaStream_t);
 int blitz_gemm_pair(const void*, int64_t, const void*, int64_t, void*, int64_t, const void*, int, int, int, int, int, int, int, int, int, int,
                     void*, int64_t, unsigned*, int, int*, float, float, cudaStream_t);
-int blitz_gemm_wide(const void*, int64_t, const void*, int64_t, void*, int64_t, const void*, int, int, int, int, int, int, int, int, int,
-                    int*, float, float, int, int, int, cudaStream_t);
+int blitz_gemm_wide(const void*, int64_t, const void*, int64_t, void*, int64_t, const void*, int, int, int, int, int, int, int, int*,
+                    float, float, int, int, int, cudaStream_t);
 
 // Scratch of one device, as the kernels' own entry points describe it.
 struct BlitzGemmScratch {
@@ -54,8 +54,8 @@ int blitz_gemm_any(const void* A, int64_t lda, const void* B, int64_t ldb, void*
       return blitz_gemm_pair(A, lda, B, ldb, C, ldc, R, M, N, K, epilogue, up_col_off, dtype, static_b, 0, 0, 0, s->pair_ws, s->pair_bytes,
                              s->pair_flags, (int)s->num_pair_flags, s->status, alpha, beta, stream);
     case 3:
-      return blitz_gemm_wide(A, lda, B, ldb, C, ldc, R, M, N, K, epilogue, up_col_off, dtype, static_b, 0, 0, s->status, alpha, beta, groups,
-                             a_step, c_step, stream);
+      return blitz_gemm_wide(A, lda, B, ldb, C, ldc, R, M, N, K, epilogue, up_col_off, dtype, static_b, s->status, alpha, beta, groups, a_step,
+                             c_step, stream);
     default:
       return blitz_gemm(A, lda, B, ldb, C, ldc, R, M, N, K, 0, epilogue, up_col_off, dtype, 0, 0, s->ws, s->ws_bytes, s->tickets,
                         (int)s->num_tickets, s->status, alpha, beta, groups, a_step, c_step, stream);

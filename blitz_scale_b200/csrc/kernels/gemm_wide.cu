@@ -427,12 +427,11 @@ int blitz_gemm_wide_supported(int M, int N, int K, int b_layout, int epilogue, i
          (K & 7) == 0 && N >= 64 && (groups == 1 || ((epilogue == 0 || epilogue == 4) && K % blitz::kWideBK == 0 && N % 64 == 0));
 }
 
-// C = A W with the epilogues, pitches and diagonal blocks of blitz_gemm (N, K: of one block).  narrow: 1 = all tiles of half the
-// columns, 0 = choose, -1 = whole tiles only; group_m: row tiles that share a pass over the columns (0 = choose).
+// C = A W with the epilogues, pitches and diagonal blocks of blitz_gemm (N, K: of one block).
 // Returns a cudaError_t value, -1 for arguments it cannot take, -2 when the TMA encoder is missing.
 int blitz_gemm_wide(const void* A, int64_t lda, const void* W, int64_t ldb, void* C, int64_t ldc, const void* R, int M, int N, int K,
-                    int epilogue, int up_col_off, int dtype, int static_b, int narrow, int group_m, int* status, float alpha, float beta,
-                    int groups, int a_step, int c_step, cudaStream_t stream) {
+                    int epilogue, int up_col_off, int dtype, int static_b, int* status, float alpha, float beta, int groups,
+                    int a_step, int c_step, cudaStream_t stream) {
   using namespace blitz;
   if (groups < 1 || !blitz_gemm_wide_supported(M, N, K, 0, epilogue, groups)) return -1;
   if ((lda & 7) || (ldb & 7) || (ldc & 7) || (epi_gated(epilogue) && (up_col_off & 7))) return -1;
@@ -458,10 +457,9 @@ int blitz_gemm_wide(const void* A, int64_t lda, const void* W, int64_t ldb, void
   p.status = status;
   const int pairs_max = device_sm_count() / 2;
   const int tiles = p.tiles_m * p.tiles_n;
-  p.group_m = group_m > 0 ? group_m : 8;
-  if (p.group_m > p.tiles_m) p.group_m = p.tiles_m;
+  p.group_m = p.tiles_m < 8 ? p.tiles_m : 8;
   const int rest = tiles % pairs_max;
-  p.full = narrow > 0 ? 0 : (narrow == 0 && 2 * rest <= pairs_max) ? tiles - rest : tiles;
+  p.full = 2 * rest <= pairs_max ? tiles - rest : tiles;
   p.items = p.full + 2 * (tiles - p.full);
   const int pairs = p.items < pairs_max ? p.items : pairs_max;
 

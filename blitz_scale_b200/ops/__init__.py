@@ -292,7 +292,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
         use_wide = False
     if use_wide:
         rc = lib().blitz_gemm_wide(_p(a), a.stride(0), _p(b), b.stride(0), _p(out), out.stride(0), _p(extra), M, N, K, epi,
-                                   N if gated else 0, _dt(a), int(static_b), 0, 0, _status_ptr(a), alpha, beta,
+                                   N if gated else 0, _dt(a), int(static_b), _status_ptr(a), alpha, beta,
                                    groups, a_step, out_step, _stream())
         _check(rc, "blitz_gemm_wide")
         return out
