@@ -38,7 +38,7 @@
 // result does not depend on who that is).  Every half computes the ranges itself from the page table (a scan over the batch in
 // shared memory), so the launch does not depend on the lengths and replays from a CUDA graph.  Measured: 61 sequences of 170 .. 3500
 // tokens (67 k in all) 57 us, 82 us as whole sequences and 104 us as those before the halves.  An incomplete piece costs about 4 us
-// (fence, ticket, merge): sequences of one length are better cut into equal parts (Engine.choose_splits).
+// (fence, ticket, merge), all of them about 7 us a launch: which division serves a batch is measured at decode_parts (runtime/engine.py).
 //
 // Models that ask for it get a sliding window with kept first tokens (only the 64-token chunks that hold a visible key
 // are fetched: a sequence costs at most window + kept tokens whatever its length), soft-capped scores

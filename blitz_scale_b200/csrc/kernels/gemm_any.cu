@@ -30,16 +30,41 @@ struct BlitzGemmScratch {
   int* status;
 };
 
+// Whether more than 256 rows are better on pairs of CTAs with whole tiles of 256 x 256 (gemm_wide.cu; halves of them where a last round
+// of halves fits the 74 pairs) than on 148 CTAs with tiles of 128 x 256 or x 128 and K in parts (gemm_tcgen05.cu).  In a few rounds that
+// is a matter of which tiles fill the SMs.  Measured with cold weights, us, pairs / tiles:
+//   at most 74 tiles of 128 x 128: K in parts, which also sums less in one go
+//   at most 148: one round of tiles.  No half tiles: 300 x 6144 x 4096 25.7 / 19.5, 2048 x 1152 x 8192 45 / 33, with SiLU
+//     384 x 2816 x 2048 18.9 / 14.8.  Half tiles: 1024 x 2048 x 2048 12.5 / 11.3, into fp32 15.5 / 13.9; but epilogues that read or
+//     compute more hide behind the pairs' two accumulators: residual 512 x 2560 x 1024 8.5 / 9.5, SiLU 1000 x 1024 x 2048 16.9 / 21.2
+//     (columns that are not whole slabs of 64 keep the tiles' loads waiting: 6400 x 136 x 2048 12.3 / 15.5)
+//   at most 148 tiles of 128 x 256, but more than 74 pairs (rows that fill a little more than one tile of 256): 300 x 10240 x 4096
+//     38.7 / 34.6, with SiLU 300 x 5632 x 2048 33.9 / 29.8
+//   blocks that fill half of a tile's columns or less: 32 of 1000 x 128 x 512 11.5 / 10.7, but 32 of 4096 x 128 x 512 34.9 / 36.6; a
+//     quarter: 32 of 1574 x 64 x 512 15.6 / 12.9, 32 of 2500 21.1 / 23.4
+//   one round of whole tiles into fp32, whose epilogue nothing hides: 1290 x 2048 x 1024 17.0 / 15.5, K = 2048 22.2 / 21.5, 4096 32.5 / 33.5
+//   all others measured: 0.6 .. 1.0 of the tiles' time, for instance 1574 x 4096 x 4096 46.0 / 55.6, 8192 x 4096 x 14336 615 / 724
+static bool pairs_are_better(int M, int N, int K, int epilogue, int groups) {
+  const bool gated = epilogue == 2 || epilogue == 7, f32 = epilogue >= 4 && epilogue <= 6;
+  const int cols = gated ? 64 : 128;
+  auto tiles = [&](int rows, int columns) { return (int64_t)((M + rows - 1) / rows) * ((N + columns - 1) / columns) * groups; };
+  const int64_t narrow = tiles(128, cols), pairs = tiles(256, 2 * cols);
+  const bool odd = N < 2 * cols && N % 64 != 0;
+  if (narrow <= 74) return false;
+  if (narrow <= 148) return (2 * pairs <= 74 && (gated || epilogue == 1)) || odd;
+  if (tiles(128, 2 * cols) <= 148 && pairs > 74) return false;
+  if (N <= cols && narrow <= (2 * N <= cols ? 512 : 296)) return false;
+  if (f32 && !odd && K <= 2048 && pairs <= 74 && 2 * pairs > 74) return false;
+  return true;
+}
+
 // Which kernel takes a product with "in,out" weights: 0 the tiled one, 1 weight-streaming (its activation tile is read again with every
 // weight tile, which the SM's load path cannot keep up with beyond about 128 rows), 2 CTA pairs with K cut into parts, 3 CTA pairs over
-// whole tiles.  With at most 74 tiles of 128 x 128 the tiled one cuts K over the SMs, which is faster and sums less in one go.
+// whole tiles.
 int blitz_gemm_choice(int M, int N, int K, int epilogue, int groups) {
   if (groups == 1 && M <= 128) return blitz_gemm_decode_supported(M, N, K, 0, epilogue) ? 1 : 0;
   if (groups == 1 && M <= 256) return blitz_gemm_pair_supported(M, N, K, 0, epilogue) ? 2 : 0;
-  const int cols = epilogue == 2 || epilogue == 7 ? 64 : 128;
-  if (M > 256 && (int64_t)((M + 127) / 128) * ((N + cols - 1) / cols) * groups > 74 && blitz_gemm_wide_supported(M, N, K, 0, epilogue, groups))
-    return 3;
-  return 0;
+  return M > 256 && pairs_are_better(M, N, K, epilogue, groups) && blitz_gemm_wide_supported(M, N, K, 0, epilogue, groups) ? 3 : 0;
 }
 
 // Arguments as for blitz_gemm with "in,out" weights.

@@ -1,4 +1,4 @@
-// Weight-streaming tcgen05 GEMM for decode batches (M <= 256 tokens) on sm_100a.
+// Weight-streaming tcgen05 GEMM for decode batches on sm_100a: it takes M <= 256 tokens, the rule in gemm_any.cu sends it 128 at most.
 //
 //   C[M,N] = X[M,K] * W[K,N]      W in the serving layout ("in,out", N contiguous), 16-bit, fp32 accumulation
 //

@@ -70,3 +70,18 @@ def test_silu_of_large_negative_gates(M):
     want = (g / (1 + torch.exp(-g)) * 2.0 ** 100).expand(M, N)
     # one rounding to bf16; the exponential of fp32 numbers is off by 2 + 1.16 |x| units of fp32
     assert bool(((got - want).abs() <= want.abs() * (2.0 ** -8 + 110 * 2.0 ** -23)).all())
+
+
+# at the lines of the rule that chooses between this kernel and the tiled one (tests/test_gemm_choice_cpu.py), both sides
+@pytest.mark.parametrize("M,N,K,epi", [(384, 6144, 136, "store"), (385, 6144, 136, "store"), (1024, 2304, 72, "add"), (1152, 2304, 72, "add"),
+                                       (300, 9472, 64, "store"), (300, 9480, 64, "store"), (1300, 2048, 2048, "axpy"), (1300, 2048, 2056, "axpy")])
+def test_default_dispatch(M, N, K, epi):
+    from blitz_scale_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    a, w = torch.randn(M, K, device=DEV, generator=g).bfloat16(), (torch.randn(K, N, device=DEV, generator=g) * K ** -0.5).bfloat16()
+    old = torch.randn(M, N, device=DEV, generator=g).to(torch.float32 if epi == "axpy" else torch.bfloat16)
+    want = a.float() @ w.float() + (old.float() if epi != "store" else 0)
+    out = ops.gemm(a, w, out=old.clone(), residual=old if epi == "add" else None, epilogue=epi)
+    ops.check_status()
+    # one rounding of the result, and 32-bit sums in another order
+    assert float(((out.float() - want).abs() - (1e-5 if epi == "axpy" else 2.0 ** -8) * want.abs()).max()) <= 2e-5 * K ** 0.5
