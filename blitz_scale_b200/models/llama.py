@@ -47,7 +47,7 @@ class StepMeta:
     num_tokens: int = 0
     num_splits: int = 1
     seq_slot: Optional[torch.Tensor] = None                 # [B] state slot of every row (-1: padding row)
-    singles: int = 0                                        # of a ragged step: leading rows with one token
+    singles: int = 0                                        # of a ragged step: leading rows with one token that go through the decode kernels
 
 
 class TPComm:
@@ -145,8 +145,8 @@ class LlamaRunner:
     def _prefill_attention(self, l: int, m: StepMeta) -> None:
         """The pass's rows against everything the cache holds for their sequences (rope_kv_store has just added the
         rows' own keys and values): earlier chunks of a long prompt are simply a longer page list.  Leading rows of one token
-        (`m.singles`) are a decode batch: as tiles of 128 rows they would be padding (43 of them, 700 keys each, beside a portion
-        of 1531 tokens: 221 us with them among the tiles, 115 and 38 apart)."""
+        (`m.singles`) are a decode batch: as tiles of 128 rows they would be padding (see singles_apart in runtime/engine.py for how
+        many make it worth a kernel of their own)."""
         T, ns = m.num_tokens, m.singles
         if ns:
             ops.attn_decode(self.qkv[:ns], self.kv[l], m.page_indices, m.page_indptr[:ns + 1], m.last_page_len[:ns],

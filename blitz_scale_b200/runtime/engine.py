@@ -66,6 +66,16 @@ def decode_parts(rows: int, kv_heads: int, longest: int, tokens: int) -> int:
     return int(not (late and shared))
 
 
+def singles_apart(q_heads: int, single_lens: Sequence[int], portion_lens: Sequence[int]) -> bool:
+    """Whether the single tokens of a ragged step (keys of each; keys of the portions) go through decode attention instead of being
+    tiles of the prompts' kernel.  As tiles each takes a head's tile time, 3 us and 1 us per 64 keys, on one of 148 SMs; in a kernel
+    of their own they cost 7 to 12 us.  Few of them fill SMs that the portions leave idle at the end, the longer the longer the
+    portions.  Measured with 32 heads, together / apart, us: a portion of 1531 with 1, 3, 8, 43 singles of 1000 keys 39.6* / 47.1,
+    44.2* / 48.8, 69.6 / 51.1*, 210 / 80*; one of 300 with 1 and 8 of 300 12.8* / 20.8, 29.2 / 22.0*; one of 1531 behind 2311 with 4
+    and 8 of 1000 114.5* / 126.8, 146 / 129* (* chosen)."""
+    return q_heads * sum(3 + n / 64 for n in single_lens) > 148 * (10 + max(portion_lens, default=0) / 500)
+
+
 class Engine:
     def __init__(self, model: str | ModelConfig, *, num_pages: int, page_size: int = 64, max_batch: int = 256,
                  max_batch_tokens: int = 8192, tp: int = 1, tp_rank: int = 0, dtype=torch.bfloat16,
@@ -138,7 +148,7 @@ class Engine:
         L, d = self.layout, self.dev
         kv_lens = list(kv_lens) if kv_lens else list(seq_lens)
         if prefill and work is None:
-            # the leading single tokens of a ragged step go through the decode kernels
+            # leading single tokens that go through the decode kernels
             work = ops.prefill_work_list(seq_lens, kv_lens, self.page_size, self.device, skip=singles)
         return StepMeta(kv_lens_host=kv_lens, prefill_work=work,
                         ids=d[L.ids:L.ids + T], pos=d[L.pos:L.pos + T], slot=d[L.slot:L.slot + T],
@@ -334,6 +344,8 @@ class Engine:
                 else:
                     got = self.runner.logits[torch.tensor(at, device=self.device)].float()
         else:
+            if singles and self.cfg.family != "hybrid" and not singles_apart(self.cfg.q_heads // self.tp, kv_lens[:singles], kv_lens[singles:]):
+                singles = 0
             splits = self.choose_splits(singles, max(kv_lens[:singles]), sum(kv_lens[:singles])) if singles else 1
             m = self._views(T, rows, P, True, q_lens, splits=splits, kv_lens=kv_lens, singles=singles)
             with nvtx_range("step"):

@@ -81,3 +81,29 @@ def test_every_caller_says_how_many_tokens():
         E.Engine.choose_splits(E.Engine.__new__(E.Engine), 1, 1000)
     calls = [line for f in (ROOT / "bench.py", *(ROOT / "bench").glob("*.py")) for line in f.read_text().splitlines() if "choose_splits(" in line]
     assert calls and all("page_size" in line for line in calls)
+
+
+# keys of the singles, keys of the portion, apart; 32 heads
+SINGLES = [([60], 300, False), ([300], 300, False), ([1000], 1531, False), ([1000] * 3, 1531, False), ([300] * 2, 3842, False),
+           ([1000] * 4, 3842, False), ([4000], 1531, True), ([1000] * 8, 1531, True), ([300] * 16, 1531, True), ([60] * 43, 300, True),
+           ([1000] * 8, 3842, True), ([700] * 43, 3842, True)]
+
+
+@pytest.mark.parametrize("singles,portion,apart", SINGLES)
+def test_few_single_tokens_stay_beside_the_portion(singles, portion, apart):
+    """What the step asks of its runner: leading rows that go through the decode kernels, out of those with one token."""
+    eng = E.Engine.__new__(E.Engine)
+    eng.cfg, eng.tp, eng.use_graphs, eng.max_batch = get_config("llama3_8b"), 1, False, 256
+    eng.layout, eng.host_np, eng._h2d = types.SimpleNamespace(page_indices=0), None, lambda n: None
+    n, kv = len(singles), [*singles, portion]
+
+    class Asked(Exception):
+        pass
+
+    def views(T, rows, P, prefill, q_lens, splits, kv_lens, singles):
+        raise Asked(singles)
+    eng._views = views
+    fill = lambda *a: (n + 100, 0, n + 1, n, list(range(n + 1)), [1] * n + [100], kv)
+    with pytest.raises(Asked) as got:
+        eng._step_pass(types.SimpleNamespace(fill_step=fill), [1] * n + [100], [])
+    assert got.value.args == (n if apart else 0,)
