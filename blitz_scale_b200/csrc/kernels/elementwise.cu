@@ -52,8 +52,8 @@ __device__ __forceinline__ uint4 scaled8(const uint4& v, const uint4& w, float s
 // ADD = false: out = x * rsqrt(mean(x^2) + eps) * w
 // ADD = true : residual += x; out = RMSNorm(residual) * w     (out may alias x)
 // A block per row.  In a decode step latency counts, so a thread requests its weights together with its columns, keeps both (further
-// ones, beyond 8192 columns, are read again) and waits at one barrier: with the rotation below, 3693 -> 3652 us for a decode step of one
-// sequence through 32 layers of 4096 columns.  (A warp per row without any barrier takes 28.6 us for 8192 x 4096 by itself, this 40.9, but a
+// ones, beyond 8192 columns, are read again) and waits at one barrier: 2.4 -> 1.9 us for one row of 4096 columns, 38.5 -> 30.0 us for
+// 8192 rows.  (A warp per row without any barrier takes 28.6 us for 8192 x 4096 by itself, this 40.9, but a
 // prompt's pass of 8192 tokens took the same 95.7 ms with either.)
 template <typename T, bool ADD>
 __global__ void rms_norm_kernel(const T* __restrict__ x, T* __restrict__ residual, const T* __restrict__ w,
@@ -355,14 +355,6 @@ __global__ void rope_kv_store_kernel(T* __restrict__ qkv, const int32_t* __restr
   T* kdst = kv_layer + (static_cast<int64_t>(page) * 2) * plane + static_cast<int64_t>(off) * kv_heads * head_dim;
   T* vdst = kdst + plane;
 
-  // a thread's first pair of vectors is on its way while the angles are computed
-  const int rot_items = (q_heads + kv_heads) * vec_per_half;
-  uint4 first[2];
-  auto at = [&](int it) { return row + static_cast<int64_t>(it / vec_per_half) * head_dim + it % vec_per_half * 8; };
-  if (threadIdx.x < rot_items) {
-    first[0] = *reinterpret_cast<const uint4*>(at(threadIdx.x));
-    first[1] = *reinterpret_cast<const uint4*>(at(threadIdx.x) + half);
-  }
   // the angle of pair i depends on the token's position only: computed once per token (accurate sincosf: positions
   // of thousands of radians) and shared by all heads through shared memory
   __shared__ float s_cs[kRopeMaxHalf], s_sn[kRopeMaxHalf];
@@ -371,17 +363,14 @@ __global__ void rope_kv_store_kernel(T* __restrict__ qkv, const int32_t* __restr
     sincosf(p * inv_freq, &s_sn[i], &s_cs[i]);
   }
   __syncthreads();
+  const int rot_items = (q_heads + kv_heads) * vec_per_half;
   for (int it = threadIdx.x; it < rot_items; it += blockDim.x) {
     const int head = it / vec_per_half;
     const int v = it % vec_per_half;
     T* hp = row + static_cast<int64_t>(head) * head_dim;
     float a[8], b[8];
-    if (it != threadIdx.x) {
-      first[0] = *reinterpret_cast<const uint4*>(hp + v * 8);
-      first[1] = *reinterpret_cast<const uint4*>(hp + half + v * 8);
-    }
-    unpack8<T>(first[0], a);
-    unpack8<T>(first[1], b);
+    unpack8<T>(*reinterpret_cast<uint4*>(hp + v * 8), a);
+    unpack8<T>(*reinterpret_cast<uint4*>(hp + half + v * 8), b);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float cs = s_cs[v * 8 + j], sn = s_sn[v * 8 + j];
