@@ -11,6 +11,7 @@
 #include "launch.cuh"
 #include "ptx.cuh"
 #include "scalar.cuh"
+#include "tmap.cuh"
 
 namespace blitz {
 
@@ -49,15 +50,13 @@ __device__ __forceinline__ uint4 scaled8(const uint4& v, const uint4& w, float s
   return pack8<T>(f);
 }
 
-// ADD = false: out = x * rsqrt(mean(x^2) + eps) * w
-// ADD = true : residual += x; out = RMSNorm(residual) * w     (out may alias x)
+// out = x * rsqrt(mean(x^2) + eps) * w     (out may alias x)
 // A block per row.  In a decode step latency counts, so a thread requests its weights together with its columns, keeps both (further
 // ones, beyond 8192 columns, are read again) and waits at one barrier: 2.4 -> 1.9 us for one row of 4096 columns, 38.5 -> 30.0 us for
-// 8192 rows.  (A warp per row without any barrier takes 28.6 us for 8192 x 4096 by itself, this 40.9, but a
-// prompt's pass of 8192 tokens took the same 95.7 ms with either.)
-template <typename T, bool ADD>
-__global__ void rms_norm_kernel(const T* __restrict__ x, T* __restrict__ residual, const T* __restrict__ w,
-                                T* __restrict__ out, int hidden, float eps) {
+// 8192 rows.  (A warp per row without any barrier takes 28.6 us for those by itself, but a prompt's pass of 8192 tokens took the same
+// 95.7 ms with either.)
+template <typename T>
+__global__ void rms_norm_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ out, int hidden, float eps) {
   ptx::griddep_launch_dependents();
   ptx::griddep_wait();
   __shared__ float red[32];
@@ -65,7 +64,6 @@ __global__ void rms_norm_kernel(const T* __restrict__ x, T* __restrict__ residua
   const int nvec = hidden >> 3;
   const uint4* xv = reinterpret_cast<const uint4*>(x + base);
   const uint4* wv = reinterpret_cast<const uint4*>(w);
-  uint4* rv = ADD ? reinterpret_cast<uint4*>(residual + base) : nullptr;
   uint4 mine = make_uint4(0, 0, 0, 0), weights = mine;
   const bool has = threadIdx.x < nvec;
   if (has) {
@@ -73,32 +71,65 @@ __global__ void rms_norm_kernel(const T* __restrict__ x, T* __restrict__ residua
     weights = __ldg(wv + threadIdx.x);
   }
   float ss = 0.f;
-  auto take = [&](int i, uint4& v) {  // adds the residual (ADD), counts the squares
+  auto count = [&](const uint4& v) {
     float f[8];
     unpack8<T>(v, f);
-    if (ADD) {
-      float r[8];
-      unpack8<T>(rv[i], r);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] += r[j];
-      v = pack8<T>(f);
-      rv[i] = v;
-      unpack8<T>(v, f);  // normalise the rounded residual, as a separate add kernel would
-    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
   };
-  if (has) take(threadIdx.x, mine);
-  for (int i = threadIdx.x + blockDim.x; i < nvec; i += blockDim.x) {
-    uint4 v = xv[i];
-    take(i, v);
-  }
+  if (has) count(mine);
+  for (int i = threadIdx.x + blockDim.x; i < nvec; i += blockDim.x) count(xv[i]);
   ss = block_sum1(ss, red);
   const float scale = rsqrtf(ss / static_cast<float>(hidden) + eps);
   uint4* ov = reinterpret_cast<uint4*>(out + base);
   if (has) ov[threadIdx.x] = scaled8<T>(mine, weights, scale);
-  const uint4* src = ADD ? rv : xv;
-  for (int i = threadIdx.x + blockDim.x; i < nvec; i += blockDim.x) ov[i] = scaled8<T>(src[i], __ldg(wv + i), scale);
+  for (int i = threadIdx.x + blockDim.x; i < nvec; i += blockDim.x) ov[i] = scaled8<T>(xv[i], __ldg(wv + i), scale);
+}
+
+// residual += x; out = RMSNorm(residual) * w     (out may alias x)
+// KEEP: a thread keeps its first columns and weights as above.  That takes the registers of a second block of 1024 threads on an SM, so
+// with more rows than SMs and blocks that wide (beyond 4096 columns) the sums are read again instead.  us, kept and read again: one row
+// of 4096 columns 2.05 / 2.45, of 8192 2.7 / 3.1; 256 rows of 4096 3.1 / 3.6, of 12288 6.7 / 5.4; 8192 rows of 8192 123 / 100.
+template <typename T, bool KEEP>
+__global__ void add_rms_norm_kernel(const T* __restrict__ x, T* __restrict__ residual, const T* __restrict__ w, T* __restrict__ out,
+                                    int hidden, float eps) {
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
+  __shared__ float red[32];
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * hidden;
+  const int nvec = hidden >> 3;
+  const uint4* xv = reinterpret_cast<const uint4*>(x + base);
+  const uint4* wv = reinterpret_cast<const uint4*>(w);
+  uint4* rv = reinterpret_cast<uint4*>(residual + base);
+  float ss = 0.f;
+  auto sum = [&](int i, const uint4& a, const uint4& b) {  // stores the sum, counts its squares
+    float f[8], r[8];
+    unpack8<T>(a, f);
+    unpack8<T>(b, r);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] += r[j];
+    const uint4 packed = pack8<T>(f);
+    rv[i] = packed;
+    unpack8<T>(packed, f);  // normalise the rounded residual, as a separate add kernel would
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    return packed;
+  };
+  int first = threadIdx.x;
+  uint4 mine, weights;
+  const bool has = KEEP && first < nvec;
+  if (has) {
+    const uint4 a = xv[first], b = rv[first];
+    weights = __ldg(wv + first);
+    mine = sum(first, a, b);
+  }
+  if (KEEP) first += blockDim.x;
+  for (int i = first; i < nvec; i += blockDim.x) sum(i, xv[i], rv[i]);
+  ss = block_sum1(ss, red);
+  const float scale = rsqrtf(ss / static_cast<float>(hidden) + eps);
+  uint4* ov = reinterpret_cast<uint4*>(out + base);
+  if (has) ov[threadIdx.x] = scaled8<T>(mine, weights, scale);
+  for (int i = first; i < nvec; i += blockDim.x) ov[i] = scaled8<T>(rv[i], __ldg(wv + i), scale);
 }
 
 // ------------------------------------------------------------------ SiLU * mul, residual add
@@ -421,8 +452,8 @@ int blitz_rms_norm(const void* x, const void* w, void* out, int num_tokens, int 
   if (num_tokens <= 0) return 0;
   if (hidden & 7) return -1;
   cudaError_t blitz_last = cudaSuccess;
-  BLITZ_DISPATCH_DTYPE(dtype, (blitz_last = launch_pdl(rms_norm_kernel<T, false>, dim3(num_tokens), dim3(pick_threads(hidden >> 3)), 0, stream,
-                                  (const T*)x, nullptr, (const T*)w, (T*)out, hidden, eps)));
+  BLITZ_DISPATCH_DTYPE(dtype, (blitz_last = launch_pdl(rms_norm_kernel<T>, dim3(num_tokens), dim3(pick_threads(hidden >> 3)), 0, stream,
+                                  (const T*)x, (const T*)w, (T*)out, hidden, eps)));
   return (int)blitz_last;
 }
 
@@ -432,8 +463,10 @@ int blitz_add_rms_norm(const void* x, void* residual, const void* w, void* out, 
   if (num_tokens <= 0) return 0;
   if (hidden & 7) return -1;
   cudaError_t blitz_last = cudaSuccess;
-  BLITZ_DISPATCH_DTYPE(dtype, (blitz_last = launch_pdl(rms_norm_kernel<T, true>, dim3(num_tokens), dim3(pick_threads(hidden >> 3)), 0, stream,
-                                  (const T*)x, (T*)residual, (const T*)w, (T*)out, hidden, eps)));
+  const int threads = pick_threads(hidden >> 3);
+  const bool keep = threads < 1024 || num_tokens <= device_sm_count();
+  BLITZ_DISPATCH_DTYPE(dtype, (blitz_last = launch_pdl(keep ? add_rms_norm_kernel<T, true> : add_rms_norm_kernel<T, false>, dim3(num_tokens), dim3(threads), 0,
+                                  stream, (const T*)x, (T*)residual, (const T*)w, (T*)out, hidden, eps)));
   return (int)blitz_last;
 }
 

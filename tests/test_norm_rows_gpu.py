@@ -23,10 +23,10 @@ def test_rms_norm(H, dt):
         assert torch.equal(x, out[:T])
 
 
-@pytest.mark.parametrize("H", [8, 264, 8192, 8200, 16392])
+@pytest.mark.parametrize("H", [8, 264, 4096, 4104, 8192, 8200, 16392])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
 def test_add_rms_norm(H, dt):
-    """With a residual, which is rounded before it is normed and read again where a row is wider than what the threads keep."""
+    """With a residual, which is rounded before it is normed: rows below, at and beyond what the threads keep, more and fewer than SMs."""
     from blitz_scale_b200 import ops
     for T in (1, 149):
         x, r = torch.randn(T, H, device="cuda").to(dt), torch.randn(T, H, device="cuda").to(dt)
