@@ -29,12 +29,10 @@
 // the warps, division, store) runs beside the other half's chunks.  Measured, 32 query and 8 KV heads of 128, 256 x 513 tokens,
 // whole sequences: 111 us with one group, 98 us so (5.5 TB/s).
 //
-// Pieces.  num_splits >= 1: (sequence, KV head, split) items in a grid-stride loop over the halves.  num_splits = 0 (the serving
-// path): the chunks of all sequences laid end to end are cut into equal contiguous ranges, as many as there are halves per KV head,
-// and every half takes one head of one range, so that neither a long sequence nor a small batch leaves SMs idle; the halves that
+// Pieces.  num_splits >= 1: (sequence, KV head, split) items in a grid-stride loop over the halves.  num_splits = 0: the
+// chunks of all sequences laid end to end are cut into equal contiguous ranges, as many as there are halves per KV head, and every half takes one head of one range, so that neither a long sequence nor a small batch leaves SMs idle; the halves that
 // stream the heads of the same tokens do so at the same time (a token's heads are neighbours in memory).  A range's first and last
-// sequence may be incomplete: such pieces go to
-// scratch as fp32 partials, and whichever half finishes an item's last piece combines them (in the order of the ranges, so that the
+// sequence may be incomplete: such pieces go to scratch as fp32 partials, and whichever half finishes an item's last piece combines them (in the order of the ranges, so that the
 // result does not depend on who that is).  Every half computes the ranges itself from the page table (a scan over the batch in
 // shared memory), so the launch does not depend on the lengths and replays from a CUDA graph.  Measured: 61 sequences of 170 .. 3500
 // tokens (67 k in all) 57 us, 82 us as whole sequences and 104 us as those before the halves.  An incomplete piece costs about 4 us
