@@ -176,9 +176,9 @@ class Engine:
             return None
         return b
 
-    def choose_splits(self, rows: int, max_len: int, tokens: int) -> int:
+    def choose_splits(self, rows: int, max_len: int, tokens: int = 0) -> int:
         """How decode attention divides the keys of `rows` sequences (rows of padding not counted), the longest of max_len and `tokens`
-        in all: see decode_parts."""
+        in all (0: not known, taken for unequal lengths): see decode_parts."""
         if self.cfg.family == "hybrid":
             # (latent attention divides its keys by itself)
             kv_heads, max_len = self.cfg.attention_work(max_len, ("attention",))

