@@ -39,11 +39,11 @@ def decode_parts(rows: int, kv_heads: int, longest: int, tokens: int) -> int:
     into n parts each; 0: equal ranges of all of them, whatever their lengths.
 
     One of the 296 halves of the SMs takes a chunk of 64 keys in 0.7 us until they wait for HBM (all of them at work: 1.5 us).  Parts cost
-    a merge kernel, 2.8 us, so they have to save seven chunks, and more where they bring second halves of SMs to work: those start late
-    and share what their SM is given.  Ranges cost 7 us (pieces, tickets, merges), so they pay where the end of a launch would
-    otherwise leave most halves idle for longer than that.  Measured behind a small kernel, us, KV heads of 128, whole / parts / ranges
-    (* chosen):
-      8 heads, 1 sequence of 300, 500, 1000, 100k tokens:  7.8* / 9.2 (4) / 9.2,  9.9 / 8.7 (8)* / 9.2,  15.8 / 9.6 (16)* / 10.8,
+    a merge kernel, 2.8 us, so they have to save seven chunks, beyond eight parts two with every doubling, and more where they bring
+    second halves of SMs to work: those start late and share what their SM is given.  Ranges cost 7 us (pieces, tickets, merges), so
+    they pay where the end of a launch would otherwise leave most halves idle for longer than that.  Measured behind a small kernel, us,
+    KV heads of 128, whole / parts / ranges (* chosen):
+      8 heads, 1 sequence of 300, 500, 1000, 100k tokens:  7.8* / 9.2 (4) / 9.2,  9.9 / 8.7 (8)* / 9.2,  15.8 / 9.6 (8)* / 10.8,
         1085 / 72 (32)* / 76;  1 head, 100k: 1084 / 44 (32)* / 55
       8 heads, 3, 12, 18 and 25 of 1000:  16.1 / 11.8 (4)* / 15.0,  16.7* / 17.7 (2) / 23.0,  18.4* / 22.6 (2) / 26.5,  23.7* / - / 30.9
       8 heads, 38, 150 and 256 of 1000:  41.8 / - / 37.7*,  109.3 / - / 107.7*,  168.7* / - / 172.3
@@ -54,7 +54,8 @@ def decode_parts(rows: int, kv_heads: int, longest: int, tokens: int) -> int:
     equal = 4 * rows * longest <= 5 * tokens
     for parts in (32, 16, 8, 4, 2):
         n, part = items * parts, -(-chunks // parts)
-        fits = n <= 128 and (parts <= 16 or part > 1) or n <= 192 and part >= (16 if parts == 2 else 8) or n <= 256 and part >= 16
+        fits = n <= 128 and (parts <= 8 or -(-2 * chunks // parts) - part >= 2) or n <= 192 and part >= (16 if parts == 2 else 8) or \
+            n <= 256 and part >= 16
         if fits and parts <= chunks and chunks - part >= 7:
             return parts if equal or part <= 60 or not shared else 0
     if items <= 296:         # (in chunks at the full rate of HBM: what the longest one takes beyond an equal share)
@@ -416,7 +417,7 @@ class Engine:
         self._graphs[(Bp, splits)] = g
         return g
 
-    def precapture(self, max_batch: Optional[int] = None, contexts: Sequence[int] = (64, 512, 1024, 4096, 16384)) -> int:
+    def precapture(self, max_batch: Optional[int] = None, contexts: Sequence[int] = (64, 1024, 2048, 4096, 16384)) -> int:
         """Capture the decode graphs of every batch bucket up to `max_batch` (default: the engine's) and of the
         split-KV choices that contexts of the given lengths select, so that no request pays for a capture later.
         The captures run on padded rows only (an empty batch): graph topology and buffer addresses do not depend
