@@ -20,10 +20,11 @@ def test_chunked_prefill_equals_single_pass(model, lens):
         b = eng.new_batch(1, [core.SeqSpec(i, p, 6) for i, p in enumerate(prompts)])
         assert b is not None
         seqs = [[t] for t in eng.prefill(b)]
-        logits = eng.runner.logits[:len(lens)].float().clone()
+        logits = [eng.runner.logits[:len(lens)].float().clone()]
         for _ in range(4):
             for sq, t in zip(seqs, eng.decode(b)):
                 sq.append(t)
+            logits.append(eng.runner.logits[:len(lens)].float().clone())
         ops.check_status()
         outs.append((seqs, logits))
         b.clear()
@@ -32,8 +33,18 @@ def test_chunked_prefill_equals_single_pass(model, lens):
         torch.cuda.empty_cache()
     (one, l1), (chunked, l2) = outs
     # the same attention in different tilings: logits agree closely; tokens are equal unless two candidates tie
-    err = float((l1 - l2).norm() / l1.norm())
+    err = float((l1[0] - l2[0]).norm() / l1[0].norm())
     assert err < 2e-2, err
-    agree = sum(int(a == b_) for x, y in zip(one, chunked) for a, b_ in zip(x, y))
-    total = sum(len(x) for x in one)
-    assert agree >= 0.9 * total, (agree, total, one, chunked)
+    ties = 0
+    for r, (x, y) in enumerate(zip(one, chunked)):
+        at = next((i for i, (a, c) in enumerate(zip(x, y)) if a != c), None)
+        if at is None:
+            continue
+        # the passes before were of the same tokens: their logits agree as closely, and the two candidates are at most two units of
+        # bf16 (2^-7 of the value at most) apart in both; what follows is another text
+        ties += 1
+        p, q = l1[at][r], l2[at][r]
+        assert float((p - q).norm() / p.norm()) < 2e-2, (r, at)
+        for row in (p, q):
+            assert abs(float(row[x[at]] - row[y[at]])) <= 2 * 2 ** -7 * float(row.max()), (r, at, one, chunked)
+    assert ties <= 1, (one, chunked)
