@@ -300,7 +300,7 @@ class Engine:
         counts = list(counts)
         want = [list(w) for w in want] if len(want) else [[] for _ in counts]
         total = sum(len(w) for w in want)
-        if 0 < sum(counts) <= self.max_batch_tokens and all(0 <= p < c for w, c in zip(want, counts) for p in w):
+        if 0 < sum(counts) <= self.max_batch_tokens and len(want) <= len(counts) and all(0 <= p < c for w, c in zip(want, counts) for p in w):
             # one pass, whose rows come in the order asked for
             return self._step_pass(batch, counts, [(i, p) for i, w in enumerate(want) for p in w])
         first = [sum(len(w) for w in want[:i]) for i in range(len(want))]
