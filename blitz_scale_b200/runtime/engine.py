@@ -41,13 +41,16 @@ def decode_parts(rows: int, kv_heads: int, longest: int, tokens: int) -> int:
     One of the 296 halves of the SMs takes a chunk of 64 keys in 0.7 us until they wait for HBM (all of them at work: 1.5 us).  Parts cost
     a merge kernel, 2.8 us, so they have to save seven chunks, beyond eight parts two with every doubling, and more where they bring
     second halves of SMs to work: those start late and share what their SM is given.  Ranges cost 7 us (pieces, tickets, merges), so
-    they pay where the end of a launch would otherwise leave most halves idle for longer than that.  Measured behind a small kernel, us,
-    KV heads of 128, whole / parts / ranges (* chosen):
+    they pay where the end of a launch would otherwise leave most halves idle for longer than that.  Four and eight parts pay up to 256
+    of them: behind a small kernel they cost a microsecond or two more than half as many, but whole
+    steps are shorter with them.  Decode steps, ms, half as many parts / these: 16 x 1000 tokens, 4 KV heads of 128 and 64, 8 layers
+    1.332 / 1.326 (4 parts), unequal 1.398 / 1.342;  8 x 1000 1.117 / 1.097 (8), unequal 1.134 / 1.100;  3 x 1000, 8 heads of 128, 2 layers
+    0.962 / 0.947 (8).  Measured behind a small kernel, us, KV heads of 128, whole / parts / ranges (* chosen):
       8 heads, 1 sequence of 300, 500, 1000, 100k tokens:  7.8* / 9.2 (4) / 9.2,  9.9 / 8.7 (8)* / 9.2,  15.8 / 9.6 (8)* / 10.8,
         1085 / 72 (32)* / 76;  1 head, 100k: 1084 / 44 (32)* / 55
-      8 heads, 3, 12, 18 and 25 of 1000:  16.1 / 11.8 (4)* / 15.0,  16.7* / 17.7 (2) / 23.0,  18.4* / 22.6 (2) / 26.5,  23.7* / - / 30.9
+      8 heads, 3, 12, 18 and 25 of 1000:  16.1 / 11.8 (4; now 8) / 15.0,  16.7* / 17.7 (2) / 23.0,  18.4* / 22.6 (2) / 26.5,  23.7* / - / 30.9
       8 heads, 38, 150 and 256 of 1000:  41.8 / - / 37.7*,  109.3 / - / 107.7*,  168.7* / - / 172.3
-      8 heads, unequal, 5 up to 1000, 16 up to 16k:  15.9 / 13.6 (2)* / 20.1,  180 / 123 (2) / 105*;  61 up to 300, 600 and 4000:
+      8 heads, unequal, 5 up to 1000, 16 up to 16k:  15.9 / 13.6 (2; now 4) / 20.1,  180 / 123 (2) / 105*;  61 up to 300, 600 and 4000:
         17.9* / - / 24.2,  25.7* / - / 30.8,  102.7 / - / 92.2*"""
     items, chunks = rows * kv_heads, -(-longest // 64)
     shared = rows <= ops.ATTN_DECODE_SHARED_ROWS
@@ -55,7 +58,7 @@ def decode_parts(rows: int, kv_heads: int, longest: int, tokens: int) -> int:
     for parts in (32, 16, 8, 4, 2):
         n, part = items * parts, -(-chunks // parts)
         fits = n <= 128 and (parts <= 8 or -(-2 * chunks // parts) - part >= 2) or n <= 192 and part >= (16 if parts == 2 else 8) or \
-            n <= 256 and part >= 16
+            n <= 256 and part >= (2 if parts in (4, 8) else 16)
         if fits and parts <= chunks and chunks - part >= 7:
             return parts if equal or part <= 60 or not shared else 0
     if items <= 296:         # (in chunks at the full rate of HBM: what the longest one takes beyond an equal share)

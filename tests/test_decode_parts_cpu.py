@@ -24,7 +24,7 @@ def test_rows_of_padding_do_not_count():
         raise Captured(rows, splits)
     eng._capture = capture
     # (3, 5, 12, 18: parts or whole sequences as measured at 1000 tokens of 8 KV heads; 25 and 200 whole)
-    for B, rows, want in [(1, 1, 8), (3, 4, 4), (5, 8, 2), (12, 16, 1), (18, 24, 1), (25, 32, 1), (200, 256, 1)]:
+    for B, rows, want in [(1, 1, 8), (3, 4, 8), (5, 8, 4), (12, 16, 1), (18, 24, 1), (25, 32, 1), (200, 256, 1)]:
         batch = types.SimpleNamespace(size=B, max_seq_len=lambda: 1000, num_pages=lambda B=B: 16 * B, fill_decode=lambda *a: 0)
         with pytest.raises(Captured) as got:
             eng.decode(batch)
@@ -40,11 +40,13 @@ RULE = [
     # few heads and long contexts: as many parts as there are halves for
     ((1, 1, 100_000, 100_000), 32), ((1, 8, 100_000, 100_000), 32), ((2, 8, 16_000, 32_000), 16), ((1, 1, 1000, 1000), 8), ((1, 8, 1500, 1500), 8), ((1, 8, 1700, 1700), 16),
     ((1, 8, 500, 500), 8), ((1, 8, 4000, 4000), 16), ((5, 8, 4000, 20_000), 4),
+    # second halves of SMs for parts of four and eight
+    ((16, 4, 1000, 16_000), 4), ((16, 4, 3000, 48_000), 4), ((16, 4, 1000, 9000), 4), ((8, 4, 1000, 8000), 8), ((3, 8, 700, 2100), 8), ((9, 8, 1000, 9000), 1),
     # one length: whole where the SMs are full, ranges where a last round would be nearly empty
     ((256, 8, 513, 256 * 513), 1), ((37, 8, 4000, 37 * 4000), 1), ((38, 8, 4000, 38 * 4000), 0), ((64, 8, 4000, 64 * 4000), 1),
     ((38, 8, 200, 38 * 200), 1),
     # unequal: parts where there are few, else ranges
-    ((2, 8, 600, 900), 8), ((2, 8, 4000, 4100), 8), ((5, 8, 1000, 3000), 2), ((16, 8, 16_000, 100_000), 0), ((61, 8, 3500, 61 * 1100), 0),
+    ((2, 8, 600, 900), 8), ((2, 8, 4000, 4100), 8), ((5, 8, 1000, 3000), 4), ((16, 8, 16_000, 100_000), 0), ((61, 8, 3500, 61 * 1100), 0),
     ((200, 1, 16_000, 200 * 8000), 0),
     # more sequences than ranges are dealt out for
     ((257, 8, 4000, 257 * 1000), 1), ((300, 1, 1000, 300_000), 1),
