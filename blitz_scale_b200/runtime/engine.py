@@ -45,7 +45,8 @@ def decode_parts(rows: int, kv_heads: int, longest: int, tokens: int) -> int:
     of them: behind a small kernel they cost a microsecond or two more than half as many, but whole
     steps are shorter with them.  Decode steps, ms, half as many parts / these: 16 x 1000 tokens, 4 KV heads of 128 and 64, 8 layers
     1.332 / 1.326 (4 parts), unequal 1.398 / 1.342;  8 x 1000 1.117 / 1.097 (8), unequal 1.134 / 1.100;  3 x 1000, 8 heads of 128, 2 layers
-    0.962 / 0.947 (8).  Measured behind a small kernel, us, KV heads of 128, whole / parts / ranges (* chosen):
+    0.962 / 0.947 (8);  Llama-3-8B, 8 heads, 32 layers: 5 x 700 whole 3.794 / 3.701 (4), 4 x 3000 3.861 / 3.812 (8), 8 x 1000 3.765 / 3.796 (4),
+    unequal 3.975 / 3.855.  Measured behind a small kernel, us, KV heads of 128, whole / parts / ranges (* chosen):
       8 heads, 1 sequence of 300, 500, 1000, 100k tokens:  7.8* / 9.2 (4) / 9.2,  9.9 / 8.7 (8)* / 9.2,  15.8 / 9.6 (8)* / 10.8,
         1085 / 72 (32)* / 76;  1 head, 100k: 1084 / 44 (32)* / 55
       8 heads, 3, 12, 18 and 25 of 1000:  16.1 / 11.8 (4; now 8) / 15.0,  16.7* / 17.7 (2) / 23.0,  18.4* / 22.6 (2) / 26.5,  23.7* / - / 30.9
