@@ -28,7 +28,8 @@
 // Replaces the cuBLAS calls of the reference at decode sizes (src/util/cublas_wrapper.h:31-141; call
 // sites src/layer/attn.h:137-215, src/layer/glu.h:109-136).
 //
-// Roles (192 threads): warp 0 = TMA producer, warp 1 = UMMA issuer + TMEM owner, warps 2..5 = epilogue.
+// Roles (320 threads): warp 0 = TMA producer, warp 1 = UMMA issuer + TMEM owner, warps 2..9 = epilogue (TMEM lane quarter = warp % 4;
+// the two warps of a quarter take every other eight tokens).
 #include "launch.cuh"
 #include "ptx.cuh"
 #include "tmap.cuh"
@@ -38,7 +39,8 @@
 
 namespace blitz {
 
-constexpr int kDecThreads = 192;
+constexpr int kDecThreads = 320;
+constexpr int kDecEpiThreads = 256;
 constexpr int kDecBK = 64;
 constexpr int kDecTile = 128;  // output features per tile = UMMA M
 constexpr int kDecMaxSplit = 8;
@@ -55,7 +57,7 @@ struct DecGemmParams {
   int tiles;         // 128-feature tiles
   int split;         // CTAs per tile = cluster size
   int kb_per_split;  // K blocks per CTA of a cluster
-  int slice;         // tokens each cluster rank reduces and stores (multiple of 32: TMEM is read 32 columns at a time)
+  int slice;         // tokens each cluster rank reduces and stores (multiple of 8: TMEM is read 8 columns at a time)
   int slabs;         // the weights' columns come in whole slabs of 64, and tmap_w loads a tile of them at once
   int static_w;      // weights do not depend on earlier kernels of the stream
   float alpha;       // axpy; soft cap; limit of the clamped unit
@@ -75,14 +77,9 @@ struct DecCfg {
     const int s = usable_bytes(smem_bytes) / (x_stage_bytes(npad) + w_bytes);
     return s > kMaxStages ? kMaxStages : s;
   }
-  // The epilogue reads TMEM 32 columns at a time, so an accumulator is read up to `extent` columns from its
-  // start: (halves - 1) * npad + M rounded up to 32.
-  __host__ __device__ static int extent(int M, int npad, int halves) { return (halves - 1) * npad + ((M + 31) & ~31); }
-  __host__ __device__ static int num_acc(int M, int npad, int halves, int split) {
-    return (split == 1 && halves * npad + extent(M, npad, halves) <= 512) ? 2 : 1;
-  }
-  __host__ __device__ static int tmem_cols(int M, int npad, int halves, int split) {
-    const int need = (num_acc(M, npad, halves, split) - 1) * halves * npad + extent(M, npad, halves);
+  __host__ __device__ static int num_acc(int npad, int halves, int split) { return (split == 1 && 2 * halves * npad <= 512) ? 2 : 1; }
+  __host__ __device__ static int tmem_cols(int npad, int halves, int split) {
+    const int need = num_acc(npad, halves, split) * halves * npad;
     int c = 32;
     while (c < need) c <<= 1;
     return c;
@@ -104,49 +101,54 @@ __device__ __forceinline__ float dec_f32<__half>(__half v) { return __half2float
 
 __device__ __forceinline__ float dec_silu(float x) { return x / (1.0f + __expf(-x)); }
 
-// EPI: 0 store, 1 add residual, 2 silu(gate)*up, 4 store as fp32, 5 C += alpha * acc with C fp32, 6 alpha * tanh(acc / alpha)
-// as fp32.  Thread = output feature n; tokens b0 .. min(b0 + 32, b_end).
-// A warp writes 64 contiguous bytes per token.
+// The epilogue takes 8 tokens of a thread's feature at a time in rolled loops: its instructions run once per launch, right behind a
+// stream of weights that has displaced them from every cache, so each line of code costs a fetch of its own.  From the last product
+// to the last store, us, 32 tokens unrolled / eight in a loop: 4096 x 4096 with 1 and 61 tokens 7.9 / 2.3 and 11.8 / 3.8, 4096 x 14336
+// 10.2 / 2.3 and 10.0 / 3.0, 14336 gate and up columns x 4096 with 61 9.0 / 3.6.  A decode step of Llama-3-8B with 1, 61 (67 k keys) and 117
+// rows: 3.62 / 3.14, 5.65 / 4.90, 4.84 / 4.21 ms.
+
+// What tokens t .. t + 7 of feature n had before (1: the residual, 5: C itself).  C may be R: a thread reads and writes its own
+// elements only, so they can be requested before the accumulator is complete.
 template <typename T, int EPI>
-__device__ __forceinline__ void dec_store32(const DecGemmParams& p, const float (&g)[32], const float (&u)[32], int n,
-                                            int b0, int b_end) {
-  if (n >= p.N) return;
-  if (epi_f32(EPI)) {
-    float* cf = reinterpret_cast<float*>(p.C) + n;
-    float old[32];
-    const float inv = EPI == 6 ? 1.f / p.alpha : 0.f;
-    if (EPI == 5) {
+__device__ __forceinline__ void dec_old8(const DecGemmParams& p, int n, int t, int t_end, float (&old)[8]) {
+  if (EPI != 1 && EPI != 5) return;
+  const int64_t at = static_cast<int64_t>(t) * p.ldc + n;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) old[i] = (b0 + i < b_end) ? cf[static_cast<int64_t>(b0 + i) * p.ldc] : 0.f;
+  for (int i = 0; i < 8; ++i) {
+    old[i] = 0.f;
+    if (n < p.N && t + i < t_end)
+      old[i] = EPI == 5 ? reinterpret_cast<const float*>(p.C)[at + i * p.ldc] : dec_f32<T>(reinterpret_cast<const T*>(p.R)[at + i * p.ldc]);
+  }
+}
+
+// EPI: 0 store, 1 add residual, 2 silu(gate)*up, 4 store as fp32, 5 C += alpha * acc with C fp32, 6 alpha * tanh(acc / alpha)
+// as fp32.  Tokens t .. min(t + 8, t_end) of feature n; a warp writes 64 contiguous bytes per token.
+template <typename T, int EPI>
+__device__ __forceinline__ void dec_store8(const DecGemmParams& p, const float (&g)[8], const float (&u)[8], const float (&old)[8],
+                                           float bias_g, float bias_u, int n, int t, int t_end) {
+  const int64_t at = static_cast<int64_t>(t) * p.ldc + n;
+  const float inv = EPI == 6 ? 1.f / p.alpha : 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float v = g[i];
+    if (EPI == 1) v += old[i];
+    if (EPI == 2) v = dec_silu(v) * u[i];
+    if (EPI == 5) v = old[i] + p.alpha * v;
+    if (EPI == 6) v = p.alpha * ptx::tanh_ex2(v * inv);
+    if (EPI == kEpiClampGlu) v = clamp_glu(v + bias_g, u[i] + bias_u, p.alpha, p.beta);
+    if (n < p.N && t + i < t_end) {
+      if (epi_f32(EPI)) reinterpret_cast<float*>(p.C)[at + i * p.ldc] = v;
+      else reinterpret_cast<T*>(p.C)[at + i * p.ldc] = dec_cvt<T>(v);
     }
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (b0 + i < b_end) cf[static_cast<int64_t>(b0 + i) * p.ldc] = EPI == 5 ? old[i] + p.alpha * g[i] : EPI == 6 ? p.alpha * ptx::tanh_ex2(g[i] * inv) : g[i];
-    return;
   }
-  T* c = reinterpret_cast<T*>(p.C) + n;
-  float res[32], bias_g = 0.f, bias_u = 0.f;
-  if (EPI == kEpiClampGlu) {
-    bias_g = ldf<T>(reinterpret_cast<const T*>(p.R) + n);
-    bias_u = ldf<T>(reinterpret_cast<const T*>(p.R) + p.up_col_off + n);
-  }
-  if (EPI == 1) {
-    // C may alias R (in-place residual update): read all residual values before the first store, otherwise
-    // every load would have to wait for the store before it
-    const T* r = reinterpret_cast<const T*>(p.R) + n;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) res[i] = (b0 + i < b_end) ? dec_f32<T>(r[static_cast<int64_t>(b0 + i) * p.ldc]) : 0.f;
-  }
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const int b = b0 + i;
-    if (b < b_end) {
-      float v = g[i];
-      if (EPI == 2) v = dec_silu(v) * u[i];
-      if (EPI == kEpiClampGlu) v = clamp_glu(v + bias_g, u[i] + bias_u, p.alpha, p.beta);
-      if (EPI == 1) v += res[i];
-      c[static_cast<int64_t>(b) * p.ldc] = dec_cvt<T>(v);
-    }
+}
+
+template <typename T, int EPI>
+__device__ __forceinline__ void dec_bias(const DecGemmParams& p, int n, float& g, float& u) {
+  g = u = 0.f;
+  if (EPI == kEpiClampGlu && n < p.N) {
+    g = ldf<T>(reinterpret_cast<const T*>(p.R) + n);
+    u = ldf<T>(reinterpret_cast<const T*>(p.R) + p.up_col_off + n);
   }
 }
 
@@ -159,8 +161,8 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
   constexpr int kWBytes = kHalves * kDecTile * kDecBK * 2;  // weight bytes per stage
   constexpr uint32_t kFmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
   const int cols = kHalves * p.npad;  // TMEM columns per accumulator
-  const int num_acc = Cfg::num_acc(p.M, p.npad, kHalves, p.split);
-  const int tmem_cols = Cfg::tmem_cols(p.M, p.npad, kHalves, p.split);
+  const int num_acc = Cfg::num_acc(p.npad, kHalves, p.split);
+  const int tmem_cols = Cfg::tmem_cols(p.npad, kHalves, p.split);
   const int S = Cfg::num_stages(p.npad, kWBytes, p.smem_bytes);
   const int x_stage = Cfg::x_stage_bytes(p.npad);
   const uint32_t idesc = ptx::make_idesc_f16(kFmt, 1u, 0u, kDecTile, static_cast<uint32_t>(p.npad));
@@ -190,7 +192,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&tfull_bar[i], 1);
-      ptx::mbar_init(&tempty_bar[i], 128);
+      ptx::mbar_init(&tempty_bar[i], kDecEpiThreads);
     }
     *abort_flag = 0;
     ptx::fence_mbar_init();
@@ -331,15 +333,19 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue warps (128 threads)
+    // ------------------------------------------------------------ epilogue warps (256 threads)
     ptx::griddep_wait();
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     const int feat = q * 32 + lane;
+    const int t0 = ((warp - 2) >> 2) * 8;
     if (p.split == 1) {
       int acc = 0;
       uint32_t acc_phase = 0;
       for (int w = blockIdx.x; w < num_items; w += gridDim.x) {
         const int n = w * kDecTile + feat;
+        float old[8] = {}, bias_g, bias_u;
+        dec_bias<T, EPI>(p, n, bias_g, bias_u);
+        dec_old8<T, EPI>(p, n, t0, p.M, old);
         if (!ptx::bounded_mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) {
           if (p.status && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
           break;
@@ -347,22 +353,21 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
         ptx::tc_fence_after_sync();
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * cols);
 #pragma unroll 1
-        for (int c = 0; c < p.M; c += 32) {
-          uint32_t v[32];
-          float g[32], up[32];
-          ptx::tmem_ld_32x32(taddr + c, v);
-          if (epi_gated(EPI)) {
-            uint32_t t[32];
-            ptx::tmem_ld_32x32(taddr + p.npad + c, t);
-            ptx::tmem_ld_wait();
+        for (int t = t0; t < p.M; t += 16) {
+          uint32_t v[8], w8[8];
+          float g[8], up[8], next[8] = {};
+          ptx::tmem_ld_32x8(taddr + t, v);
+          if (epi_gated(EPI)) ptx::tmem_ld_32x8(taddr + p.npad + t, w8);
+          dec_old8<T, EPI>(p, n, t + 16, p.M, next);
+          ptx::tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) up[i] = __uint_as_float(t[i]);
-          } else {
-            ptx::tmem_ld_wait();
+          for (int i = 0; i < 8; ++i) {
+            g[i] = __uint_as_float(v[i]);
+            up[i] = epi_gated(EPI) ? __uint_as_float(w8[i]) : 0.f;
           }
+          dec_store8<T, EPI>(p, g, up, old, bias_g, bias_u, n, t, p.M);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) g[i] = __uint_as_float(v[i]);
-          dec_store32<T, EPI>(p, g, up, n, c, p.M);
+          for (int i = 0; i < 8; ++i) old[i] = next[i];
         }
         ptx::tc_fence_before_sync();
         ptx::mbar_arrive(&tempty_bar[acc]);
@@ -385,10 +390,17 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     const int tile = blockIdx.x / p.split;
     const bool epi = warp >= 2;
     const int q = warp & 3, feat = q * 32 + lane;
+    const int t0 = ((warp - 2) >> 2) * 8;  // (of a slice)
     const int groups = p.slice >> 2;                             // float4 groups per slice
     const uint32_t src_stride = kHalves * groups * (kDecTile * 16);  // bytes per source rank
+    const int n = tile * kDecTile + feat;
+    const int t_beg = crank * p.slice;
+    const int t_end = min(p.M, t_beg + p.slice);
+    float old[8] = {}, bias_g = 0.f, bias_u = 0.f;
     bool acc_ready = false;
     if (epi) {
+      dec_bias<T, EPI>(p, n, bias_g, bias_u);
+      dec_old8<T, EPI>(p, n, t_beg + t0, t_end, old);
       acc_ready = ptx::bounded_mbar_wait(&tfull_bar[0], 0, abort_flag);
       if (!acc_ready && p.status && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
       ptx::tc_fence_after_sync();
@@ -397,28 +409,24 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     ptx::cluster_arrive_release();
     ptx::cluster_wait_acquire();
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-    const uint32_t zone = ptx::smem_u32(smem);
+    const uint32_t zone = ptx::smem_u32(smem) + static_cast<uint32_t>(feat) * 16u;
     if (epi && acc_ready) {
-      // send every foreign slice of the accumulator to its owner
-      for (int h = 0; h < kHalves; ++h) {
+      // send every foreign slice of the accumulator to its owner, the next rank's first
 #pragma unroll 1
-        for (int c = 0; c < p.M; c += 32) {
-          uint32_t v[32];
-          ptx::tmem_ld_32x32(taddr + h * p.npad + c, v);
-          ptx::tmem_ld_wait();
+      for (int k = 1; k < p.split; ++k) {
+        const int owner = crank + k < p.split ? crank + k : crank + k - p.split;
+        const int beg = owner * p.slice, end = min(p.M, beg + p.slice);
+        const uint32_t dst = ptx::mapa_shared(zone + static_cast<uint32_t>(crank) * src_stride, static_cast<uint32_t>(owner));
+#pragma unroll 1
+        for (int t = beg + t0; t < end; t += 16) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int t0 = c + 4 * j;
-            if (t0 < p.M) {
-              const int owner = t0 / p.slice;
-              if (owner != crank) {
-                const int grp = (t0 - owner * p.slice) >> 2;
-                const uint32_t local = zone + static_cast<uint32_t>(crank) * src_stride +
-                                       static_cast<uint32_t>((h * groups + grp) * kDecTile + feat) * 16u;
-                ptx::st_shared_cluster_v4(ptx::mapa_shared(local, static_cast<uint32_t>(owner)), v[4 * j], v[4 * j + 1],
-                                          v[4 * j + 2], v[4 * j + 3]);
-              }
-            }
+          for (int h = 0; h < kHalves; ++h) {
+            uint32_t v[8];
+            ptx::tmem_ld_32x8(taddr + h * p.npad + t, v);
+            ptx::tmem_ld_wait();
+            const uint32_t at = dst + static_cast<uint32_t>(h * groups + ((t - beg) >> 2)) * (kDecTile * 16);
+            ptx::st_shared_cluster_v4(at, v[0], v[1], v[2], v[3]);
+            ptx::st_shared_cluster_v4(at + kDecTile * 16, v[4], v[5], v[6], v[7]);
           }
         }
       }
@@ -427,44 +435,37 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     ptx::cluster_arrive_release();
     ptx::cluster_wait_acquire();
     if (epi && acc_ready) {
-      const int t_beg = crank * p.slice;
-      const int t_end = min(p.M, t_beg + p.slice);
-      const int n = tile * kDecTile + feat;
+      const uint8_t* mine = smem + static_cast<size_t>(feat) * 16;
 #pragma unroll 1
-      for (int c = t_beg; c < t_end; c += 32) {
-        float g[32], up[32];
+      for (int t = t_beg + t0; t < t_end; t += 16) {
+        float g[8], up[8] = {}, next[8] = {};
+        dec_old8<T, EPI>(p, n, t + 16, t_end, next);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) g[i] = up[i] = 0.f;
         for (int h = 0; h < kHalves; ++h) {
-          uint32_t own[32];
-          ptx::tmem_ld_32x32(taddr + h * p.npad + c, own);
+          uint32_t own[8];
+          float sum[8];
+          ptx::tmem_ld_32x8(taddr + h * p.npad + t, own);
           ptx::tmem_ld_wait();
-          for (int s = 0; s < p.split; ++s) {  // rank order: the sum does not depend on timing
-            if (s == crank) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                if (h == 0) g[i] += __uint_as_float(own[i]);
-                else up[i] += __uint_as_float(own[i]);
-              }
-            } else {
-              const uint8_t* zs = smem + static_cast<size_t>(s) * src_stride;
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                if (c + 4 * j < t_end) {
-                  const int grp = (c + 4 * j - t_beg) >> 2;
-                  const float4 f = *reinterpret_cast<const float4*>(
-                      zs + static_cast<size_t>((h * groups + grp) * kDecTile + feat) * 16);
-                  if (h == 0) {
-                    g[4 * j] += f.x; g[4 * j + 1] += f.y; g[4 * j + 2] += f.z; g[4 * j + 3] += f.w;
-                  } else {
-                    up[4 * j] += f.x; up[4 * j + 1] += f.y; up[4 * j + 2] += f.z; up[4 * j + 3] += f.w;
-                  }
-                }
-              }
+          for (int i = 0; i < 8; ++i) sum[i] = 0.f;
+          const uint8_t* zs = mine + static_cast<size_t>(h * groups + ((t - t_beg) >> 2)) * (kDecTile * 16);
+#pragma unroll 1
+          for (int s = 0; s < p.split; ++s, zs += src_stride) {  // rank order: the sum does not depend on timing
+            float4 a = make_float4(__uint_as_float(own[0]), __uint_as_float(own[1]), __uint_as_float(own[2]), __uint_as_float(own[3]));
+            float4 b = make_float4(__uint_as_float(own[4]), __uint_as_float(own[5]), __uint_as_float(own[6]), __uint_as_float(own[7]));
+            if (s != crank) {
+              a = *reinterpret_cast<const float4*>(zs);
+              b = *reinterpret_cast<const float4*>(zs + kDecTile * 16);
             }
+            sum[0] += a.x; sum[1] += a.y; sum[2] += a.z; sum[3] += a.w;
+            sum[4] += b.x; sum[5] += b.y; sum[6] += b.z; sum[7] += b.w;
           }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) (h == 0 ? g : up)[i] = sum[i];
         }
-        dec_store32<T, EPI>(p, g, up, n, c, t_end);
+        dec_store8<T, EPI>(p, g, up, old, bias_g, bias_u, n, t, t_end);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) old[i] = next[i];
       }
     }
   }
@@ -516,7 +517,7 @@ static cudaError_t launch_dec(const CUtensorMap& tx, const CUtensorMap& tw, DecG
   if (split > p.num_kb) split = p.num_kb;
   const int stage_area = DecCfg::num_stages(p.npad, halves * kDecTile * kDecBK * 2, p.smem_bytes) * stage_bytes;
   while (split > 1) {
-    const int slice = (((p.M + split - 1) / split) + 31) & ~31;
+    const int slice = (((p.M + split - 1) / split) + 7) & ~7;
     const int64_t zone = (int64_t)split * halves * (slice / 4) * kDecTile * 16;
     const int kbs = (p.num_kb + split - 1) / split;
     const bool every_rank_has_work = (int64_t)kbs * (split - 1) < p.num_kb;
@@ -526,7 +527,7 @@ static cudaError_t launch_dec(const CUtensorMap& tx, const CUtensorMap& tw, DecG
   if (split < 1) split = 1;
   p.split = split;
   p.kb_per_split = (p.num_kb + split - 1) / split;
-  p.slice = (((p.M + split - 1) / split) + 31) & ~31;
+  p.slice = (((p.M + split - 1) / split) + 7) & ~7;
   int grid;
   if (split > 1) {
     grid = p.tiles * split;
