@@ -58,9 +58,37 @@ static bool pairs_are_better(int M, int N, int K, int epilogue, int groups) {
   return true;
 }
 
+// 129 to 256 rows: the weight-streaming kernel (1), whole or half tiles of 256 x 256 on CTA pairs (3), or those with K cut into parts
+// (2).  The first is as fast as its loads, 128 + M rows of 128 bytes per K block and CTA, with as many parts of K as clusters fit, and
+// adds an exchange of the parts' sums; the second takes a quarter of a microsecond per K block of a round of half tiles, 0.4 of whole ones.
+// Measured behind a small kernel with cold weights, us, 1 / 2 / 3:
+//   4096 x 4096 with a residual, 144 and 256 rows 15.9 / 21.0 / 20.3, 20.9 / 21.8 / 20.7;  6144 columns 18.0 / 23.3 / 21.0, 24.9 / 23.9 / 21.3
+//   4096 columns of K = 14336 32.4 / 39.8 / 59.0, 42.6 / 40.9 / 60.5;  2048 of it 19.3 / 49.9 / 57.4, 28.0 / 50.4 / 57.3
+//   128256 columns of K = 4096 181 / 214 / 202, 248 / 245 / 212;  8192 of K = 1024 11.4 / 14.5 / 9.7, 15.0 / 15.9 / 10.1
+//   6144 columns of K = 8192, 200 and 256 rows 34.5 / 35.6 / 38.8, 40.5 / 35.7 / 39.3
+// Gated units need both accumulators' weights at once: fewer stages, and beyond 192 rows room for fewer parts.  144, 192 and 256 rows:
+//   14336 x 4096 49.3 / 57.0 / 56.6, 54.3 / 57.5 / 57.7, 66.7 / 58.3 / 58.2;  8192 x 4096 36.0 / 35.9 / 34.8, 38.3 / 36.7 / 35.5, 62.1 / 37.4 / 36.2
+//   2816 x 2048 15.7 / 19.1 / 14.3, 17.5 / 19.3 / 14.5, 36.1 / 19.1 / 15.1
+// Over 32 shapes of which one in six is of a gated unit: within 1 % of the fastest of the three on average, 28 % with (2) for all.
+int blitz_gemm_few_rows(int M, int N, int K, int epilogue) {
+  const int tiles = (N + 127) / 128, wide = (N + 255) / 256, kb = (K + 63) / 64;
+  if (epilogue == 2 || epilogue == 7) return M <= 192 && tiles > 74 ? 1 : 3;
+  if (M > 224 && K >= 8192 && 2 * wide <= 74 && (int64_t)N * K >= 48 << 20) return 2;
+  static const int clusters[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};  // of that many CTAs that 148 SMs hold
+  int parts = 148 / tiles < 8 ? 148 / tiles : 8;
+  if (parts > kb) parts = kb;
+  while (parts > 1 && tiles > clusters[parts]) --parts;
+  if (parts < 1) parts = 1;
+  const float exchange = parts > 1 ? 0.027f * M : epilogue == 1 ? 0.07f * M : 1.5f;  // (one part: a residual's loads are exposed)
+  const float streaming = 1.25e-3f * (128 + M) * ((kb + parts - 1) / parts) * ((tiles + 147) / 148) + exchange;
+  const int rest = wide % 74;
+  const float rounds = 2 * wide <= 74 ? 0.625f : wide / 74 + (rest == 0 ? 0.f : 2 * rest <= 74 ? 0.65f : 1.f);
+  return streaming <= 0.4f * kb * rounds + 1.5f ? 1 : 3;
+}
+
 // Which kernel takes a product with "in,out" weights: 0 the tiled one, 1 weight-streaming (its activation tile is read again with every
-// weight tile, which the SM's load path cannot keep up with beyond about 128 rows), 2 CTA pairs with K cut into parts, 3 CTA pairs over
-// whole tiles.
+// weight tile), 2 the one that blitz_gemm_few_rows names (CTA pairs with K cut into parts if the caller asks for parts or tiles),
+// 3 CTA pairs over whole tiles.
 int blitz_gemm_choice(int M, int N, int K, int epilogue, int groups) {
   if (groups == 1 && M <= 128) return blitz_gemm_decode_supported(M, N, K, 0, epilogue) ? 1 : 0;
   if (groups == 1 && M <= 256) return blitz_gemm_pair_supported(M, N, K, 0, epilogue) ? 2 : 0;
@@ -72,7 +100,9 @@ int blitz_gemm_any(const void* A, int64_t lda, const void* B, int64_t ldb, void*
                    int epilogue, int up_col_off, int dtype, int static_b, const BlitzGemmScratch* s, float alpha, float beta, int groups,
                    int a_step, int c_step, cudaStream_t stream) {
   if (!s) return -1;
-  switch (blitz_gemm_choice(M, N, K, epilogue, groups)) {
+  int kernel = blitz_gemm_choice(M, N, K, epilogue, groups);
+  if (kernel == 2) kernel = blitz_gemm_few_rows(M, N, K, epilogue);  // (what one of the three takes the others take too)
+  switch (kernel) {
     case 1:
       return blitz_gemm_decode(A, lda, B, ldb, C, ldc, R, M, N, K, epilogue, up_col_off, dtype, static_b, 0, s->status, alpha, beta, stream);
     case 2:

@@ -121,6 +121,19 @@ __device__ __forceinline__ void dec_old8(const DecGemmParams& p, int n, int t, i
   }
 }
 
+// Asks for the lines of tokens t_beg .. t_end, those of every `step` eight from t on, ahead of dec_old8: a warp's share of a token's row
+// is one line.
+template <typename T, int EPI>
+__device__ __forceinline__ void dec_old_ahead(const DecGemmParams& p, int n0, int t, int t_end, int step, int lane) {
+  if ((EPI != 1 && EPI != 5) || n0 >= p.N) return;
+#pragma unroll 1
+  for (t += (lane >> 3) * step + (lane & 7); t < t_end; t += 4 * step) {
+    const int64_t at = static_cast<int64_t>(t) * p.ldc + n0;
+    const void* line = EPI == 5 ? static_cast<const void*>(reinterpret_cast<const float*>(p.C) + at) : static_cast<const void*>(reinterpret_cast<const T*>(p.R) + at);
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
+  }
+}
+
 // EPI: 0 store, 1 add residual, 2 silu(gate)*up, 4 store as fp32, 5 C += alpha * acc with C fp32, 6 alpha * tanh(acc / alpha)
 // as fp32.  Tokens t .. min(t + 8, t_end) of feature n; a warp writes 64 contiguous bytes per token.
 template <typename T, int EPI>
@@ -132,7 +145,7 @@ __device__ __forceinline__ void dec_store8(const DecGemmParams& p, const float (
   for (int i = 0; i < 8; ++i) {
     float v = g[i];
     if (EPI == 1) v += old[i];
-    if (EPI == 2) v = dec_silu(v) * u[i];
+    if (EPI == 2) v = dec_silu(t + i < t_end ? v : 1.f) * u[i];  // (a quotient of zero leaves the division's fast path, for the whole warp)
     if (EPI == 5) v = old[i] + p.alpha * v;
     if (EPI == 6) v = p.alpha * ptx::tanh_ex2(v * inv);
     if (EPI == kEpiClampGlu) v = clamp_glu(v + bias_g, u[i] + bias_u, p.alpha, p.beta);
@@ -345,6 +358,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
         const int n = w * kDecTile + feat;
         float old[8] = {}, bias_g, bias_u;
         dec_bias<T, EPI>(p, n, bias_g, bias_u);
+        dec_old_ahead<T, EPI>(p, n - lane, t0 + 16, p.M, 16, lane);
         dec_old8<T, EPI>(p, n, t0, p.M, old);
         if (!ptx::bounded_mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) {
           if (p.status && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
@@ -400,6 +414,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     bool acc_ready = false;
     if (epi) {
       dec_bias<T, EPI>(p, n, bias_g, bias_u);
+      dec_old_ahead<T, EPI>(p, n - lane, t_beg + t0 + 16, t_end, 16, lane);
       dec_old8<T, EPI>(p, n, t_beg + t0, t_end, old);
       acc_ready = ptx::bounded_mbar_wait(&tfull_bar[0], 0, abort_flag);
       if (!acc_ready && p.status && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);

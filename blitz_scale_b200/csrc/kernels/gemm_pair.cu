@@ -28,7 +28,9 @@
 // the odd CTA up columns, so a thread finds gate and up of one output element in its own TMEM lane), write
 // 128-byte-swizzled 32 x 64 boxes to a staging area and hand them to TMA stores: a thread-per-row epilogue would
 // issue one 16-byte store per lane into 32 different rows, which the load/store unit serialises.  Residual values
-// are requested before the wait for the accumulator.
+// are requested before the wait for the accumulator.  The slabs of a tile are a rolled loop: the code runs once or twice a launch, behind
+// weights that have displaced it from every cache (unrolled / rolled, from the last accumulator to the end, us, 256 rows x 6144 and
+// 4096 x 4096, 4096 x 14336: 11.3 / 9.5, 12.3 / 10.5, 11.3 / 10; the products of a layer of Llama-3-8B with their norms 146 / 138).
 // Replaces cuBLAS at these sizes (src/util/cublas_wrapper.h:31-141 of the reference; call sites
 // src/layer/attn.h:137-215, src/layer/glu.h:109-136, src/layer/lm_head.h:89-98).
 //
@@ -344,19 +346,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
         }
         const int n_own = __popc(own_mask);
-        uint4 rpre[kPairSlabsMax][4];
-        if (EPI == 1) {
+        // the residual of the first own slab is requested before the accumulator is complete, the next one's while a slab is converted
+        uint4 res[4] = {};
+        auto residual = [&](int from, uint4 (&r)[4]) {
+          const int i = from + __ffs(own_mask >> from) - 1;  // the next own slab
+          if (EPI != 1 || i < from) return;
           const T* Rp = reinterpret_cast<const T*>(p.R) + static_cast<int64_t>(row) * p.ldc;
 #pragma unroll
-          for (int i = 0; i < kPairSlabsMax; ++i) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int col = n0 + i * 64 + ch * 32 + j * 8;
-              rpre[i][j] = make_uint4(0, 0, 0, 0);
-              if (((own_mask >> i) & 1u) && row_ok && col < p.N) rpre[i][j] = *reinterpret_cast<const uint4*>(Rp + col);
-            }
+          for (int j = 0; j < 4; ++j) {
+            const int col = n0 + i * 64 + ch * 32 + j * 8;
+            r[j] = make_uint4(0, 0, 0, 0);
+            if (row_ok && col < p.N) r[j] = *reinterpret_cast<const uint4*>(Rp + col);
           }
-        }
+        };
+        residual(0, res);
         if (!ptx::bounded_mbar_wait(&tfull_bar[slot], buf_phase, abort_flag)) {
           if (p.status && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
           alive = false;
@@ -450,7 +453,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
           uint32_t staged = 0;  // slabs staged and not yet handed to TMA
           int own_idx = 0;      // index of the current slab among the own ones
-#pragma unroll
+          // (rolled: this code runs once or twice a launch and comes from far away, see the note at the top)
+#pragma unroll 1
           for (int i = 0; i < kPairSlabsMax; ++i) {
             if (((own_mask >> i) & 1u) && n0 + i * 64 < p.N) {
               if (n_contrib > 0 && (split ? own_idx == 0 : (i % slabs_per_round) == 0)) {
@@ -514,6 +518,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 const int c = i * 64 + ch * 32;  // first of this thread's 32 output columns within the tile
                 uint32_t v[32];
                 float gt[32], up[32];
+                uint4 next[4] = {};
+                residual(i + 1, next);
                 ptx::tmem_ld_32x32(taddr + c, v);
                 if (epi_gated(EPI)) {
                   uint32_t t[32];
@@ -529,6 +535,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 if (n_contrib > 0) {
                   // ascending pair order: the sum does not depend on timing
                   const int c_in = split ? ch * 32 : c - (i / slabs_per_round) * (p.out_cols / rounds);
+#pragma unroll 1
                   for (int j = 0; j < n_contrib; ++j) {
                     const uint8_t* base = smem + (split ? static_cast<size_t>(j * n_own + own_idx) * slab_bytes
                                                         : static_cast<size_t>(j) * round_bytes) +
@@ -581,9 +588,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 if (EPI == kEpiClampGlu) {
                   float y[32];
                   clamp_glu32<T>(reinterpret_cast<const T*>(p.R), p.up_col_off, n0 + c, p.N, p.alpha, p.beta, gt, up, y);
-                  pair_convert32<T, 0>(y, up, rpre[i], o4);
+                  pair_convert32<T, 0>(y, up, res, o4);
                 } else {
-                  pair_convert32<T, EPI>(gt, up, rpre[i], o4);
+                  pair_convert32<T, EPI>(gt, up, res, o4);
                 }
                 // 128-byte rows, 16-byte chunks XOR-swizzled by row: the layout the TMA store expects
                 uint8_t* rowp = boxes + ((i & (nbuf - 1)) * 4 + q) * 4096 + lane * 128;
@@ -591,6 +598,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 for (int j = 0; j < 4; ++j)
                   *reinterpret_cast<uint4*>(rowp + (((ch * 4 + j) ^ (lane & 7)) << 4)) = o4[j];
                 staged |= 1u << i;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) res[j] = next[j];
               }
               ++own_idx;
             }

@@ -279,31 +279,35 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const bool quarter_ok = row0 < p.M;  // the same for both warps of a quarter
       const int half = w.width >> 1;
       const int slabs = (epi_gated(EPI) ? half : w.width) >> 6;  // slabs of 64 output columns: 1, 2 or 4
-      uint4 res[4][4];
-      if (EPI == 1) {
+      // the residual of the first slab is requested before the accumulator is complete, the next one's while a slab is converted
+      uint4 res[4] = {};
+      auto residual = [&](int s, uint4 (&r)[4]) {
+        if (EPI != 1 || s >= slabs) return;
         const T* Rp = reinterpret_cast<const T*>(p.R) + static_cast<int64_t>(row) * p.ldc;
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int col = w.n0 + s * 64 + ch * 32 + j * 8;
-            res[s][j] = make_uint4(0, 0, 0, 0);
-            if (s < slabs && row_ok && col < p.N) res[s][j] = *reinterpret_cast<const uint4*>(Rp + col);
-          }
-      }
+        for (int j = 0; j < 4; ++j) {
+          const int col = w.n0 + s * 64 + ch * 32 + j * 8;
+          r[j] = make_uint4(0, 0, 0, 0);
+          if (row_ok && col < p.N) r[j] = *reinterpret_cast<const uint4*>(Rp + col);
+        }
+      };
+      residual(0, res);
       if (!ptx::bounded_mbar_wait(&tfull_bar[buf], buf_phase, abort_flag)) {
         if (p.status && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
         break;
       }
       ptx::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * 256);
-#pragma unroll
-      for (int s = 0; s < 4; ++s) {
+      // (rolled: in a launch of a round or two this code runs once or twice and comes from far away)
+#pragma unroll 1
+      for (int s = 0; s < slabs; ++s) {
         const int n = w.n0 + s * 64;
-        if (s >= slabs || !quarter_ok || n >= p.N) continue;
+        if (!quarter_ok || n >= p.N) continue;
         const int c = s * 64 + ch * 32;  // first of this thread's 32 columns within the tile
         uint32_t v[32];
         float g[32], up[32];
+        uint4 next[4] = {};
+        residual(s + 1, next);
         ptx::tmem_ld_32x32(taddr + c, v);
         if (epi_gated(EPI)) {
           uint32_t t[32];
@@ -347,17 +351,22 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         if (EPI == kEpiClampGlu) {
           float y[32];
           clamp_glu32<T>(reinterpret_cast<const T*>(p.R), p.up_col_off, n + ch * 32, p.N, p.alpha, p.beta, g, up, y);
-          pair_convert32<T, 0>(y, up, res[s], o4);
+          pair_convert32<T, 0>(y, up, res, o4);
         } else if (EPI == 2) {
           // divided as IEEE does: __fdividef is off by two units and answers zero for denominators beyond 2^126 (14336 x 4096 with it and
           // so, us: 300 rows 84.5 and 88.3, 1574 rows 264.5 and 272.0, within the spread at 8192)
           float y[32];
 #pragma unroll
-          for (int k = 0; k < 32; ++k) y[k] = g[k] / (1.f + __expf(-g[k])) * up[k];
-          pair_convert32<T, 0>(y, up, res[s], o4);
+          for (int k = 0; k < 32; ++k) {
+            const float x = row_ok ? g[k] : 1.f;  // a quotient of zero leaves the division's fast path, for the whole warp
+            y[k] = x / (1.f + __expf(-x)) * up[k];
+          }
+          pair_convert32<T, 0>(y, up, res, o4);
         } else {
-          pair_convert32<T, EPI>(g, up, res[s], o4);
+          pair_convert32<T, EPI>(g, up, res, o4);
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) res[j] = next[j];
         // the quarter's two boxes in turn: the previous contents (two slabs ago) have been read out
         uint8_t* box = staging + ((box_no++ & 1) * 4 + q) * 4096;
         if (issuer) ptx::tma_store_wait_read<1>();

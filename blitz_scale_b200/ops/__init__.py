@@ -212,9 +212,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     running in this stream (model weights), so the decode kernel may start streaming it before its
     predecessor has finished.
 
-    129..256 rows with 'kn' weights go to the paired-SM kernel (two CTAs issue one 256-row
-    ``tcgen05.mma.cta_group::2``, stream-K over CTA pairs); ``pair_path`` forces (True) or forbids (False) it for
-    any M, ``pair_bnf`` / ``pair_nacc`` / ``pair_upp`` override its tile width, tiles per pair and units per pair.
+    129..256 rows with 'kn' weights go to whichever is the fastest at their size of that kernel, the one for more rows and the
+    paired-SM kernel with K in parts (two CTAs issue one 256-row ``tcgen05.mma.cta_group::2``, stream-K over CTA pairs);
+    ``pair_path`` forces (True) or forbids (False) the last for any M, ``pair_bnf`` / ``pair_nacc`` / ``pair_upp`` override its tile width, tiles per pair and units per pair.
 
     More rows with 'kn' weights go to the kernel whose CTA pairs walk 256 x 256 tiles; ``wide_path`` forces (True) or forbids
     (False) it for any M.

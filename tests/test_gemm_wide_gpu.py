@@ -85,3 +85,27 @@ def test_default_dispatch(M, N, K, epi):
     ops.check_status()
     # one rounding of the result, and 32-bit sums in another order
     assert float(((out.float() - want).abs() - (1e-5 if epi == "axpy" else 2.0 ** -8) * want.abs()).max()) <= 2e-5 * K ** 0.5
+
+
+@pytest.mark.parametrize("M", [129, 144, 192, 193, 224, 225, 256])
+@pytest.mark.parametrize("N,K,epi", [(1024, 1024, "store"), (2048, 2048, "add"), (6144, 4096, "store"), (6144, 8192, "add"), (9600, 576, "silu_mul"), (1088, 520, "silu_mul")])
+def test_between_decode_batches_and_prompts(M, N, K, epi):
+    """129 to 256 rows: whichever kernel takes them, against sums in 64 bits and the paired kernel."""
+    from blitz_scale_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    a, b, res = r(M, K), r(K, 2 * N if epi == "silu_mul" else N) * K ** -0.5, r(M, N)
+    acc = a.double() @ b.double()
+    ref = torch.nn.functional.silu(acc[:, :N]) * acc[:, N:] if epi == "silu_mul" else acc + res.double() if epi == "add" else acc
+    outs = []
+    for kw in ({}, dict(pair_path=True)):
+        out = res.clone()
+        ops.gemm(a, b, out=out, epilogue=epi, static_b=True, **(dict(residual=out) if epi == "add" else {}), **kw)
+        # one rounding of the output, and sums of K products of size K^-0.5 in fp32
+        assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all(), kw
+        outs.append(out)
+    ops.check_status()
+    used = ops.lib().blitz_gemm_few_rows(M, N, K, {"store": 0, "add": 1, "silu_mul": 2}[epi])
+    assert used in (1, 2, 3)
+    if used == 2:
+        assert torch.equal(*outs)
