@@ -7,9 +7,15 @@
 //   out[t] = x[src(t)] / sqrt(mean(x^2) + eps) * (w_offset + w)        src(t) = rows ? rows[t] + row_offset : t
 //
 // A block per token; the row stays in registers between the two passes up to 8192 columns.
+//
+// Experts' rows in 16 bits (stream_add_norm_kernel): bound by their bytes for prompts, by latency for a decode step.  A thread takes eight
+// columns, asks for the row numbers once and then for up to eight rows' pieces and the stream's at the same time, 16 bytes each; one row
+// after the other, four columns wide and with a store of the stream between groups of columns, every piece waited for the one before.
+// Measured, seven rows a token of 2048 columns: 4096 tokens 60 -> 41 us, 16 tokens 12.4 -> 4.6 us.
 #include "launch.cuh"
 #include "ptx.cuh"
 #include "scalar.cuh"
+#include <type_traits>
 
 namespace blitz {
 
@@ -106,6 +112,72 @@ __global__ void stream_norm_kernel(const StreamNormParams p) {
   for (int i = threadIdx.x + kSnKeep * blockDim.x; i < n; i += blockDim.x) write(i, load(xr + i * VEC));
 }
 
+// Only the rows to add change the stream (16-bit types, whole groups of eight columns, GROUPS of them for each thread).
+template <typename T, int GROUPS>
+__global__ void __launch_bounds__(512, 2) stream_add_norm_kernel(const StreamNormParams p) {
+  ptx::griddep_launch_dependents();
+  __shared__ float red[32];
+  const int t = blockIdx.x, n = p.hidden / 8;
+  float* xr = p.x + static_cast<int64_t>(t) * p.hidden;
+  const int32_t* add_row = p.add_row + static_cast<int64_t>(t) * p.n_add;
+  ptx::griddep_wait();
+  int rows[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) rows[k] = k < p.n_add ? add_row[k] : 0;
+  float keep[GROUPS][8];
+  float ss = 0.f;
+#pragma unroll
+  for (int g = 0; g < GROUPS; ++g) {
+    const int i = threadIdx.x + g * blockDim.x;
+    if (i >= n) continue;
+    ldf8<float>(xr + i * 8, keep[g]);
+    for (int k0 = 0; k0 < p.n_add; k0 += 8) {
+      if (k0 > 0) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) rows[k] = k0 + k < p.n_add ? add_row[k0 + k] : 0;
+      }
+      uint4 e[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        e[k] = make_uint4(0, 0, 0, 0);
+        if (k0 + k < p.n_add) e[k] = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.add) + static_cast<int64_t>(rows[k]) * p.hidden + i * 8);
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        if (k0 + k >= p.n_add) break;
+        float f[8];
+        unpack8<T>(e[k], f);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) keep[g][c] += f[c];
+      }
+    }
+    if (p.n_add > 8 && g + 1 < GROUPS) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) rows[k] = add_row[k];
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) ss += keep[g][c] * keep[g][c];
+  }
+#pragma unroll
+  for (int g = 0; g < GROUPS; ++g) {
+    const int i = threadIdx.x + g * blockDim.x;
+    if (i < n) stf8<float>(xr + i * 8, keep[g]);
+  }
+  if (p.out == nullptr) return;
+  const float scale = rsqrtf(block_sum1(ss, red) / static_cast<float>(p.hidden) + p.eps);
+  T* out = reinterpret_cast<T*>(p.out) + static_cast<int64_t>(t) * p.hidden;
+#pragma unroll
+  for (int g = 0; g < GROUPS; ++g) {
+    const int i = threadIdx.x + g * blockDim.x;
+    if (i >= n) continue;
+    float w[8];
+    ldf8<T>(reinterpret_cast<const T*>(p.w) + i * 8, w);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) w[c] = keep[g][c] * scale * (p.w_offset + w[c]);
+    stf8<T>(out + i * 8, w);
+  }
+}
+
 }  // namespace blitz
 
 extern "C" {
@@ -125,6 +197,16 @@ int blitz_stream_norm(const int32_t* ids, const void* embed, const void* step, c
   while (threads < n && threads < (n > 1024 ? 512 : 256)) threads <<= 1;
   auto go = [&](auto type, auto vec) {
     using T = decltype(type);
+    if constexpr (!std::is_same<T, float>::value) {
+      // whole 16-byte pieces of everything, nothing but rows to add, at most two groups of eight columns a thread
+      auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+      if (n_add > 0 && !init && !add_embed && step == nullptr && (hidden & 7) == 0 && hidden <= 8192 && aligned(x) && aligned(add) && aligned(out) && aligned(w)) {
+        int wide = 32;
+        while (wide < hidden / 8 && wide < 512) wide <<= 1;
+        return wide * 8 >= hidden ? launch_pdl(stream_add_norm_kernel<T, 1>, dim3(num_tokens), dim3(wide), 0, stream, p)
+                                  : launch_pdl(stream_add_norm_kernel<T, 2>, dim3(num_tokens), dim3(wide), 0, stream, p);
+      }
+    }
     constexpr int V = decltype(vec)::value;
     return n_add > 0 ? launch_pdl(stream_norm_kernel<T, V, true>, dim3(num_tokens), dim3(threads), 0, stream, p)
                      : launch_pdl(stream_norm_kernel<T, V, false>, dim3(num_tokens), dim3(threads), 0, stream, p);

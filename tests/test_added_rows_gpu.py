@@ -1,0 +1,27 @@
+"""Experts' rows added to an fp32 stream, and its norm: sizes at the edges of a thread's columns and of the rows in flight."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H", [8, 264, 2048, 4096, 4104, 8192, 8200])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 17])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_rows_in_flight(H, n, dt):
+    from blitz_scale_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(H + n)
+    T = 37
+    x = torch.randn(T, H, generator=g, device="cuda")
+    y, w = torch.randn(50, H, generator=g, device="cuda").to(dt), torch.randn(H, generator=g, device="cuda").to(dt)
+    rows = torch.randint(0, 50, (T, n), generator=g, device="cuda")
+    want = x.double() + y.double()[rows].sum(1)
+    normed = want * torch.rsqrt((want * want).mean(1, keepdim=True) + 1e-3) * (1 + w.double())
+    for keep_out in (True, False):
+        xd, out = x.clone(), torch.empty(T, H, dtype=dt, device="cuda") if keep_out else None
+        ops.stream_norm(xd, w if keep_out else None, 1e-3, out, w_offset=1.0, add=y, add_rows=rows.to(torch.int32))
+        # sums of n + 1 numbers of size one in fp32; one rounding of the output
+        assert ((xd.double() - want).abs() <= 2.0 ** -23 * (n + 1) * (1 + y.double().abs()[rows].sum(1))).all()
+        if keep_out:
+            assert ((out.double() - normed).abs() <= (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11) * normed.abs() + 1e-5).all()
+    ops.check_status()
