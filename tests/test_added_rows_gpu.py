@@ -25,3 +25,21 @@ def test_rows_in_flight(H, n, dt):
         if keep_out:
             assert ((out.double() - normed).abs() <= (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11) * normed.abs() + 1e-5).all()
     ops.check_status()
+
+
+@pytest.mark.parametrize("H", [8, 264, 2048, 4096, 4104, 8192, 8200])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_norm_alone(H, dt):
+    from blitz_scale_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x, w = torch.randn(37, H, generator=g, device="cuda"), torch.randn(H, generator=g, device="cuda").to(dt)
+    before, out = x.clone(), torch.full((38, H), -7.0, device="cuda", dtype=dt)
+    ops.stream_norm(x, w, 1e-3, out[:37], w_offset=1.0)
+    want = x.double() * torch.rsqrt((x.double() ** 2).mean(1, keepdim=True) + 1e-3) * (1 + w.double())
+    assert ((out[:37].double() - want).abs() <= (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11) * want.abs() + 1e-5).all()
+    assert torch.equal(x, before) and (out[37] == -7.0).all()
+    rows = torch.tensor([36, 0, 17], device="cuda", dtype=torch.int32)      # what the kernel for everything takes
+    some = torch.empty(3, H, device="cuda", dtype=dt)
+    ops.stream_norm(x, w, 1e-3, some, w_offset=1.0, rows=rows)
+    assert ((some.double() - want[rows.long()]).abs() <= (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11) * want[rows.long()].abs() + 1e-5).all()
+    ops.check_status()
