@@ -206,6 +206,8 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();  // queries, keys, values and the work list come from earlier kernels
   const uint32_t tmem_S = tmem_base;        // S_t (and P_t over its first 64 columns) at + 128 t
   const uint32_t tmem_O = tmem_base + 256;  // O_t at + VD t
 
@@ -648,8 +650,7 @@ static int launch_paged_prefill(const CUtensorMap (&tm)[3], const PagedPrefillPa
     return cudaFuncSetAttribute(attn_prefill_paged_kernel<T, HD, VD, POLY, EXT, BIAS, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   });
   if (e != cudaSuccess) return (int)e;
-  attn_prefill_paged_kernel<T, HD, VD, POLY, EXT, BIAS, SIG><<<grid, kPpThreads, kSmem, stream>>>(tm[0], tm[1], tm[2], p);
-  return (int)cudaGetLastError();
+  return (int)launch_pdl(attn_prefill_paged_kernel<T, HD, VD, POLY, EXT, BIAS, SIG>, dim3(grid), dim3(kPpThreads), (size_t)kSmem, stream, tm[0], tm[1], tm[2], p);
 }
 
 static long long* g_pp_trace = nullptr;
