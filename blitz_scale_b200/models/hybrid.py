@@ -81,6 +81,12 @@ class HybridRunner:
         self._gates = torch.empty(max_tokens * 2 * rw, dtype=torch.float32, device=dev) if rw else None
         ck = max((m.heads * m.dim for m in cfg.run_mixers() if m.kind in ("gla", "wkv")), default=0)
         self._cum = torch.empty(max_tokens * ck, dtype=torch.float32, device=dev) if ck and dt == torch.bfloat16 else None
+        # column layout of every layer's projection, and which of the different ones it is
+        layouts: Dict[tuple, int] = {}
+        self._columns = []
+        for s in cfg.layer_specs:
+            cols, width = s.in_columns()
+            self._columns.append((cols, width, layouts.setdefault((width, tuple(cols.items())), len(layouts))))
         self._init_experts(max_tokens, dev, dt)
         self._init_streams(max_tokens, max_batch, dev, dt)
         self._init_latent(max_tokens, max_batch, dev, dt)
@@ -106,6 +112,16 @@ class HybridRunner:
     @staticmethod
     def _rot_key(m: AttentionMixer) -> tuple:
         return (m.rot_dims, m.rot_base, m.yarn)
+
+    def _projection(self, l: int, m: StepMeta) -> tuple:
+        """Buffer of layer l's projection in this pass, [T, width], and its parts by name."""
+        cols, width, layout = self._columns[l]
+        T = m.num_tokens
+
+        def make(base):
+            proj = base[:T * width].view(T, width)
+            return proj, {n: proj[:, at:at + w] for n, (at, w) in cols.items()}
+        return m.view(("proj", layout), self._proj, make)
 
     def _w(self, l: int, name: str) -> torch.Tensor:
         return self.seg[f"layers.{l}.{name}"]
@@ -191,25 +207,24 @@ class HybridRunner:
         if c.streams:
             return self._run_layer_streams(r, l, spec, m)
         step = self.seg["loop_step"][run.step] if run.step >= 0 else None
-        h = self.normed[:T]
+        h, res = m.rows("normed", self.normed, T), m.rows("res", self.res, T)
         needs_ids = r == 0 or run.add_embed
         if r == 0:
             self._pending = None
-        ops.stream_norm(self.res[:T], self._w(l, "norm1"), c.rms_eps, h, w_offset=c.norm_offset, ids=m.ids if needs_ids else None,
+        ops.stream_norm(res, self._w(l, "norm1"), c.rms_eps, h, w_offset=c.norm_offset, ids=m.ids if needs_ids else None,
                         embed=self.seg["embed"] if needs_ids else None, init=r == 0, add_embed=run.add_embed, step=step,
                         **self._take_pending())
-        cols, width = spec.in_columns()
-        proj = self._proj[:T * width].view(T, width)
+        proj, parts = self._projection(l, m)
         ops.gemm(h, self._w(l, "in"), out=proj, static_b=True)
-        mid = self._mid[self._mid_key(spec)][:T]
-        parts = {n: proj[:, at:at + w] for n, (at, w) in cols.items()}
+        key = self._mid_key(spec)
+        mid = m.rows(key, self._mid[key], T)
         getattr(self, "_" + spec.mixer.kind)(r, l, spec.mixer, parts, mid, m)
         if spec.ff:
-            ops.gemm(h, self._w(l, "gate_up"), out=mid[:, spec.mix_rows:], epilogue="silu_mul", static_b=True)
-        ops.gemm(mid, self._w(l, "out"), out=self.res[:T], epilogue="axpy", alpha=c.residual_mult, static_b=True)
+            ops.gemm(h, self._w(l, "gate_up"), out=m.view(("ff", spec.mix_rows), mid, lambda t: t[:, spec.mix_rows:]), epilogue="silu_mul", static_b=True)
+        ops.gemm(mid, self._w(l, "out"), out=res, epilogue="axpy", alpha=c.residual_mult, static_b=True)
         if spec.moe:
-            ops.stream_norm(self.res[:T], self._w(l, "norm2"), c.rms_eps, h, w_offset=c.norm_offset)
-            out, plan = self._experts(l, spec.moe, h)
+            ops.stream_norm(res, self._w(l, "norm2"), c.rms_eps, h, w_offset=c.norm_offset)
+            out, plan = self._experts(l, spec.moe, h, m)
             self._pending = (out, plan.place)
 
     def _streams(self, norm: Optional[str] = None, **what) -> None:
@@ -221,9 +236,12 @@ class HybridRunner:
         else:
             ops.stream_rms(self.res, eps=self.cfg.rms_eps, w=self.seg[norm] if norm else None, w_offset=self.cfg.norm_offset, **what)
 
-    def _join(self, l: int, q: int, T: int, **more) -> torch.Tensor:
+    def _join(self, l: int, q: int, m: StepMeta, **more) -> torch.Tensor:
         """Input of sublayer q of layer l; the streams take up what is pending."""
-        take, h = self._pending is not None, more.pop("out", self.normed[:T])
+        T = m.num_tokens
+        take, h = self._pending is not None, more.pop("out", None)
+        if h is None:
+            h = m.rows("normed", self.normed, T)
         self._streams(f"layers.{l}.norm{q}", n=T, read=self._w(l, f"hc{q}_in"), out=h, write=take, **more)
         self._fresh = self._fresh and not take
         return h
@@ -234,11 +252,11 @@ class HybridRunner:
         T, H, rc = m.num_tokens, self.cfg.hidden, self.cache.runs[r]
         mu = self._w(l, "mu") if mx.kind == "wkv" else None
         width = H * (mu.shape[0] if mu is not None else 1)
-        out = self._mixed[:T * width].view(T, width)
+        out = m.view(("mixed", width), self._mixed, lambda t: t[:T * width].view(T, width))
         conv = self._w(l, "mix_conv")
         if not m.is_prefill:
-            return self._join(l, 1, T, out=out, tokens=ops.TokenState(conv, rc.mix_hist, mu, rc.shift), pos=m.pos, seq_slot=m.seq_slot)
-        h = self._join(l, 1, T, out=self._unmixed[:T])
+            return self._join(l, 1, m, out=out, tokens=ops.TokenState(conv, rc.mix_hist, mu, rc.shift), pos=m.pos, seq_slot=m.seq_slot)
+        h = self._join(l, 1, m, out=m.rows("unmixed", self._unmixed, T))
         shift = dict(mu=mu, shift=rc.shift, last=self._last_h) if mu is not None else {}
         return ops.token_conv(h, conv, rc.mix_hist, out, m.pos, m.tok_indptr, m.seq_slot, residual=True, **shift)
 
@@ -252,15 +270,15 @@ class HybridRunner:
         T, c = m.num_tokens, self.cfg
         if r == 0:
             self._pending, self._fresh, self._ids = None, True, m.ids
-        h, y = self._join_convolved(r, l, spec.mixer, m) if c.mix_taps else self._join(l, 1, T), self._y[:T]
-        cols, width = spec.in_columns()
-        mid = self._mid[self._mid_key(spec)][:T]
+        h, y = self._join_convolved(r, l, spec.mixer, m) if c.mix_taps else self._join(l, 1, m), m.rows("y", self._y, T)
+        key = self._mid_key(spec)
+        mid = m.rows(key, self._mid[key], T)
         if spec.mixer.kind == "wkv":                 # its projections have an input each
             self._wkv(r, l, spec.mixer, h, mid, m)
         else:
-            proj = self._proj[:T * width].view(T, width)
+            proj, parts = self._projection(l, m)
             ops.gemm(h, self._w(l, "in"), out=proj, static_b=True)
-            getattr(self, "_" + spec.mixer.kind)(r, l, spec.mixer, {n: proj[:, at:at + w] for n, (at, w) in cols.items()}, mid, m)
+            getattr(self, "_" + spec.mixer.kind)(r, l, spec.mixer, parts, mid, m)
         if spec.mixer.kind == "parallel":
             both, H = self._y[:2 * T].view(T, 2 * c.hidden), c.hidden
             ops.gemm(mid, self._w(l, "out"), out=both[:, :H], static_b=True)
@@ -270,16 +288,16 @@ class HybridRunner:
             ops.gemm(mid, self._w(l, "out"), out=y, static_b=True)
             self._leave(l, 1, y)
         if spec.ff_after:
-            h = self._join(l, 2, T)
-            act = self._ff[:T * spec.ff_after_pad].view(T, spec.ff_after_pad)
+            h = self._join(l, 2, m)
+            act = m.view(("ff", spec.ff_after_pad), self._ff, lambda t: t[:T * spec.ff_after_pad].view(T, spec.ff_after_pad))
             unit = (dict(epilogue="clamp_glu", alpha=spec.unit.limit, beta=spec.unit.beta, bias=self._w(l, "gate_up_b")) if spec.unit
                     else dict(epilogue="silu_mul"))
             ops.gemm(h, self._w(l, "gate_up"), out=act, static_b=True, **unit)
             ops.gemm(act, self._w(l, "down"), out=y, static_b=True)
             self._leave(l, 2, y, **(dict(bias=self._w(l, "down_b")) if spec.unit else {}))
         elif spec.moe:
-            h = self._join(l, 2, T)
-            out, plan = self._experts(l, spec.moe, h)
+            h = self._join(l, 2, m)
+            out, plan = self._experts(l, spec.moe, h, m)
             self._leave(l, 2, out, place=plan.place, ident=plan.ident, prev=h if spec.moe.identity else None)
 
     def _take_pending(self) -> dict:
@@ -291,11 +309,11 @@ class HybridRunner:
         if self._pending and not self.cfg.streams:
             ops.stream_norm(self.res[:T], None, 0.0, None, **self._take_pending())
 
-    def _experts(self, l: int, e: ExpertsSpec, h: torch.Tensor) -> tuple:
+    def _experts(self, l: int, e: ExpertsSpec, h: torch.Tensor, m: StepMeta) -> tuple:
         """Output rows of the chosen experts, and the plan that says whose they are."""
         T, H = h.shape
         plan = self._plans[self._plan_key(e)]
-        z = self._router[:T * e.router_cols].view(T, e.router_cols)
+        z = m.view(("router", e.router_cols), self._router, lambda t: t[:T * e.router_cols].view(T, e.router_cols))
         # few columns: beyond a decode batch, narrow tiles with K split keep more SMs loading
         narrow = dict(bn=64, split_k=4 if T <= 2048 else 1) if T > ops.DECODE_GEMM_MAX_M else {}
         ops.gemm(h, self._w(l, "router"), out=z, static_b=True, **narrow)
@@ -305,8 +323,9 @@ class HybridRunner:
         ops.moe_route(z, plan, weight_on_input=e.weight_on_input, renormalize=e.renormalize, softmax=e.softmax,
                       correction=self._w(l, "correction") if e.correction else None, groups=e.groups, keep=e.keep,
                       tile_rows=128 if tc else 64)
-        width = max(e.ff_pad, e.shared_pad)
-        act, out = self._act[:plan.rows * width].view(plan.rows, width), self._expert_out[:plan.rows]
+        width, rows = max(e.ff_pad, e.shared_pad), plan.rows
+        act = m.view(("experts", rows, width), self._act, lambda t: t[:rows * width].view(rows, width))
+        out = m.rows("expert_out", self._expert_out, rows)
         ops.gemm_grouped(h, up, plan, act, shared=s_up, gather=True, act="silu_gate" if e.gated else "relu2", factors=True)
         ops.gemm_grouped(act, down, plan, out, shared=s_down)
         return out, plan
@@ -336,9 +355,10 @@ class HybridRunner:
         args = dict(q_heads=mx.heads, kv_heads=mx.kv_heads, head_dim=mx.dim, page_size=self.page_size, sm_scale=mx.scale, **extra)
         ns = m.singles if m.is_prefill else m.batch
         if ns:
-            ops.attn_decode(p["q"][:ns], kv, m.page_indices, m.page_indptr[:ns + 1], m.last_page_len[:ns],
-                            num_splits=m.num_splits, workspace=self._workspace(ns, mx, m.num_splits), out=mid[:ns], static_table=True,
-                            gate=gate[:ns] if gate is not None else None, **args)
+            ops.attn_decode(m.rows("q", p["q"], ns), kv, m.page_indices, m.rows("page_indptr", m.page_indptr, ns + 1),
+                            m.rows("last_page_len", m.last_page_len, ns), num_splits=m.num_splits,
+                            workspace=self._workspace(ns, mx, m.num_splits), out=m.rows("mid", mid, ns), static_table=True,
+                            gate=m.rows("gate", gate, ns) if gate is not None else None, **args)
         if m.batch > ns:
             ops.attn_prefill_paged(p["q"], kv, m.page_indices, m.prefill_work, out=mid, gate=gate, **args)
 
@@ -359,20 +379,23 @@ class HybridRunner:
         freqs, gate = self._freqs[(mx.rot_dim, mx.rot_base, None)], p.get("g")
         ops.latent_store(p["dq"], p["dkv"], m.pos, m.slot, kv, self._w(l, "dq_norm"), self._w(l, "dkv_norm"), freqs, eps=self.cfg.rms_eps,
                          interleaved=mx.interleaved)
-        q = self._q[:T * H * mx.qdim].view(T, H * mx.qdim)
+        q = m.view(("latent q", H * mx.qdim), self._q, lambda t: t[:T * H * mx.qdim].view(T, H * mx.qdim))
         ops.gemm(p["dq"], self._w(l, "uq"), out=q, static_b=True)
         rotate = dict(heads=H, dim=mx.dim, rot=mx.rot_dim, interleaved=mx.interleaved)
         extra = dict(window=mx.window, sink=self._w(l, "sink") if mx.sink else None)
         n = m.batch if not m.is_prefill else m.singles if self._expands(mx, q.dtype) else T    # rows that go through the latent space
         if n:
-            ql, ol = self._q_latent[:n * H * W].view(n, H * W), self._o_latent[:n * H * R].view(n, H * R)
-            ops.gemm(q[:n], self._w(l, "uk"), out=ql, groups=H, a_step=mx.qdim, out_step=W, static_b=True)
-            ops.latent_rotate(q[:n], ql[:, R:], m.pos[:n], freqs, out_step=W, **rotate)
+            ql = m.view(("latent queries", n, H * W), self._q_latent, lambda t: t[:n * H * W].view(n, H * W))
+            ol = m.view(("latent outputs", n, H * R), self._o_latent, lambda t: t[:n * H * R].view(n, H * R))
+            qn = m.rows("latent q", q, n)
+            ops.gemm(qn, self._w(l, "uk"), out=ql, groups=H, a_step=mx.qdim, out_step=W, static_b=True)
+            ops.latent_rotate(qn, m.view(("rotated", R), ql, lambda t: t[:, R:]), m.rows("pos", m.pos, n), freqs, out_step=W, **rotate)
             single = not m.is_prefill or n == m.singles
-            g = gate[:n] if gate is not None else None
+            g = m.rows("gate", gate, n) if gate is not None else None
             if ops.attn_latent_supported(ql, n if single else min(n, ops.ATTN_LATENT_ROWS), H, kv):
                 rows = m.batch if not single else n
-                ops.attn_latent(ql, kv, m.page_indices, m.page_indptr[:rows + 1], m.last_page_len[:rows], heads=H, scale=mx.scale,
+                ops.attn_latent(ql, kv, m.page_indices, m.rows("page_indptr", m.page_indptr, rows + 1),
+                                m.rows("last_page_len", m.last_page_len, rows), heads=H, scale=mx.scale,
                                 workspace=self._latent_ws, out=ol, gate=g, static_table=True, **extra,
                                 **({} if single else dict(pos=m.pos[:n], tok_indptr=m.tok_indptr)))
             else:
@@ -380,14 +403,15 @@ class HybridRunner:
                                 m.page_indices, ol, q_heads=H, kv_heads=1, dim=W, page_size=self.page_size, scale=mx.scale, gate=g, **extra)
             # few rows: a tile per head is enough, and an exchange of K splits would cost more than it saves
             narrow = dict(bn=64, split_k=1) if n <= ops.PAIR_GEMM_MAX_M else {}
-            ops.gemm(ol, self._w(l, "uv"), out=mid[:n, :H * mx.vdim], groups=H, a_step=R, out_step=mx.vdim, static_b=True, **narrow)
+            ops.gemm(ol, self._w(l, "uv"), out=m.view(("latent mid", n, H * mx.vdim), mid, lambda t: t[:n, :H * mx.vdim]), groups=H, a_step=R, out_step=mx.vdim, static_b=True, **narrow)
         if n < T:
             self._latent_prompts(l, mx, q, gate, kv, mid, m, n, freqs, rotate, extra)
 
     def _latent_prompts(self, l: int, mx: LatentAttentionMixer, q, gate, kv: ops.LatentKV, mid, m: StepMeta, n: int, freqs, rotate, extra) -> None:
         """Rows from n on: keys and values of all their sequences' cached rows are expanded into a pool of their own, some heads
         at a time where that would be large.  With a window only the pages that one of a sequence's rows sees."""
-        ops.latent_rotate(q[n:], q[n:, mx.dim:], m.pos[n:], freqs, out_step=mx.qdim, **rotate)
+        ops.latent_rotate(m.view(("from", n), q, lambda t: t[n:]), m.view(("from", n, mx.dim), q, lambda t: t[n:, mx.dim:]),
+                          m.view(("pos from", n), m.pos, lambda t: t[n:]), freqs, out_step=mx.qdim, **rotate)
         ps = self.page_size
         index, pages, np_ = self._expanded_pages(m, n, mx.window, q.device)
         rows = ops.latent_gather(kv, pages, self._room("rows", (np_ * ps, mx.width), q.dtype))

@@ -20,7 +20,7 @@ src/layer/attn.h:217-233, src/layer/glu.h:138-154); the LM head exchanges one
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from typing import List, Optional
+from typing import Callable, Dict, List, Optional
 
 import torch
 
@@ -48,6 +48,22 @@ class StepMeta:
     num_splits: int = 1
     seq_slot: Optional[torch.Tensor] = None                 # [B] state slot of every row (-1: padding row)
     singles: int = 0                                        # of a ragged step: leading rows with one token that go through the decode kernels
+    _views: Dict = field(default_factory=dict)              # see `view`
+
+    def view(self, key, base: torch.Tensor, make: Callable):
+        """``make(base)``, made once in this pass: a view costs its caller 1.3 us, as much as half a launch, and the layers of a pass ask
+        for the same ones.  (The entry holds ``base``: another tensor under this key makes another view.)"""
+        have = self._views.get(key)
+        if have is None or have[0] is not base:
+            have = self._views[key] = (base, make(base))
+        return have[1]
+
+    def rows(self, key, base: torch.Tensor, n: int) -> torch.Tensor:
+        """The first n rows of ``base``."""
+        have = self._views.get((key, n))
+        if have is None or have[0] is not base:
+            have = self._views[(key, n)] = (base, base[:n])
+        return have[1]
 
 
 class TPComm:
@@ -76,6 +92,7 @@ class LlamaRunner:
         cfg = seg.cfg
         self.cfg: ModelConfig = cfg
         self.seg, self.kv, self.comm = seg, kv_cache, comm
+        self._kv_layers = list(kv_cache.unbind(0))
         self.tp = seg.tp
         self.qh, self.kvh, self.hd = cfg.q_heads // self.tp, cfg.kv_heads // self.tp, cfg.head_dim
         self.inter = cfg.inter // self.tp
@@ -125,21 +142,23 @@ class LlamaRunner:
 
     def attention_block(self, l: int, m: StepMeta) -> None:
         T, c = m.num_tokens, self.cfg
-        ops.rms_norm(self.res[:T], self._w(l, "input_ln"), c.rms_eps, out=self.normed[:T])
-        ops.gemm(self.normed[:T], self._w(l, "qkv"), static_b=True, out=self.qkv[:T])
-        ops.rope_kv_store(self.qkv[:T], m.pos[:T], m.slot[:T], self.kv[l], q_heads=self.qh, kv_heads=self.kvh,
+        res, normed, qkv, attn = (m.rows(n, t, T) for n, t in (("res", self.res), ("normed", self.normed), ("qkv", self.qkv), ("attn", self.attn)))
+        kv = self._kv_layers[l]
+        ops.rms_norm(res, self._w(l, "input_ln"), c.rms_eps, out=normed)
+        ops.gemm(normed, self._w(l, "qkv"), static_b=True, out=qkv)
+        ops.rope_kv_store(qkv, m.rows("pos", m.pos, T), m.rows("slot", m.slot, T), kv, q_heads=self.qh, kv_heads=self.kvh,
                           head_dim=self.hd, page_size=self.page_size, rope_theta=c.rope_theta)
         if m.is_prefill:
             self._prefill_attention(l, m)
         else:
-            ops.attn_decode(self.qkv[:T], self.kv[l], m.page_indices, m.page_indptr, m.last_page_len,
+            ops.attn_decode(qkv, kv, m.page_indices, m.page_indptr, m.last_page_len,
                             q_heads=self.qh, kv_heads=self.kvh, head_dim=self.hd, page_size=self.page_size,
                             num_splits=m.num_splits, workspace=self._workspace(m.batch, m.num_splits), static_table=True,
-                            out=self.attn[:T])
+                            out=attn)
         if self.tp == 1:
-            ops.gemm(self.attn[:T], self._w(l, "o"), static_b=True, out=self.res[:T], residual=self.res[:T], epilogue="add")
+            ops.gemm(attn, self._w(l, "o"), static_b=True, out=res, residual=res, epilogue="add")
         else:
-            ops.gemm(self.attn[:T], self._w(l, "o"), static_b=True, out=self.tmp[:T])
+            ops.gemm(attn, self._w(l, "o"), static_b=True, out=self.tmp[:T])
             self.comm.all_reduce_(self.tmp[:T])
 
     def _prefill_attention(self, l: int, m: StepMeta) -> None:
@@ -147,18 +166,19 @@ class LlamaRunner:
         rows' own keys and values): earlier chunks of a long prompt are simply a longer page list.  Leading rows of one token
         (`m.singles`) are a decode batch: as tiles of 128 rows they would be padding (see singles_apart in runtime/engine.py for how
         many make it worth a kernel of their own)."""
-        T, ns = m.num_tokens, m.singles
+        T, ns, kv = m.num_tokens, m.singles, self._kv_layers[l]
         if ns:
-            ops.attn_decode(self.qkv[:ns], self.kv[l], m.page_indices, m.page_indptr[:ns + 1], m.last_page_len[:ns],
-                            q_heads=self.qh, kv_heads=self.kvh, head_dim=self.hd, page_size=self.page_size,
-                            num_splits=m.num_splits, workspace=self._workspace(ns, m.num_splits), static_table=True, out=self.attn[:ns])
+            ops.attn_decode(m.rows("qkv", self.qkv, ns), kv, m.page_indices, m.rows("page_indptr", m.page_indptr, ns + 1),
+                            m.rows("last_page_len", m.last_page_len, ns), q_heads=self.qh, kv_heads=self.kvh, head_dim=self.hd,
+                            page_size=self.page_size, num_splits=m.num_splits, workspace=self._workspace(ns, m.num_splits), static_table=True,
+                            out=m.rows("attn", self.attn, ns))
             if m.batch == ns:
                 return
         if m.prefill_work is None:      # a caller that built the step by hand
             m.prefill_work = ops.prefill_work_list(m.seq_lens_host, m.kv_lens_host or m.seq_lens_host, self.page_size,
                                                    self.qkv.device, skip=ns)
-        ops.attn_prefill_paged(self.qkv[:T], self.kv[l], m.page_indices, m.prefill_work, q_heads=self.qh,
-                               kv_heads=self.kvh, head_dim=self.hd, page_size=self.page_size, out=self.attn[:T])
+        ops.attn_prefill_paged(m.rows("qkv", self.qkv, T), kv, m.page_indices, m.prefill_work, q_heads=self.qh,
+                               kv_heads=self.kvh, head_dim=self.hd, page_size=self.page_size, out=m.rows("attn", self.attn, T))
 
     def last_rows(self, m: StepMeta) -> torch.Tensor:
         """[batch, hidden]: the state `head` starts from, for the last row of every sequence of a prefill pass."""
@@ -174,17 +194,18 @@ class LlamaRunner:
 
     def ffn_block(self, l: int, m: StepMeta) -> None:
         T, c = m.num_tokens, self.cfg
+        res, normed, act = (m.rows(n, t, T) for n, t in (("res", self.res), ("normed", self.normed), ("act", self.act)))
         if self.tp == 1:
-            ops.rms_norm(self.res[:T], self._w(l, "post_ln"), c.rms_eps, out=self.normed[:T])
+            ops.rms_norm(res, self._w(l, "post_ln"), c.rms_eps, out=normed)
         else:
-            ops.add_rms_norm(self.tmp[:T], self.res[:T], self._w(l, "post_ln"), c.rms_eps, out=self.normed[:T])
-        ops.gemm(self.normed[:T], self._w(l, "gate_up"), static_b=True, out=self.act[:T], epilogue="silu_mul")
+            ops.add_rms_norm(self.tmp[:T], res, self._w(l, "post_ln"), c.rms_eps, out=normed)
+        ops.gemm(normed, self._w(l, "gate_up"), static_b=True, out=act, epilogue="silu_mul")
         if self.tp == 1:
-            ops.gemm(self.act[:T], self._w(l, "down"), static_b=True, out=self.res[:T], residual=self.res[:T], epilogue="add")
+            ops.gemm(act, self._w(l, "down"), static_b=True, out=res, residual=res, epilogue="add")
         else:
-            ops.gemm(self.act[:T], self._w(l, "down"), static_b=True, out=self.tmp[:T])
+            ops.gemm(act, self._w(l, "down"), static_b=True, out=self.tmp[:T])
             self.comm.all_reduce_(self.tmp[:T])
-            ops.add_residual(self.res[:T], self.tmp[:T])
+            ops.add_residual(res, self.tmp[:T])
 
     def run_layer(self, l: int, m: StepMeta) -> None:
         self.attention_block(l, m)

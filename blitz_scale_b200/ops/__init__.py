@@ -187,14 +187,6 @@ def _scratch_of(index: int) -> int:
     return (_gemm_scratch.get(index) or _once(_gemm_scratch, index, make))[0]
 
 
-def _tensor_core_operands(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, N: int, K: int) -> bool:
-    """Sizes, pitches and base addresses the TMA-fed kernels need (16-byte rows and bases; fp32 outputs are accessed 32
-    bytes at a time)."""
-    return (N % 8 == 0 and K % 8 == 0 and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0 and out.stride(0) % 8 == 0
-            and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0
-            and out.data_ptr() % (32 if out.dtype == torch.float32 else 16) == 0)
-
-
 def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *, residual=None,
          epilogue: str = "store", alpha: float = 1.0, beta: float = 1.0, bias: Optional[torch.Tensor] = None, groups: int = 1, a_step: int = 0, out_step: int = 0, b_layout: str = "kn", bn: int = 0, split_k: int = 0, static_b: bool = False,
          decode_path: Optional[bool] = None, decode_split: int = 0, pair_path: Optional[bool] = None,
@@ -227,51 +219,58 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     group to the next one in a and out, where the blocks' columns are parts of wider ones.  fp32 operands, and 16-bit ones
     whose sizes the tensor-core kernels do not take, run on the CUDA cores in fp32 arithmetic.
     """
-    assert a.is_cuda and a.dim() == 2 and b.dim() == 2 and a.stride(1) == 1 and b.stride(1) == 1
-    M, K = a.shape
+    assert a.is_cuda and a.dim() == 2 and b.dim() == 2
+    # (shapes, pitches and addresses are asked for once: a launch costs its caller more in such questions than in itself)
+    (M, K), (b_rows, bcols), (lda, a_step1), (ldb, b_step1) = a.shape, b.shape, a.stride(), b.stride()
+    assert a_step1 == 1 and b_step1 == 1
+    kn, dt = b_layout == "kn", a.dtype
     if groups > 1 or a_step or out_step:
-        assert b.shape[0] % groups == 0 and epilogue == "store" and b_layout == "kn"
-        K = b.shape[0] // groups
-        a_step, out_step = a_step or K, out_step or b.shape[1]
-        assert a_step * (groups - 1) + K <= a.shape[1] and out_step >= b.shape[1]
-    if b_layout == "kn":
-        assert b.shape[0] == K * groups
-        bcols = b.shape[1]
+        assert b_rows % groups == 0 and epilogue == "store" and kn
+        K = b_rows // groups
+        a_step, out_step = a_step or K, out_step or bcols
+        assert a_step * (groups - 1) + K <= a.shape[1] and out_step >= bcols
+    if kn:
+        assert b_rows == K * groups
     else:
-        assert b.shape[1] == K
-        bcols = b.shape[0]
+        assert bcols == K
+        bcols = b_rows
     epi = _EPI[epilogue]
     gated = epi in (2, 7)
     N = bcols // 2 if gated else bcols
     if epi == 7:
-        assert bias is not None and bias.is_contiguous() and bias.numel() == bcols and bias.dtype == a.dtype and alpha > 0
+        assert bias is not None and bias.is_contiguous() and bias.numel() == bcols and bias.dtype == dt and alpha > 0
     if out is None:
-        out = torch.empty((M, groups * N), dtype=a.dtype, device=a.device)
-    assert out.stride(1) == 1 and out.shape[0] == M
-    assert out.shape[1] >= out_step * (groups - 1) + N if out_step else out.shape[1] == N
+        out = torch.empty((M, groups * N), dtype=dt, device=a.device)
+    (out_rows, out_cols), (ldc, c_step1), out_dt = out.shape, out.stride(), out.dtype
+    assert c_step1 == 1 and out_rows == M
+    assert out_cols >= out_step * (groups - 1) + N if out_step else out_cols == N
     if epi in (5, 6):
-        assert out.dtype == torch.float32
-    elif out.dtype != a.dtype:
-        assert epi == 0 and out.dtype == torch.float32
+        assert out_dt == torch.float32
+    elif out_dt != dt:
+        assert epi == 0 and out_dt == torch.float32
         epi = _EPI_STORE_F32
     if M == 0:
         return out
-    if a.dtype == torch.float32 or (a_step | out_step) % 8 or not _tensor_core_operands(a, b, out, N, K):
-        if epi == 1 or b_layout != "kn":
+    pa, pb, pc = a.data_ptr(), b.data_ptr(), out.data_ptr()
+    # sizes, pitches and base addresses the TMA-fed kernels need: 16-byte rows and bases; fp32 outputs are accessed 32 bytes at a time
+    whole = not ((N | K | lda | ldb | ldc) & 7 or (pa | pb) & 15 or pc & (31 if out_dt == torch.float32 else 15))
+    if dt == torch.float32 or (a_step | out_step) % 8 or not whole:
+        if epi == 1 or not kn:
             raise TypeError("gemm: epilogue 'add' and 'nk' weights need the tensor-core kernels")
-        assert b.dtype == a.dtype
+        assert b.dtype == dt
         _check(lib().blitz_gemm_simt(_p(a), a.stride(0), _p(b), b.stride(0), _p(out), out.stride(0), M, N, K, epi,
                                      N if gated else 0, _p(bias), alpha, beta, groups, a_step, out_step, _dt3(a), _stream()), "blitz_gemm_simt")
         return out
     if epi == 1:
-        assert residual is not None and residual.shape == (M, N) and residual.stride(0) == out.stride(0)
+        assert residual is not None and residual.shape == (M, N) and residual.stride(0) == ldc
     extra = bias if epi == 7 else residual
-    if b_layout == "kn" and not (bn or split_k or decode_split or pair_bnf or pair_upp or pair_nacc) and \
+    if kn and not (bn or split_k or decode_split or pair_bnf or pair_upp or pair_nacc) and \
             decode_path is None and pair_path is None and wide_path is None:
-        rc = lib().blitz_gemm_any(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(), out.stride(0), _p(extra), M, N, K, epi,
-                                  N if gated else 0, _dt(a), int(static_b), _scratch_of(a.get_device()), alpha, beta, groups, a_step, out_step,
+        rc = lib().blitz_gemm_any(pa, lda, pb, ldb, pc, ldc, None if extra is None else extra.data_ptr(), M, N, K, epi,
+                                  N if gated else 0, _dt(a), 1 if static_b else 0, _scratch_of(a.get_device()), alpha, beta, groups, a_step, out_step,
                                   _stream())
-        _check(rc, "blitz_gemm")
+        if rc:
+            _check(rc, "blitz_gemm")
         return out
     # the kernel that a hint asks for, or else the choice without hints
     layout = 0 if b_layout == "kn" else 1

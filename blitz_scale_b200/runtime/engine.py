@@ -354,12 +354,13 @@ class Engine:
             splits = self.choose_splits(singles, max(kv_lens[:singles]), sum(kv_lens[:singles])) if singles else 1
             m = self._views(T, rows, P, True, q_lens, splits=splits, kv_lens=kv_lens, singles=singles)
             with nvtx_range("step"):
-                self.runner.forward(m, with_head=False)
+                # (ahead of the pass, and without waiting for the stream: behind it the copy would hold back the head's launches)
                 starts = [0, *accumulate(q_lens)]
-                flat = [starts[row_of[b]] + p for b, p in src]
+                flat = torch.tensor([starts[row_of[b]] + p for b, p in src], dtype=torch.int32).to(self.device, non_blocking=True)
+                self.runner.forward(m, with_head=False)
                 parts = []
-                for i in range(0, len(flat), self.max_batch):
-                    idx = torch.tensor(flat[i:i + self.max_batch], dtype=torch.int32, device=self.device)
+                for i in range(0, flat.numel(), self.max_batch):
+                    idx = flat[i:i + self.max_batch]
                     parts.append(self.runner.logits_of(idx.numel(), idx).to(torch.float32, copy=True))
                 got = parts[0] if len(parts) == 1 else torch.cat(parts) if parts else None
         torch.cuda.current_stream().synchronize()       # the staging arrays are reused by the next pass
