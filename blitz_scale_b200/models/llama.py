@@ -147,7 +147,7 @@ class LlamaRunner:
         ops.rms_norm(res, self._w(l, "input_ln"), c.rms_eps, out=normed)
         ops.gemm(normed, self._w(l, "qkv"), static_b=True, out=qkv)
         ops.rope_kv_store(qkv, m.rows("pos", m.pos, T), m.rows("slot", m.slot, T), kv, q_heads=self.qh, kv_heads=self.kvh,
-                          head_dim=self.hd, page_size=self.page_size, rope_theta=c.rope_theta)
+                          head_dim=self.hd, page_size=self.page_size, rope_theta=c.rope_theta, static_meta=True)
         if m.is_prefill:
             self._prefill_attention(l, m)
         else:

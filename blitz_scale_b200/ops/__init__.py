@@ -364,6 +364,15 @@ def add_residual(residual: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
     return residual
 
 
+def to_fp32(x: torch.Tensor) -> torch.Tensor:
+    """A copy of ``x`` in fp32."""
+    if x.dtype not in _DT or not x.is_contiguous() or x.numel() % 8 or x.data_ptr() % 16:
+        return x.to(torch.float32, copy=True)
+    out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+    _check(lib().blitz_widen(_p(x), _p(out), x.numel(), _dt(x), _stream()), "blitz_widen")
+    return out
+
+
 def gather_last(x: torch.Tensor, indptr: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     B, H = indptr.numel() - 1, x.shape[1]
     if out is None:
@@ -395,14 +404,16 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
 
 
 def rope_kv_store(qkv: torch.Tensor, pos: torch.Tensor, slot: torch.Tensor, kv_layer: torch.Tensor, *, q_heads: int,
-                  kv_heads: int, head_dim: int, page_size: int, rope_theta: float) -> None:
-    """Rotate q and k of ``qkv`` in place and write rotated k and v to ``kv_layer`` ([pages, 2, page, kvh, hd])."""
+                  kv_heads: int, head_dim: int, page_size: int, rope_theta: float, static_meta: bool = False) -> None:
+    """Rotate q and k of ``qkv`` in place and write rotated k and v to ``kv_layer`` ([pages, 2, page, kvh, hd]).  ``static_meta``
+    promises that ``pos`` and ``slot`` are not written by kernels still running in this stream (the copy that brings them is no
+    kernel): the angles are then computed while the projection is still running."""
     T = qkv.shape[0]
     assert qkv.is_contiguous() and qkv.shape[1] == (q_heads + 2 * kv_heads) * head_dim
     assert pos.dtype == torch.int32 and slot.dtype == torch.int32
     max_pages = kv_layer.shape[0]
     _check(lib().blitz_rope_kv_store(_p(qkv), _p(pos), _p(slot), _p(kv_layer), T, q_heads, kv_heads, head_dim,
-                                     page_size, max_pages, rope_theta, _status_ptr(qkv), _dt(qkv),
+                                     page_size, max_pages, rope_theta, int(static_meta), _status_ptr(qkv), _dt(qkv),
                                      _stream()), "blitz_rope_kv_store")
 
 

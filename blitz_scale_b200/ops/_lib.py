@@ -88,7 +88,8 @@ def _declare(L: ctypes.CDLL) -> None:
     sig("blitz_gather_last", [c_p, c_p, c_p, c_i, c_i, c_i, c_p])
     sig("blitz_argmax", [c_p, c_i, c_i, c_i64, c_p, c_p, c_i, c_i, c_p])
     sig("blitz_sample", [c_p, c_i, c_i, c_i64, c_p, c_p, c_p, c_p, c_u64, c_p, c_i, c_p])
-    sig("blitz_rope_kv_store", [c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_f, c_p, c_i, c_p])
+    sig("blitz_widen", [c_p, c_p, c_i64, c_i, c_p])
+    sig("blitz_rope_kv_store", [c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_f, c_i, c_p, c_i, c_p])
     sig("blitz_attn_decode_workspace_bytes", [c_i, c_i, c_i, c_i], c_i64)
     sig("blitz_attn_decode", [c_p, c_i64, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_f,
                               c_i, c_i, c_i, c_i, c_f, c_p, c_p, c_i, c_p, c_i64, c_i, c_p, c_i, c_p])

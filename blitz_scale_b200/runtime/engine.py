@@ -345,7 +345,7 @@ class Engine:
             if src:
                 at = [row_of[b] for b, _ in src]
                 if at == list(range(len(at))):
-                    got = self.runner.logits[:len(at)].to(torch.float32, copy=True)
+                    got = ops.to_fp32(self.runner.logits[:len(at)])
                 else:
                     got = self.runner.logits[torch.tensor(at, device=self.device)].float()
         else:
@@ -361,7 +361,7 @@ class Engine:
                 parts = []
                 for i in range(0, flat.numel(), self.max_batch):
                     idx = flat[i:i + self.max_batch]
-                    parts.append(self.runner.logits_of(idx.numel(), idx).to(torch.float32, copy=True))
+                    parts.append(ops.to_fp32(self.runner.logits_of(idx.numel(), idx)))
                 got = parts[0] if len(parts) == 1 else torch.cat(parts) if parts else None
         torch.cuda.current_stream().synchronize()       # the staging arrays are reused by the next pass
         batch.advance(counts)
