@@ -14,6 +14,8 @@ int blitz_gemm_decode(const void*, int64_t, const void*, int64_t, void*, int64_t
                       float, float, cudaStream_t);
 int blitz_gemm_pair(const void*, int64_t, const void*, int64_t, void*, int64_t, const void*, int, int, int, int, int, int, int, int, int, int,
                     void*, int64_t, unsigned*, int, int*, float, float, cudaStream_t);
+int blitz_gemm_quad_supported(int, int, int, int, int);
+int blitz_gemm_quad(const void*, int64_t, const void*, int64_t, void*, int64_t, const void*, int, int, int, int, int, int, int*, float, cudaStream_t);
 int blitz_gemm_wide(const void*, int64_t, const void*, int64_t, void*, int64_t, const void*, int, int, int, int, int, int, int, int*,
                     float, float, int, int, int, cudaStream_t);
 
@@ -58,32 +60,48 @@ static bool pairs_are_better(int M, int N, int K, int epilogue, int groups) {
   return true;
 }
 
-// 129 to 256 rows: the weight-streaming kernel (1), whole or half tiles of 256 x 256 on CTA pairs (3), or those with K cut into parts
-// (2).  The first is as fast as its loads, 128 + M rows of 128 bytes per K block and CTA, with as many parts of K as clusters fit, and
-// adds an exchange of the parts' sums; the second takes a quarter of a microsecond per K block of a round of half tiles, 0.4 of whole ones.
-// Measured behind a small kernel with cold weights, us, 1 / 2 / 3:
-//   4096 x 4096 with a residual, 144 and 256 rows 15.9 / 21.0 / 20.3, 20.9 / 21.8 / 20.7;  6144 columns 18.0 / 23.3 / 21.0, 24.9 / 23.9 / 21.3
-//   4096 columns of K = 14336 32.4 / 39.8 / 59.0, 42.6 / 40.9 / 60.5;  2048 of it 19.3 / 49.9 / 57.4, 28.0 / 50.4 / 57.3
-//   128256 columns of K = 4096 181 / 214 / 202, 248 / 245 / 212;  8192 of K = 1024 11.4 / 14.5 / 9.7, 15.0 / 15.9 / 10.1
+// Whether K in halves over clusters of four (gemm_quad.cu) takes a product in one round: 33 of its clusters are resident on 148 SMs, and a
+// second round costs as much as the first.  More than 256 rows in one round, us, tiles of 128 rows (gemm_tcgen05.cu) / whole or half tiles on CTA
+// pairs / these: 300 rows x 2048 columns of K = 256 11.0 / 6.1 / 7.0, 512 13.2 / 7.0 / 7.5, 1024 16.0 / 9.4 / 8.5, 4096 17.9 / 19.6 / 13.0, 14336
+// 31.0 / 54.2 / 28.3;  1000 x 1024 of K = 2048 16.8 / 16.6 / 12.5;  3000 x 128 of K = 2048 17.3 / 15.4 / 12.6.  (Two rounds, 300 x 4096 of
+// K = 4096: 22.7 / 21.6 / 25.8.)
+static bool one_round_of_quads(int M, int N, int K, int epilogue) {
+  return (int64_t)((M + 255) / 256) * ((N + 127) / 128) <= 33 && blitz_gemm_quad_supported(M, N, K, 0, epilogue);
+}
+
+// 129 to 256 rows: the weight-streaming kernel (1), whole or half tiles of 256 x 256 on CTA pairs (3), those with K cut into parts (2), or
+// K in halves over clusters of four (4).  The first is as fast as its loads, 128 bytes per row and column of a K block and CTA, with as many parts of
+// K as clusters fit, and adds an exchange of the parts' sums; the third takes a quarter of a microsecond per K block of a round of half tiles, 0.4 of
+// whole ones; the fourth 0.13 to 0.23 per two K blocks, the more the more columns stream.  Estimates below are in us, without what
+// all of them cost.  Measured behind a small kernel with cold weights, us, 1 / 2 / 3 / 4:
+//   4096 x 4096 with a residual, 136 and 256 rows 16.1 / 20.8 / 20.4 / 13.8, 21.0 / 22.0 / 21.1 / 14.2;  6144 columns 17.9 / 23.5 / 21.0 / 25.4,
+//     25.2 / 24.0 / 21.5 / 26.0
+//   4096 columns of K = 14336 32.3 / 40.7 / 59.7 / 32.6, 42.4 / 41.6 / 60.1 / 34.0;  2048 of it 19.0 / 48.1 / 53.1 / 26.7, 27.3 / 47.6 / 54.2 / 28.0
+//   1024 columns of K = 4096 10.5 / 19.9 / 18.4 / 11.6, 13.3 / 20.1 / 18.3 / 11.6;  4096 of K = 1024 11.6 / 15.6 / 9.3 / 8.3, 15.2 / 16.3 / 9.6 / 8.8
+//   128256 columns of K = 4096, 144 and 256 181 / 214 / 202 / -, 248 / 245 / 212 / -;  8192 of K = 1024 11.4 / 14.5 / 9.7, 15.0 / 15.9 / 10.1
 //   6144 columns of K = 8192, 200 and 256 rows 34.5 / 35.6 / 38.8, 40.5 / 35.7 / 39.3
 // Gated units need both accumulators' weights at once: fewer stages, and beyond 192 rows room for fewer parts.  144, 192 and 256 rows:
 //   14336 x 4096 49.3 / 57.0 / 56.6, 54.3 / 57.5 / 57.7, 66.7 / 58.3 / 58.2;  8192 x 4096 36.0 / 35.9 / 34.8, 38.3 / 36.7 / 35.5, 62.1 / 37.4 / 36.2
 //   2816 x 2048 15.7 / 19.1 / 14.3, 17.5 / 19.3 / 14.5, 36.1 / 19.1 / 15.1
-// Over 32 shapes of which one in six is of a gated unit: within 1 % of the fastest of the three on average, 28 % with (2) for all.
+// Over 40 shapes at 3 to 7 numbers of rows: within 1 % of the fastest on average; (2) for all of them: 28 % (without (4) among the others).
 int blitz_gemm_few_rows(int M, int N, int K, int epilogue) {
   const int tiles = (N + 127) / 128, wide = (N + 255) / 256, kb = (K + 63) / 64;
   if (epilogue == 2 || epilogue == 7) return M <= 192 && tiles > 74 ? 1 : 3;
-  if (M > 224 && K >= 8192 && 2 * wide <= 74 && (int64_t)N * K >= 48 << 20) return 2;
+  const bool quads = one_round_of_quads(M, N, K, epilogue);
+  if (!quads && M > 224 && K >= 8192 && 2 * wide <= 74 && (int64_t)N * K >= 48 << 20) return 2;
   static const int clusters[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};  // of that many CTAs that 148 SMs hold
   int parts = 148 / tiles < 8 ? 148 / tiles : 8;
   if (parts > kb) parts = kb;
   while (parts > 1 && tiles > clusters[parts]) --parts;
   if (parts < 1) parts = 1;
-  const float exchange = parts > 1 ? 0.027f * M : epilogue == 1 ? 0.07f * M : 1.5f;  // (one part: a residual's loads are exposed)
-  const float streaming = 1.25e-3f * (128 + M) * ((kb + parts - 1) / parts) * ((tiles + 147) / 148) + exchange;
+  const bool all = parts > 1 && parts * tiles >= 120;  // (what nearly all SMs load together is less than what each can)
+  const float exchange = parts > 1 ? 0.027f * M + (all ? 2.f : 0.f) : epilogue == 1 ? 0.07f * M : 1.5f;  // (one part: a residual's loads are exposed)
+  const float streaming = ((kb + parts - 1) / parts) * ((tiles + 147) / 148) * (0.18f + 0.0011f * M) * (all ? 1.2f : 1.f) + exchange;
   const int rest = wide % 74;
   const float rounds = 2 * wide <= 74 ? 0.625f : wide / 74 + (rest == 0 ? 0.f : 2 * rest <= 74 ? 0.65f : 1.f);
-  return streaming <= 0.4f * kb * rounds + 1.5f ? 1 : 3;
+  const float whole = 0.4f * kb * rounds + 1.5f;
+  const float halves = quads ? 3.5f + ((kb + 1) / 2) * (0.13f + 0.0031f * tiles) : 1e30f;
+  return halves < whole && halves < streaming ? 4 : streaming <= whole ? 1 : 3;
 }
 
 // Which kernel takes a product with "in,out" weights: 0 the tiled one, 1 weight-streaming (its activation tile is read again with every
@@ -101,8 +119,11 @@ int blitz_gemm_any(const void* A, int64_t lda, const void* B, int64_t ldb, void*
                    int a_step, int c_step, cudaStream_t stream) {
   if (!s) return -1;
   int kernel = blitz_gemm_choice(M, N, K, epilogue, groups);
-  if (kernel == 2) kernel = blitz_gemm_few_rows(M, N, K, epilogue);  // (what one of the three takes the others take too)
+  if (kernel == 2) kernel = blitz_gemm_few_rows(M, N, K, epilogue);  // (what (2) takes (1) and (3) take too)
+  else if (kernel != 1 && groups == 1 && M > 256 && one_round_of_quads(M, N, K, epilogue)) kernel = K > 512 ? 4 : 3;
   switch (kernel) {
+    case 4:
+      return blitz_gemm_quad(A, lda, B, ldb, C, ldc, R, M, N, K, epilogue, dtype, static_b, s->status, alpha, stream);
     case 1:
       return blitz_gemm_decode(A, lda, B, ldb, C, ldc, R, M, N, K, epilogue, up_col_off, dtype, static_b, 0, s->status, alpha, beta, stream);
     case 2:

@@ -190,7 +190,7 @@ def _scratch_of(index: int) -> int:
 def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *, residual=None,
          epilogue: str = "store", alpha: float = 1.0, beta: float = 1.0, bias: Optional[torch.Tensor] = None, groups: int = 1, a_step: int = 0, out_step: int = 0, b_layout: str = "kn", bn: int = 0, split_k: int = 0, static_b: bool = False,
          decode_path: Optional[bool] = None, decode_split: int = 0, pair_path: Optional[bool] = None,
-         pair_bnf: int = 0, pair_upp: int = 0, pair_nacc: int = 0, wide_path: Optional[bool] = None) -> torch.Tensor:
+         pair_bnf: int = 0, pair_upp: int = 0, pair_nacc: int = 0, wide_path: Optional[bool] = None, quad_path: bool = False) -> torch.Tensor:
     """``out = a @ b`` on tcgen05 with a fused epilogue.
 
     a: [M, K].  b: [K, N] when ``b_layout == 'kn'`` (weights stored in,out) or [N, K] for ``'nk'``.
@@ -209,7 +209,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     ``pair_path`` forces (True) or forbids (False) the last for any M, ``pair_bnf`` / ``pair_nacc`` / ``pair_upp`` override its tile width, tiles per pair and units per pair.
 
     More rows with 'kn' weights go to the kernel whose CTA pairs walk 256 x 256 tiles; ``wide_path`` forces (True) or forbids
-    (False) it for any M.
+    (False) it for any M.  Where few column tiles of a deep product would leave pairs idle, two pairs take half of K each;
+    ``quad_path`` forces that kernel for any M.
 
     ``out`` may be fp32 with 16-bit operands (the accumulator is stored unrounded); epilogue 'axpy' adds
     ``alpha * (a @ b)`` to an fp32 ``out`` (residual streams kept in 32 bits); 'softcap' stores
@@ -265,7 +266,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
         assert residual is not None and residual.shape == (M, N) and residual.stride(0) == ldc
     extra = bias if epi == 7 else residual
     if kn and not (bn or split_k or decode_split or pair_bnf or pair_upp or pair_nacc) and \
-            decode_path is None and pair_path is None and wide_path is None:
+            decode_path is None and pair_path is None and wide_path is None and not quad_path:
         rc = lib().blitz_gemm_any(pa, lda, pb, ldb, pc, ldc, None if extra is None else extra.data_ptr(), M, N, K, epi,
                                   N if gated else 0, _dt(a), 1 if static_b else 0, _scratch_of(a.get_device()), alpha, beta, groups, a_step, out_step,
                                   _stream())
@@ -274,6 +275,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
         return out
     # the kernel that a hint asks for, or else the choice without hints
     layout = 0 if b_layout == "kn" else 1
+    if quad_path:
+        assert groups == 1 and lib().blitz_gemm_quad_supported(M, N, K, layout, epi)
+        _check(lib().blitz_gemm_quad(pa, lda, pb, ldb, pc, ldc, _p(extra), M, N, K, epi, _dt(a), int(static_b), _status_ptr(a), alpha, _stream()),
+               "blitz_gemm_quad")
+        return out
     choice = lib().blitz_gemm_choice(M, N, K, epi, groups) if layout == 0 and bn == 0 and split_k == 0 else 0
     use_dec, use_pair, use_wide = choice == 1, choice == 2, choice == 3
     if decode_path is not None:

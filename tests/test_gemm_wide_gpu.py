@@ -106,6 +106,6 @@ def test_between_decode_batches_and_prompts(M, N, K, epi):
         outs.append(out)
     ops.check_status()
     used = ops.lib().blitz_gemm_few_rows(M, N, K, {"store": 0, "add": 1, "silu_mul": 2}[epi])
-    assert used in (1, 2, 3)
+    assert used in (1, 2, 3, 4)
     if used == 2:
         assert torch.equal(*outs)
