@@ -99,8 +99,6 @@ __device__ __forceinline__ float dec_f32<__nv_bfloat16>(__nv_bfloat16 v) { retur
 template <>
 __device__ __forceinline__ float dec_f32<__half>(__half v) { return __half2float(v); }
 
-__device__ __forceinline__ float dec_silu(float x) { return x / (1.0f + __expf(-x)); }
-
 // The epilogue takes 8 tokens of a thread's feature at a time in rolled loops: its instructions run once per launch, right behind a
 // stream of weights that has displaced them from every cache, so each line of code costs a fetch of its own.  From the last product
 // to the last store, us, 32 tokens unrolled / eight in a loop: 4096 x 4096 with 1 and 61 tokens 7.9 / 2.3 and 11.8 / 3.8, 4096 x 14336
@@ -141,11 +139,13 @@ __device__ __forceinline__ void dec_store8(const DecGemmParams& p, const float (
                                            float bias_g, float bias_u, int n, int t, int t_end) {
   const int64_t at = static_cast<int64_t>(t) * p.ldc + n;
   const float inv = EPI == 6 ? 1.f / p.alpha : 0.f;
+  float unit[8];
+  if (EPI == 2) silu_mul(g, u, unit);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     float v = g[i];
     if (EPI == 1) v += old[i];
-    if (EPI == 2) v = dec_silu(t + i < t_end ? v : 1.f) * u[i];  // (a quotient of zero leaves the division's fast path, for the whole warp)
+    if (EPI == 2) v = unit[i];
     if (EPI == 5) v = old[i] + p.alpha * v;
     if (EPI == 6) v = p.alpha * ptx::tanh_ex2(v * inv);
     if (EPI == kEpiClampGlu) v = clamp_glu(v + bias_g, u[i] + bias_u, p.alpha, p.beta);

@@ -4,6 +4,7 @@
 //   7   clamped gated unit with biases:  g <- min(g + b_g, limit),  u <- clamp(u + b_u, -limit, limit),
 //       g sigmoid(beta g) (u + 1)
 #pragma once
+#include "ptx.cuh"
 #include "scalar.cuh"
 
 namespace blitz {
@@ -11,6 +12,48 @@ namespace blitz {
 constexpr int kEpiClampGlu = 7;
 __host__ __device__ constexpr bool epi_gated(int epi) { return epi == 2 || epi == kEpiClampGlu; }
 __host__ __device__ constexpr bool epi_f32(int epi) { return epi >= 4 && epi <= 6; }
+
+// N silus of gate values times up values: x / (1 + e^-x) * u.  The quotient is Markstein's (IBM J. Res. Dev. 34, 1990): an approximate
+// reciprocal refined by one residual, and the quotient by its own, a dozen instructions without a branch, whose result is the IEEE quotient
+// but for an occasional last bit.  The compiler's division takes a branch per element, and leaves its fast path for a quotient of
+// zero.  What this form does not hold for, infinities, NaN and denominators beyond 2^126, is divided by the compiler's.
+// (__fdividef: off by two units, and zero for those denominators.)
+template <int N>
+__device__ __forceinline__ void silu_mul(const float (&x)[N], const float (&u)[N], float (&y)[N]) {
+  float d[N], most = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) y[i] = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    d[i] = 1.f + __expf(-x[i]);
+    const float larger = fmaxf(fabsf(x[i]), d[i]);
+    most = larger < 8e37f ? most : INFINITY;
+  }
+  if (most == 0.f) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      float r = ptx::rcp_approx(d[i]);
+      r = fmaf(fmaf(-d[i], r, 1.f), r, r);
+      const float q = x[i] * r;
+      y[i] = fmaf(fmaf(-d[i], q, x[i]), r, q) * u[i];
+    }
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < N; ++i) {  // (one division's code for all of them; indexed by constants, the arrays stay in registers)
+      float a = 0.f, b = 1.f, c = 0.f;
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        if (j != i) continue;
+        a = x[j];
+        b = d[j];
+        c = u[j];
+      }
+      const float z = a / b * c;
+#pragma unroll
+      for (int j = 0; j < N; ++j) y[j] = j == i ? z : y[j];
+    }
+  }
+}
 
 __device__ __forceinline__ float clamp_glu(float g, float u, float limit, float beta) {
   g = fminf(g, limit);

@@ -152,8 +152,6 @@ __device__ __forceinline__ float2 unpack2<__half>(uint32_t u) {
   return __half22float2(*reinterpret_cast<__half2*>(&u));
 }
 
-__device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
-
 // Epilogue of 32 consecutive output columns of one row: acc (and up for silu_mul) -> C.
 template <typename T, int EPI>
 __device__ __forceinline__ void store_chunk(const GemmParams& p, const float (&acc)[32], const float (&up)[32], int row,
@@ -189,8 +187,10 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const float (&a
 #pragma unroll
     for (int i = 0; i < 16; ++i) out[i] = pack2<T>(y[2 * i], y[2 * i + 1]);
   } else if (epi_gated(EPI)) {
+    float y[32];
+    silu_mul(acc, up, y);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) out[i] = pack2<T>(silu_f(acc[2 * i]) * up[2 * i], silu_f(acc[2 * i + 1]) * up[2 * i + 1]);
+    for (int i = 0; i < 16; ++i) out[i] = pack2<T>(y[2 * i], y[2 * i + 1]);
   } else if (EPI == kEpiAdd) {
     const T* Rp = reinterpret_cast<const T*>(p.R);
 #pragma unroll

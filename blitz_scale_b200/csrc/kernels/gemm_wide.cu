@@ -353,14 +353,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           clamp_glu32<T>(reinterpret_cast<const T*>(p.R), p.up_col_off, n + ch * 32, p.N, p.alpha, p.beta, g, up, y);
           pair_convert32<T, 0>(y, up, res, o4);
         } else if (EPI == 2) {
-          // divided as IEEE does: __fdividef is off by two units and answers zero for denominators beyond 2^126 (14336 x 4096 with it and
-          // so, us: 300 rows 84.5 and 88.3, 1574 rows 264.5 and 272.0, within the spread at 8192)
           float y[32];
-#pragma unroll
-          for (int k = 0; k < 32; ++k) {
-            const float x = row_ok ? g[k] : 1.f;  // a quotient of zero leaves the division's fast path, for the whole warp
-            y[k] = x / (1.f + __expf(-x)) * up[k];
-          }
+          silu_mul(g, up, y);
           pair_convert32<T, 0>(y, up, res, o4);
         } else {
           pair_convert32<T, EPI>(g, up, res, o4);
