@@ -34,10 +34,12 @@ struct RopeStoreParams {
   int* status;
 };
 
+// (Wide accesses without a norm: 40 registers, six blocks an SM; a token's chain of loads, sines and stores is waited for by more of them.
+// 4096 tokens of 16 + 4 heads of 128, 64 dimensions rotated: 24.0 us with four, 20.2 so.)
 enum RopeMode : int { kRopeAny = 0, kRopeWidePairs = 1, kRopeWideHalves = 2 };  // wide: eight elements per access
 
 template <typename T, int MODE, bool NORM>
-__global__ void __launch_bounds__(NORM && MODE == kRopeWideHalves ? 1024 : 256, NORM && MODE == kRopeWideHalves ? 1 : MODE == kRopeAny ? 5 : 4) rope_store_kernel(const RopeStoreParams p) {
+__global__ void __launch_bounds__(NORM && MODE == kRopeWideHalves ? 1024 : 256, NORM && MODE == kRopeWideHalves ? 1 : MODE == kRopeAny ? 5 : NORM ? 4 : 6) rope_store_kernel(const RopeStoreParams p) {
   ptx::griddep_launch_dependents();
   ptx::griddep_wait();
   extern __shared__ float s_ang[];  // [rot_dims / 2] cos, [rot_dims / 2] sin
