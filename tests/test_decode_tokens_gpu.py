@@ -5,7 +5,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 25, 61, 121, 128, 249])
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 8, 9, 16, 17, 25, 61, 121, 128, 249])
 @pytest.mark.parametrize("split", [1, 2, 3, 4, 8])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_token_groups(M, split, dtype):
