@@ -381,14 +381,14 @@ __global__ void sample_kernel(const T* __restrict__ logits, int vocab, int64_t s
 // A negative slot skips the cache write (bounds: slot < max_pages * page_size
 // is checked; a bad slot sets *status and skips).
 constexpr int kRopeMaxHalf = 128;  // head_dim <= 256
-template <typename T>
+template <typename T, bool STATIC>
 __global__ void rope_kv_store_kernel(T* __restrict__ qkv, const int32_t* __restrict__ pos,
                                      const int32_t* __restrict__ slot, T* __restrict__ kv_layer, int q_heads,
                                      int kv_heads, int head_dim, int page_size, int max_pages, float log2_theta,
-                                     int static_meta, int* __restrict__ status) {
+                                     int* __restrict__ status) {
   ptx::griddep_launch_dependents();
-  // positions that no kernel in flight writes: slots and angles are ready when the projection is (one row: 3.6 -> 2.0 us behind it)
-  if (!static_meta) ptx::griddep_wait();
+  // STATIC: positions that no kernel in flight writes: slots and angles are ready when the projection is (one row: 3.6 -> 2.0 us behind it)
+  if (!STATIC) ptx::griddep_wait();
   const int t = blockIdx.x;
   const int half = head_dim >> 1;
   const int vec_per_half = half >> 3;
@@ -413,7 +413,7 @@ __global__ void rope_kv_store_kernel(T* __restrict__ qkv, const int32_t* __restr
     const float inv_freq = exp2f(-(2.0f * static_cast<float>(i) / static_cast<float>(head_dim)) * log2_theta);
     sincosf(p * inv_freq, &s_sn[i], &s_cs[i]);
   }
-  if (static_meta) ptx::griddep_wait();
+  if (STATIC) ptx::griddep_wait();
   __syncthreads();
   const int rot_items = (q_heads + kv_heads) * vec_per_half;
   for (int it = threadIdx.x; it < rot_items; it += blockDim.x) {
@@ -560,9 +560,9 @@ int blitz_rope_kv_store(void* qkv, const int32_t* pos, const int32_t* slot, void
   if ((head_dim & 15) || head_dim > 2 * kRopeMaxHalf) return -1;
   const float log2_theta = log2f(rope_theta);
   cudaError_t blitz_last = cudaSuccess;
-  BLITZ_DISPATCH_DTYPE(dtype, (blitz_last = launch_pdl(rope_kv_store_kernel<T>, dim3(num_tokens), dim3(256), 0, stream,
+  BLITZ_DISPATCH_DTYPE(dtype, (blitz_last = launch_pdl(static_meta ? rope_kv_store_kernel<T, true> : rope_kv_store_kernel<T, false>, dim3(num_tokens), dim3(256), 0, stream,
                                   (T*)qkv, pos, slot, (T*)kv_layer, q_heads, kv_heads, head_dim, page_size, max_pages,
-                                  log2_theta, static_meta, status)));
+                                  log2_theta, status)));
   return (int)blitz_last;
 }
 

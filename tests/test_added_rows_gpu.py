@@ -72,3 +72,4 @@ def test_rotation_with_positions_known_ahead(T):
         outs.append((qkv, kv))
     assert all(torch.equal(a, b) for a, b in zip(*outs))
     ops.check_status()
+
