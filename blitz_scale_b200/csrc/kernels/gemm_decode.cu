@@ -1,4 +1,5 @@
-// Weight-streaming tcgen05 GEMM for decode batches on sm_100a: it takes M <= 256 tokens, the rule in gemm_any.cu sends it 128 at most.
+// Weight-streaming tcgen05 GEMM for decode batches on sm_100a: M <= 256 tokens, all products of 128 at most and, beyond, those that the
+// rule in gemm_any.cu sends here.
 //
 //   C[M,N] = X[M,K] * W[K,N]      W in the serving layout ("in,out", N contiguous), 16-bit, fp32 accumulation
 //
@@ -524,8 +525,9 @@ static cudaError_t launch_dec(const CUtensorMap& tx, const CUtensorMap& tw, DecG
   const int halves = epi_gated(EPI) ? 2 : 1;
   const int stage_bytes = DecCfg::x_stage_bytes(p.npad) + halves * kDecTile * kDecBK * 2;
   // One CTA per SM.  BLITZ_DECODE_OCC=2 runs two CTAs per SM on half the shared memory each (so that one CTA's
-  // set-up or reduction overlaps the other's weight stream); measured on B200 it changes nothing (15.2 vs 15.3 us
-  // at M=16, N=6144, K=4096), so it stays an experiment switch.
+  // set-up or reduction overlaps the other's weight stream); alone that changes nothing (15.2 vs 15.3 us
+  // at M=16, N=6144, K=4096), and less shared memory lets two CTAs of one grid share an SM while others idle (a decode step
+  // of Llama-3-8B 3.6 -> 4.0 to 4.5 ms), so it stays an experiment switch.
   int occ = 1;
   if (occ_env == 1 || occ_env == 2) occ = occ_env;
   if (DecCfg::num_stages(p.npad, halves * kDecTile * kDecBK * 2, DecCfg::kSmemBytesHalf) < 2) occ = 1;

@@ -14,6 +14,9 @@
 // Each CTA loads only its own halves with plain per-CTA TMA (no cluster multicast anywhere); the bytes of both
 // are counted on the even CTA's barrier, whose elected thread issues the instructions for the pair.
 //
+// Of the products that name no kernel, the rule in gemm_any.cu sends here only those of more than 224 rows that are deep and too wide for K in
+// halves (256 rows x 6144 columns of K = 8192, us: 40.5 weight-streaming, 35.7 here, 39.3 on whole tiles); others ask for parts or tiles.
+//
 // Scheduling.  Work is cut into units of (super tile, 64-wide K block); pair p takes the units
 // [p*upp, (p+1)*upp) in order, so all pairs finish together whatever the tile count (stream-K).  A pair whose
 // range starts inside a super tile contributes fp32 partials for it (its FIRST piece of work: written to

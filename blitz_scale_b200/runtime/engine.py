@@ -39,7 +39,7 @@ def decode_parts(rows: int, kv_heads: int, longest: int, tokens: int) -> int:
     into n parts each; 0: equal ranges of all of them, whatever their lengths.
 
     One of the 296 halves of the SMs takes a chunk of 64 keys in 0.7 us until they wait for HBM (all of them at work: 1.5 us).  Parts cost
-    a merge kernel, 2.8 us, so they have to save seven chunks, beyond eight parts two with every doubling, and more where they bring
+    a merge kernel, 2.6 us, so they have to save seven chunks, beyond eight parts two with every doubling, and more where they bring
     second halves of SMs to work: those start late and share what their SM is given.  Ranges cost 7 us (pieces, tickets, merges), so
     they pay where the end of a launch would otherwise leave most halves idle for longer than that.  Four and eight parts pay up to 256
     of them: behind a small kernel they cost a microsecond or two more than half as many, but whole
