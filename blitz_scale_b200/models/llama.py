@@ -48,7 +48,7 @@ class StepMeta:
     num_splits: int = 1
     seq_slot: Optional[torch.Tensor] = None                 # [B] state slot of every row (-1: padding row)
     singles: int = 0                                        # of a ragged step: leading rows with one token that go through the decode kernels
-    _views: Dict = field(default_factory=dict)              # see `view`
+    _views: Dict = field(default_factory=dict, init=False, repr=False, compare=False)   # see `view`; a copy with other sizes has its own
 
     def view(self, key, base: torch.Tensor, make: Callable):
         """``make(base)``, made once in this pass: a view costs its caller 1.3 us, as much as half a launch, and the layers of a pass ask
