@@ -372,7 +372,7 @@ def add_residual(residual: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
 
 def to_fp32(x: torch.Tensor) -> torch.Tensor:
     """A copy of ``x`` in fp32."""
-    if x.dtype not in _DT or not x.is_contiguous() or x.numel() % 8 or x.data_ptr() % 16:
+    if not x.is_cuda or x.dtype not in _DT or not x.is_contiguous() or x.numel() % 8 or x.data_ptr() % 16:
         return x.to(torch.float32, copy=True)
     out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
     _check(lib().blitz_widen(_p(x), _p(out), x.numel(), _dt(x), _stream()), "blitz_widen")
