@@ -48,6 +48,9 @@ class StepMeta:
     num_splits: int = 1
     seq_slot: Optional[torch.Tensor] = None                 # [B] state slot of every row (-1: padding row)
     singles: int = 0                                        # of a ragged step: leading rows with one token that go through the decode kernels
+    # `pos` and `slot` are read ahead of the pass's own order: no kernel that may still run when the pass starts writes them.  Whoever
+    # makes a step whose positions come by a copy may say so; a step whose positions a kernel writes leaves it.
+    static_positions: bool = False
     _views: Dict = field(default_factory=dict, init=False, repr=False, compare=False)   # see `view`; a copy with other sizes has its own
 
     def view(self, key, base: torch.Tensor, make: Callable):
@@ -147,7 +150,7 @@ class LlamaRunner:
         ops.rms_norm(res, self._w(l, "input_ln"), c.rms_eps, out=normed)
         ops.gemm(normed, self._w(l, "qkv"), static_b=True, out=qkv)
         ops.rope_kv_store(qkv, m.rows("pos", m.pos, T), m.rows("slot", m.slot, T), kv, q_heads=self.qh, kv_heads=self.kvh,
-                          head_dim=self.hd, page_size=self.page_size, rope_theta=c.rope_theta, static_meta=True)
+                          head_dim=self.hd, page_size=self.page_size, rope_theta=c.rope_theta, static_meta=m.static_positions)
         if m.is_prefill:
             self._prefill_attention(l, m)
         else:

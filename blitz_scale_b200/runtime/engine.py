@@ -155,7 +155,8 @@ class Engine:
         if prefill and work is None:
             # leading single tokens that go through the decode kernels
             work = ops.prefill_work_list(seq_lens, kv_lens, self.page_size, self.device, skip=singles)
-        return StepMeta(kv_lens_host=kv_lens, prefill_work=work,
+        # (positions and slots come by the copy in _h2d)
+        return StepMeta(kv_lens_host=kv_lens, prefill_work=work, static_positions=True,
                         ids=d[L.ids:L.ids + T], pos=d[L.pos:L.pos + T], slot=d[L.slot:L.slot + T],
                         page_indices=d[L.page_indices:L.page_indices + max(P, 1)],
                         page_indptr=d[L.page_indptr:L.page_indptr + B + 1],

@@ -75,7 +75,7 @@ class MetaBuilder:
         ids, pos, slot, tokptr, pgptr, last, pidx = self._views(T, B, len(idx))
         return StepMeta(ids=ids, pos=pos, slot=slot, page_indices=pidx, page_indptr=pgptr, last_page_len=last,
                         tok_indptr=tokptr, seq_lens_host=[len(p) for p in prompts], is_prefill=True, batch=B,
-                        num_tokens=T)
+                        num_tokens=T, static_positions=True)
 
     def decode(self, last_tokens, seq_lens, page_tables, pad_to: int = 0, num_splits: int = 1) -> StepMeta:
         """seq_lens[b] = tokens already in the cache; the new token is written at that position.
@@ -117,4 +117,4 @@ class MetaBuilder:
         ids, pos, slot, tokptr, pgptr, last, pidx = self._views(Bp, Bp, self.max_pages)
         return StepMeta(ids=ids, pos=pos, slot=slot, page_indices=pidx, page_indptr=pgptr, last_page_len=last,
                         tok_indptr=None, seq_lens_host=[], is_prefill=False, batch=Bp, num_tokens=Bp,
-                        num_splits=num_splits)
+                        num_splits=num_splits, static_positions=True)
