@@ -55,7 +55,9 @@ class StepMeta:
 
     def view(self, key, base: torch.Tensor, make: Callable):
         """``make(base)``, made once in this pass: a view costs its caller 1.3 us, as much as half a launch, and the layers of a pass ask
-        for the same ones.  (The entry holds ``base``: another tensor under this key makes another view.)"""
+        for the same ones.  ``make`` may depend on ``key``, which says all that sets one view of ``base`` apart from another, and on the
+        number of tokens.  (The entry holds ``base``: another tensor under this key makes another view.)"""
+        key = (key, self.num_tokens)
         have = self._views.get(key)
         if have is None or have[0] is not base:
             have = self._views[key] = (base, make(base))
@@ -63,9 +65,9 @@ class StepMeta:
 
     def rows(self, key, base: torch.Tensor, n: int) -> torch.Tensor:
         """The first n rows of ``base``."""
-        have = self._views.get((key, n))
+        have = self._views.get(("rows", key, n))
         if have is None or have[0] is not base:
-            have = self._views[(key, n)] = (base, base[:n])
+            have = self._views[("rows", key, n)] = (base, base[:n])
         return have[1]
 
 
