@@ -396,10 +396,8 @@ __global__ void rope_kv_store_kernel(T* __restrict__ qkv, const int32_t* __restr
   T* row = qkv + t * row_stride;
   const float p = static_cast<float>(pos[t]);
   int s = slot[t];
-  if (s >= max_pages * page_size) {
-    if (threadIdx.x == 0 && status) atomicCAS(status, 0, kStatusBadIndex);
-    s = -1;
-  }
+  const bool bad = s >= max_pages * page_size;
+  if (bad) s = -1;
   const int page = s >= 0 ? s / page_size : 0;
   const int off = s >= 0 ? s % page_size : 0;
   const int64_t plane = static_cast<int64_t>(page_size) * kv_heads * head_dim;
@@ -414,6 +412,7 @@ __global__ void rope_kv_store_kernel(T* __restrict__ qkv, const int32_t* __restr
     sincosf(p * inv_freq, &s_sn[i], &s_cs[i]);
   }
   if (STATIC) ptx::griddep_wait();
+  if (bad && threadIdx.x == 0 && status) atomicCAS(status, 0, kStatusBadIndex);  // (behind the wait, as every write)
   __syncthreads();
   const int rot_items = (q_heads + kv_heads) * vec_per_half;
   for (int it = threadIdx.x; it < rot_items; it += blockDim.x) {
