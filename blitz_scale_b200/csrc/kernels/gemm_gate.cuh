@@ -5,6 +5,7 @@
 //       g sigmoid(beta g) (u + 1)
 #pragma once
 #include "ptx.cuh"
+#include "quotient.cuh"
 #include "scalar.cuh"
 
 namespace blitz {
@@ -13,11 +14,9 @@ constexpr int kEpiClampGlu = 7;
 __host__ __device__ constexpr bool epi_gated(int epi) { return epi == 2 || epi == kEpiClampGlu; }
 __host__ __device__ constexpr bool epi_f32(int epi) { return epi >= 4 && epi <= 6; }
 
-// N silus of gate values times up values: x / (1 + e^-x) * u.  The quotient is Markstein's (IBM J. Res. Dev. 34, 1990): an approximate
-// reciprocal refined by one residual, and the quotient by its own, a dozen instructions without a branch, whose result is the IEEE quotient
-// but for an occasional last bit.  The compiler's division takes a branch per element, and leaves its fast path for a quotient of
-// zero.  What this form does not hold for, infinities, NaN and denominators beyond 2^126, is divided by the compiler's.
-// (__fdividef: off by two units, and zero for those denominators.)
+// N silus of gate values times up values: x / (1 + e^-x) * u, the quotient as IEEE has it (quotient.cuh; tests/native/quotient_check.cpp
+// compares the two) without a branch per element: the compiler's division takes one, and leaves its fast path for a quotient of zero.
+// Infinities, NaN and denominators beyond 8e37 are divided by the compiler's.
 template <int N>
 __device__ __forceinline__ void silu_mul(const float (&x)[N], const float (&u)[N], float (&y)[N]) {
   float d[N], most = 0.f;
@@ -32,10 +31,7 @@ __device__ __forceinline__ void silu_mul(const float (&x)[N], const float (&u)[N
   if (most == 0.f) {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      float r = ptx::rcp_approx(d[i]);
-      r = fmaf(fmaf(-d[i], r, 1.f), r, r);
-      const float q = x[i] * r;
-      y[i] = fmaf(fmaf(-d[i], q, x[i]), r, q) * u[i];
+      y[i] = refined_quotient(x[i], d[i], ptx::rcp_approx(d[i])) * u[i];
     }
   } else {
 #pragma unroll 1
