@@ -27,20 +27,25 @@ template <>
 __device__ __forceinline__ float2 pair_unpack2<__half>(uint32_t u) {
   return __half22float2(*reinterpret_cast<__half2*>(&u));
 }
-// fast-math sigmoid: the epilogue after the last UMMA is exposed time, and an IEEE division per element is a long
-// dependent chain on a handful of warps
-__device__ __forceinline__ float pair_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
-
 // 32 consecutive output columns of one row -> four 16-byte chunks.  EPI: 0 store, 1 add residual (its 32 values
-// come in `res`, read before the accumulator was waited for), 2 silu(g) * u.
+// come in `res`, read before the accumulator was waited for), 2 silu(g) * u, eight at a time.
 template <typename T, int EPI>
 __device__ __forceinline__ void pair_convert32(const float (&g)[32], const float (&u)[32], const uint4 (&res)[4],
                                                uint4 (&out4)[4]) {
   uint32_t out[16];
   if (EPI == 2) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
-      out[i] = pair_pack2<T>(pair_silu(g[2 * i]) * u[2 * i], pair_silu(g[2 * i + 1]) * u[2 * i + 1]);
+    for (int j = 0; j < 4; ++j) {
+      float a[8], b[8], y[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        a[i] = g[8 * j + i];
+        b[i] = u[8 * j + i];
+      }
+      silu_mul(a, b, y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) out[4 * j + i] = pair_pack2<T>(y[2 * i], y[2 * i + 1]);
+    }
   } else if (EPI == 1) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
