@@ -187,10 +187,18 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const float (&a
 #pragma unroll
     for (int i = 0; i < 16; ++i) out[i] = pack2<T>(y[2 * i], y[2 * i + 1]);
   } else if (epi_gated(EPI)) {
-    float y[32];
-    silu_mul(acc, up, y);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) out[i] = pack2<T>(y[2 * i], y[2 * i + 1]);
+    for (int j = 0; j < 4; ++j) {  // (eight at a time: fewer registers)
+      float a[8], b[8], y[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        a[i] = acc[8 * j + i];
+        b[i] = up[8 * j + i];
+      }
+      silu_mul(a, b, y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) out[4 * j + i] = pack2<T>(y[2 * i], y[2 * i + 1]);
+    }
   } else if (EPI == kEpiAdd) {
     const T* Rp = reinterpret_cast<const T*>(p.R);
 #pragma unroll

@@ -352,10 +352,6 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           float y[32];
           clamp_glu32<T>(reinterpret_cast<const T*>(p.R), p.up_col_off, n + ch * 32, p.N, p.alpha, p.beta, g, up, y);
           pair_convert32<T, 0>(y, up, res, o4);
-        } else if (EPI == 2) {
-          float y[32];
-          silu_mul(g, up, y);
-          pair_convert32<T, 0>(y, up, res, o4);
         } else {
           pair_convert32<T, EPI>(g, up, res, o4);
         }
