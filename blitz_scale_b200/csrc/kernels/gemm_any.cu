@@ -1,7 +1,10 @@
 // The product kernels behind one entry point: which of them takes a problem is decided here, so that a launch costs the caller one
 // call (the decision and its queries took a scripting caller longer than the launch itself).
+#include "tmap.cuh"
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
+#include <mutex>
 
 extern "C" {
 
@@ -14,6 +17,8 @@ int blitz_gemm_decode(const void*, int64_t, const void*, int64_t, void*, int64_t
                       float, float, cudaStream_t);
 int blitz_gemm_pair(const void*, int64_t, const void*, int64_t, void*, int64_t, const void*, int, int, int, int, int, int, int, int, int, int,
                     void*, int64_t, unsigned*, int, int*, float, float, cudaStream_t);
+int blitz_gemm_decode_resident(int);
+int blitz_gemm_quad_resident();
 int blitz_gemm_quad_supported(int, int, int, int, int);
 int blitz_gemm_quad(const void*, int64_t, const void*, int64_t, void*, int64_t, const void*, int, int, int, int, int, int, int*, float, cudaStream_t);
 int blitz_gemm_wide(const void*, int64_t, const void*, int64_t, void*, int64_t, const void*, int, int, int, int, int, int, int, int*,
@@ -31,6 +36,42 @@ struct BlitzGemmScratch {
   int64_t num_pair_flags;
   int* status;
 };
+
+// What a device holds at once, as the kernels' own launches ask for it: SMs, clusters of 1 to 8 CTAs of the weight-streaming kernel, and
+// clusters of four of gemm_quad.cu.  Asked once per device; without one, the figures are those of a B200.
+struct GemmMachine {
+  int sms, streams[9], quads;
+};
+static const GemmMachine& machine() {
+  static constexpr GemmMachine kB200{148, {0, 148, 74, 45, 33, 26, 22, 15, 15}, 33};
+  static GemmMachine of[64];
+  static std::atomic<int> known[64];
+  static std::mutex mu;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    (void)cudaGetLastError();
+    return kB200;
+  }
+  if (!known[dev].load(std::memory_order_acquire)) {
+    std::lock_guard<std::mutex> g(mu);
+    if (!known[dev].load(std::memory_order_relaxed)) {
+      GemmMachine m = kB200;
+      m.sms = blitz::device_sm_count();
+      for (int i = 1; i <= 8; ++i)
+        if (const int n = blitz_gemm_decode_resident(i)) m.streams[i] = n;
+      if (const int n = blitz_gemm_quad_resident()) m.quads = n;
+      of[dev] = m;
+      known[dev].store(1, std::memory_order_release);
+    }
+  }
+  return of[dev];
+}
+
+// The same, one at a time: 0 SMs, 1 to 8 clusters of the weight-streaming kernel, 9 clusters of gemm_quad.cu.
+int blitz_gemm_resident(int what) {
+  const GemmMachine& m = machine();
+  return what == 0 ? m.sms : what >= 1 && what <= 8 ? m.streams[what] : what == 9 ? m.quads : -1;
+}
 
 // Whether more than 256 rows are better on pairs of CTAs with whole tiles of 256 x 256 (gemm_wide.cu; halves of them where a last round
 // of halves fits the 74 pairs) than on 148 CTAs with tiles of 128 x 256 or x 128 and K in parts (gemm_tcgen05.cu).  In a few rounds that
@@ -52,11 +93,12 @@ static bool pairs_are_better(int M, int N, int K, int epilogue, int groups) {
   auto tiles = [&](int rows, int columns) { return (int64_t)((M + rows - 1) / rows) * ((N + columns - 1) / columns) * groups; };
   const int64_t narrow = tiles(128, cols), pairs = tiles(256, 2 * cols);
   const bool odd = N < 2 * cols && N % 64 != 0;
-  if (narrow <= 74) return false;
-  if (narrow <= 148) return (2 * pairs <= 74 && (gated || epilogue == 1)) || odd;
-  if (tiles(128, 2 * cols) <= 148 && pairs > 74) return false;
-  if (N <= cols && narrow <= (2 * N <= cols ? 512 : 296)) return false;
-  if (f32 && !odd && K <= 2048 && pairs <= 74 && 2 * pairs > 74) return false;
+  const int sms = machine().sms, most = sms / 2;
+  if (narrow <= most) return false;
+  if (narrow <= sms) return (2 * pairs <= most && (gated || epilogue == 1)) || odd;
+  if (tiles(128, 2 * cols) <= sms && pairs > most) return false;
+  if (N <= cols && narrow <= (2 * N <= cols ? 512 : 2 * sms)) return false;
+  if (f32 && !odd && K <= 2048 && pairs <= most && 2 * pairs > most) return false;
   return true;
 }
 
@@ -66,7 +108,7 @@ static bool pairs_are_better(int M, int N, int K, int epilogue, int groups) {
 // 31.0 / 54.2 / 28.3;  1000 x 1024 of K = 2048 16.8 / 16.6 / 12.5;  3000 x 128 of K = 2048 17.3 / 15.4 / 12.6.  (Two rounds, 300 x 4096 of
 // K = 4096: 22.7 / 21.6 / 25.8.)
 static bool one_round_of_quads(int M, int N, int K, int epilogue) {
-  return (int64_t)((M + 255) / 256) * ((N + 127) / 128) <= 33 && blitz_gemm_quad_supported(M, N, K, 0, epilogue);
+  return (int64_t)((M + 255) / 256) * ((N + 127) / 128) <= machine().quads && blitz_gemm_quad_supported(M, N, K, 0, epilogue);
 }
 
 // 129 to 256 rows: the weight-streaming kernel (1), whole or half tiles of 256 x 256 on CTA pairs (3), those with K cut into parts (2), or
@@ -85,20 +127,21 @@ static bool one_round_of_quads(int M, int N, int K, int epilogue) {
 //   2816 x 2048 15.7 / 19.1 / 14.3, 17.5 / 19.3 / 14.5, 36.1 / 19.1 / 15.1
 // Over 40 shapes at 3 to 7 numbers of rows: within 1 % of the fastest on average; (2) for all of them: 28 % (without (4) among the others).
 int blitz_gemm_few_rows(int M, int N, int K, int epilogue) {
+  const GemmMachine& m = machine();
+  const int sms = m.sms, pairs = sms / 2;
   const int tiles = (N + 127) / 128, wide = (N + 255) / 256, kb = (K + 63) / 64;
-  if (epilogue == 2 || epilogue == 7) return M <= 192 && tiles > 74 ? 1 : 3;
+  if (epilogue == 2 || epilogue == 7) return M <= 192 && tiles > pairs ? 1 : 3;
   const bool quads = one_round_of_quads(M, N, K, epilogue);
-  if (!quads && M > 224 && K >= 8192 && 2 * wide <= 74 && (int64_t)N * K >= 48 << 20) return 2;
-  static const int clusters[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};  // of that many CTAs that 148 SMs hold
-  int parts = 148 / tiles < 8 ? 148 / tiles : 8;
+  if (!quads && M > 224 && K >= 8192 && 2 * wide <= pairs && (int64_t)N * K >= 48 << 20) return 2;
+  int parts = sms / tiles < 8 ? sms / tiles : 8;
   if (parts > kb) parts = kb;
-  while (parts > 1 && tiles > clusters[parts]) --parts;
+  while (parts > 1 && tiles > m.streams[parts]) --parts;
   if (parts < 1) parts = 1;
-  const bool all = parts > 1 && parts * tiles >= 120;  // (what nearly all SMs load together is less than what each can)
+  const bool all = parts > 1 && parts * tiles >= sms * 13 / 16;  // (what nearly all SMs load together is less than what each can)
   const float exchange = parts > 1 ? 0.027f * M + (all ? 2.f : 0.f) : epilogue == 1 ? 0.07f * M : 1.5f;  // (one part: a residual's loads are exposed)
-  const float streaming = ((kb + parts - 1) / parts) * ((tiles + 147) / 148) * (0.18f + 0.0011f * M) * (all ? 1.2f : 1.f) + exchange;
-  const int rest = wide % 74;
-  const float rounds = 2 * wide <= 74 ? 0.625f : wide / 74 + (rest == 0 ? 0.f : 2 * rest <= 74 ? 0.65f : 1.f);
+  const float streaming = ((kb + parts - 1) / parts) * ((tiles + sms - 1) / sms) * (0.18f + 0.0011f * M) * (all ? 1.2f : 1.f) + exchange;
+  const int rest = wide % pairs;
+  const float rounds = 2 * wide <= pairs ? 0.625f : wide / pairs + (rest == 0 ? 0.f : 2 * rest <= pairs ? 0.65f : 1.f);
   const float whole = 0.4f * kb * rounds + 1.5f;
   const float halves = quads ? 3.5f + ((kb + 1) / 2) * (0.13f + 0.0031f * tiles) : 1e30f;
   return halves < whole && halves < streaming ? 4 : streaming <= whole ? 1 : 3;

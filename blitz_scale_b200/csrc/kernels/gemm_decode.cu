@@ -577,6 +577,17 @@ int blitz_gemm_decode_supported(int M, int N, int K, int b_layout, int epilogue)
          ((epilogue >= 0 && epilogue <= 2) || (epilogue >= 4 && epilogue <= blitz::kEpiClampGlu)) && (N & 7) == 0 && (K & 7) == 0;
 }
 
+// How many clusters of `ctas` CTAs of this kernel the current device holds at once (0: no device to ask).
+int blitz_gemm_decode_resident(int ctas) {
+  using namespace blitz;
+  auto kern = gemm_decode_kernel<__nv_bfloat16, 0>;  // (threads and shared memory are the same for all of them)
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DecCfg::kSmemBytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return ctas == 1 ? device_sm_count() : max_active_clusters(kern, dim3(kDecThreads), DecCfg::kSmemBytes, (unsigned)ctas);
+}
+
 // C = X W (+R | silu-mul).  X [M, lda>=K], W [K, ldb>=columns] row-major, C/R [M, ldc>=N].  dtype 0 fp16, 1 bf16.
 // epilogue 0 store, 1 add R (C may be R), 2 silu(gate)*up with the up columns starting at up_col_off, 4 store with C in
 // fp32, 5 C += alpha * acc with C in fp32, 6 alpha * tanh(acc / alpha) with C in fp32, 7 clamped gated unit (gemm_gate.cuh; R:

@@ -1,5 +1,5 @@
-// Paired-SM tcgen05 GEMM with K in two halves over a cluster of four CTAs, for the few column tiles that 129 to 512 rows of a deep
-// product leave: one tile of 256 x 128 per cluster.
+// Paired-SM tcgen05 GEMM with K in two halves over a cluster of four CTAs, for products of more than 128 rows that are one round of its
+// tiles: one tile of 256 x 128 per cluster, at most as many as clusters are resident (the rule is in gemm_any.cu).
 //
 //   C[M,N] = A[M,K] * W[K,N]      W "in,out" (N contiguous), 16-bit, fp32 accumulation in TMEM
 //
@@ -322,6 +322,17 @@ extern "C" {
 int blitz_gemm_quad_supported(int M, int N, int K, int b_layout, int epilogue) {
   return M >= 1 && b_layout == 0 && (epilogue == 0 || epilogue == 1 || (epilogue >= 4 && epilogue <= 6)) && (N & 7) == 0 && (K & 7) == 0 && N >= 64 &&
          K > blitz::kQuadBK;
+}
+
+// How many of this kernel's clusters the current device holds at once (0: no device to ask).
+int blitz_gemm_quad_resident() {
+  using namespace blitz;
+  auto kern = gemm_quad_kernel<__nv_bfloat16, 0>;  // (threads and shared memory are the same for all of them)
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuadSmemBytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return max_active_clusters(kern, dim3(kQuadThreads), kQuadSmemBytes, 4u);
 }
 
 // C = A W with the epilogues and pitches of blitz_gemm.

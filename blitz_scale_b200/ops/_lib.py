@@ -67,6 +67,7 @@ def _declare(L: ctypes.CDLL) -> None:
     sig("blitz_gemm_choice", [c_i, c_i, c_i, c_i, c_i], c_i)
     sig("blitz_gemm_family", [c_i, c_i, c_i, c_i, c_i], c_i)
     sig("blitz_gemm_few_rows", [c_i, c_i, c_i, c_i], c_i)
+    sig("blitz_gemm_resident", [c_i], c_i)
     sig("blitz_gemm_wide", [c_p, c_i64, c_p, c_i64, c_p, c_i64, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_p, c_f, c_f, c_i, c_i, c_i, c_p])
     sig("blitz_gemm_wide_supported", [c_i, c_i, c_i, c_i, c_i, c_i], c_i)
     sig("blitz_gemm_quad", [c_p, c_i64, c_p, c_i64, c_p, c_i64, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_p, c_f, c_p])
