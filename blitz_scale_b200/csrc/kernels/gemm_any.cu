@@ -149,19 +149,20 @@ int blitz_gemm_few_rows(int M, int N, int K, int epilogue) {
 
 // The kernel that a call with hints starts from, before they are looked at: 0 the tiled one, 1 weight-streaming (128 rows at most), 2 CTA
 // pairs with K cut into parts (256 rows at most), 3 CTA pairs over whole tiles.
-int blitz_gemm_family(int M, int N, int K, int epilogue, int groups) {
+int blitz_gemm_choice(int M, int N, int K, int epilogue, int groups) {
   if (groups == 1 && M <= 128) return blitz_gemm_decode_supported(M, N, K, 0, epilogue) ? 1 : 0;
   if (groups == 1 && M <= 256) return blitz_gemm_pair_supported(M, N, K, 0, epilogue) ? 2 : 0;
   return M > 256 && pairs_are_better(M, N, K, epilogue, groups) && blitz_gemm_wide_supported(M, N, K, 0, epilogue, groups) ? 3 : 0;
 }
 
-// Which kernel takes a product with "in,out" weights that no hint sends elsewhere: those of blitz_gemm_family, or 4, K in halves over
-// clusters of four.  (What (2) takes the other kernels for few rows take too, and whole tiles take what (4) takes.)
-int blitz_gemm_choice(int M, int N, int K, int epilogue, int groups) {
-  const int family = blitz_gemm_family(M, N, K, epilogue, groups);
-  if (family == 2) return blitz_gemm_few_rows(M, N, K, epilogue);
+// Which kernel runs a product with "in,out" weights that carries no hint: that of blitz_gemm_choice beyond 256 rows and up to 128, the one
+// that blitz_gemm_few_rows names in between, or 4, K in halves over clusters of four, which fills a round that the others do not.  (What (2)
+// takes the other kernels for few rows take too, and whole tiles take what (4) takes.)
+int blitz_gemm_kernel(int M, int N, int K, int epilogue, int groups) {
+  const int choice = blitz_gemm_choice(M, N, K, epilogue, groups);
+  if (choice == 2) return blitz_gemm_few_rows(M, N, K, epilogue);
   if (groups == 1 && M > 256 && one_round_of_quads(M, N, K, epilogue)) return K > 512 ? 4 : 3;
-  return family;
+  return choice;
 }
 
 // Arguments as for blitz_gemm with "in,out" weights.
@@ -169,7 +170,7 @@ int blitz_gemm_any(const void* A, int64_t lda, const void* B, int64_t ldb, void*
                    int epilogue, int up_col_off, int dtype, int static_b, const BlitzGemmScratch* s, float alpha, float beta, int groups,
                    int a_step, int c_step, cudaStream_t stream) {
   if (!s) return -1;
-  switch (blitz_gemm_choice(M, N, K, epilogue, groups)) {
+  switch (blitz_gemm_kernel(M, N, K, epilogue, groups)) {
     case 4:
       return blitz_gemm_quad(A, lda, B, ldb, C, ldc, R, M, N, K, epilogue, dtype, static_b, s->status, alpha, stream);
     case 1:

@@ -280,7 +280,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
         _check(lib().blitz_gemm_quad(pa, lda, pb, ldb, pc, ldc, _p(extra), M, N, K, epi, _dt(a), int(static_b), _status_ptr(a), alpha, _stream()),
                "blitz_gemm_quad")
         return out
-    choice = lib().blitz_gemm_family(M, N, K, epi, groups) if layout == 0 and bn == 0 and split_k == 0 else 0
+    choice = lib().blitz_gemm_choice(M, N, K, epi, groups) if layout == 0 and bn == 0 and split_k == 0 else 0
     use_dec, use_pair, use_wide = choice == 1, choice == 2, choice == 3
     if decode_path is not None:
         assert not decode_path or lib().blitz_gemm_decode_supported(M, N, K, layout, epi)

@@ -64,8 +64,8 @@ def _declare(L: ctypes.CDLL) -> None:
     sig("blitz_gemm_pair_supported", [c_i, c_i, c_i, c_i, c_i], c_i)
     sig("blitz_gemm_pair_workspace_bytes", [c_i], c_i64)
     sig("blitz_gemm_any", [c_p, c_i64, c_p, c_i64, c_p, c_i64, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_p, c_f, c_f, c_i, c_i, c_i, c_p])
+    sig("blitz_gemm_kernel", [c_i, c_i, c_i, c_i, c_i], c_i)
     sig("blitz_gemm_choice", [c_i, c_i, c_i, c_i, c_i], c_i)
-    sig("blitz_gemm_family", [c_i, c_i, c_i, c_i, c_i], c_i)
     sig("blitz_gemm_few_rows", [c_i, c_i, c_i, c_i], c_i)
     sig("blitz_gemm_resident", [c_i], c_i)
     sig("blitz_gemm_wide", [c_p, c_i64, c_p, c_i64, c_p, c_i64, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_p, c_f, c_f, c_i, c_i, c_i, c_p])

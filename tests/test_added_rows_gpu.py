@@ -55,3 +55,21 @@ def test_copy_in_32_bits(shape, dt):
     part = x[:, :shape[1] - 1]                      # not contiguous: the general copy
     got = ops.to_fp32(part)
     assert got.dtype == torch.float32 and torch.equal(got.view(torch.int32), part.float().view(torch.int32))
+
+
+@pytest.mark.parametrize("T", [1, 61, 300])
+def test_rotation_with_positions_known_ahead(T):
+    from blitz_scale_b200 import ops
+    outs = []
+    for static in (False, True):
+        g = torch.Generator(device="cuda").manual_seed(T)
+        qkv = torch.randn(T, 12 * 64, generator=g, device="cuda").to(torch.bfloat16)
+        pos, slot = torch.arange(T, device="cuda", dtype=torch.int32) * 331, torch.arange(T, device="cuda", dtype=torch.int32)
+        slot[T // 2] = -1
+        kv = torch.zeros(T // 16 + 1, 2, 16, 2, 64, device="cuda", dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        ops.rope_kv_store(qkv, pos, slot, kv, q_heads=8, kv_heads=2, head_dim=64, page_size=16, rope_theta=5e5, static_meta=static)
+        outs.append((qkv, kv))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+    ops.check_status()
+

@@ -1,4 +1,4 @@
-"""What the rule for products takes a device to hold: asked of the device; the same choices as without one (tests/test_gemm_choice_cpu.py) where the answers are the same."""
+"""What the rule for products takes a device to hold: asked of the device; the same choices as without one (tests/test_gemm_kernel_cpu.py) where the answers are the same."""
 import pytest
 import torch
 
@@ -12,5 +12,5 @@ def test_resident():
     assert all(0 < got[i] * i <= got[0] for i in range(1, 9)) and 0 < 4 * got[9] <= got[0]
     print(got)
     if got == [148, 148, 74, 45, 33, 26, 22, 15, 15, 33]:       # (how many clusters fit depends on which SMs of a chip are in use)
-        from test_gemm_choice_cpu import CHOICE
-        assert all(ops.lib().blitz_gemm_choice(*shape) == want for shape, want in CHOICE)
+        from test_gemm_kernel_cpu import KERNEL
+        assert all(ops.lib().blitz_gemm_kernel(*shape) == want for shape, want in KERNEL)

@@ -72,9 +72,8 @@ def test_silu_of_large_negative_gates(M):
     assert bool(((got - want).abs() <= want.abs() * (2.0 ** -8 + 110 * 2.0 ** -23)).all())
 
 
-# at the lines of the rules that choose among this kernel, the tiled one and the one with K in halves (tests/test_gemm_choice_cpu.py), both sides
-@pytest.mark.parametrize("M,N,K,epi", [(300, 2048, 4096, "store"), (300, 2176, 4096, "add"), (300, 2048, 520, "add"), (300, 2048, 512, "axpy"),
-                                       (3000, 128, 2048, "store"), (8448, 72, 576, "axpy"), (8449, 72, 576, "store"), (384, 6144, 136, "store"), (385, 6144, 136, "store"), (1024, 2304, 72, "add"), (1152, 2304, 72, "add"),
+# at the lines of the rule that chooses between this kernel and the tiled one (tests/test_gemm_choice_cpu.py), both sides
+@pytest.mark.parametrize("M,N,K,epi", [(384, 6144, 136, "store"), (385, 6144, 136, "store"), (1024, 2304, 72, "add"), (1152, 2304, 72, "add"),
                                        (300, 9472, 64, "store"), (300, 9480, 64, "store"), (1300, 2048, 2048, "axpy"), (1300, 2048, 2056, "axpy")])
 def test_default_dispatch(M, N, K, epi):
     from blitz_scale_b200 import ops
@@ -84,10 +83,6 @@ def test_default_dispatch(M, N, K, epi):
     want = a.float() @ w.float() + (old.float() if epi != "store" else 0)
     out = ops.gemm(a, w, out=old.clone(), residual=old if epi == "add" else None, epilogue=epi)
     ops.check_status()
-    number = {"store": 0, "add": 1, "axpy": 5}[epi]
-    if ops.lib().blitz_gemm_choice(M, N, K, number, 1) == 4:          # (the kernel that the rule names has run)
-        same = ops.gemm(a, w, out=old.clone(), residual=old if epi == "add" else None, epilogue=epi, quad_path=True)
-        assert torch.equal(out, same)
     # one rounding of the result, and 32-bit sums in another order
     assert float(((out.float() - want).abs() - (1e-5 if epi == "axpy" else 2.0 ** -8) * want.abs()).max()) <= 2e-5 * K ** 0.5
 
