@@ -97,7 +97,6 @@ class LlamaRunner:
         cfg = seg.cfg
         self.cfg: ModelConfig = cfg
         self.seg, self.kv, self.comm = seg, kv_cache, comm
-        self._kv_layers = list(kv_cache.unbind(0))
         self.tp = seg.tp
         self.qh, self.kvh, self.hd = cfg.q_heads // self.tp, cfg.kv_heads // self.tp, cfg.head_dim
         self.inter = cfg.inter // self.tp
@@ -145,10 +144,14 @@ class LlamaRunner:
             ws = self._ws[key] = torch.zeros(n, dtype=torch.uint8, device=self.res.device)
         return ws
 
+    def _layer_cache(self, l: int, m: StepMeta) -> torch.Tensor:
+        """Pages of layer l in the cache that the runner has now."""
+        return m.view("kv layers", self.kv, list)[l]
+
     def attention_block(self, l: int, m: StepMeta) -> None:
         T, c = m.num_tokens, self.cfg
         res, normed, qkv, attn = (m.rows(n, t, T) for n, t in (("res", self.res), ("normed", self.normed), ("qkv", self.qkv), ("attn", self.attn)))
-        kv = self._kv_layers[l]
+        kv = self._layer_cache(l, m)
         ops.rms_norm(res, self._w(l, "input_ln"), c.rms_eps, out=normed)
         ops.gemm(normed, self._w(l, "qkv"), static_b=True, out=qkv)
         ops.rope_kv_store(qkv, m.rows("pos", m.pos, T), m.rows("slot", m.slot, T), kv, q_heads=self.qh, kv_heads=self.kvh,
@@ -171,7 +174,7 @@ class LlamaRunner:
         rows' own keys and values): earlier chunks of a long prompt are simply a longer page list.  Leading rows of one token
         (`m.singles`) are a decode batch: as tiles of 128 rows they would be padding (see singles_apart in runtime/engine.py for how
         many make it worth a kernel of their own)."""
-        T, ns, kv = m.num_tokens, m.singles, self._kv_layers[l]
+        T, ns, kv = m.num_tokens, m.singles, self._layer_cache(l, m)
         if ns:
             ops.attn_decode(m.rows("qkv", self.qkv, ns), kv, m.page_indices, m.rows("page_indptr", m.page_indptr, ns + 1),
                             m.rows("last_page_len", m.last_page_len, ns), q_heads=self.qh, kv_heads=self.kvh, head_dim=self.hd,

@@ -29,7 +29,7 @@ def test_the_runner_promises_what_the_step_does(monkeypatch, promised):
     r = LlamaRunner.__new__(LlamaRunner)
     r.cfg = types.SimpleNamespace(rms_eps=1e-5, rope_theta=1e4)
     r.res = r.normed = r.qkv = r.attn = torch.zeros(8, 4)
-    r._kv_layers, r.qh, r.kvh, r.hd, r.page_size, r.tp = [None], 1, 1, 4, 16, 1
+    r.kv, r.qh, r.kvh, r.hd, r.page_size, r.tp = [None], 1, 1, 4, 16, 1
     r._w = lambda l, n: None
     r._workspace = lambda *a: None
     r.attention_block(0, step(3, **(dict(static_positions=True) if promised else {})))
