@@ -95,6 +95,49 @@ def bench_gemm(shapes, out):
         print(json.dumps(row), flush=True)
 
 
+CHOICE_ROWS = {  # (columns, depth, epilogue): the products of the models' layers, and sizes between them
+    (4096, 4096, "add"), (6144, 4096, "store"), (4096, 14336, "add"), (14336, 4096, "silu_mul"), (128256, 4096, "store"), (2048, 2048, "add"),
+    (1024, 4096, "store"), (8192, 4096, "silu_mul"), (2816, 2048, "silu_mul"), (8192, 2048, "silu_mul"), (2048, 8192, "add"), (512, 512, "store"), (1536, 1024, "store"),
+    (3072, 2048, "store"), (4096, 1024, "store"), (4224, 2048, "store"), (5120, 8192, "add"), (6144, 8192, "add"), (8192, 8192, "add"),
+    (8192, 1024, "store"), (10240, 4096, "store"), (12288, 2048, "store"), (512, 4096, "axpy"), (2048, 14336, "axpy"), (1000, 3000, "axpy"), (3000, 1000, "add")}
+CHOICE_MORE = [(300, 2048, 256, "store"), (300, 2048, 576, "add"), (300, 2048, 4096, "store"), (300, 2048, 14336, "add"), (400, 2048, 2048, "axpy"), (512, 2048, 4096, "add"),
+               (640, 1280, 1024, "store"), (1000, 1024, 2048, "store"), (1024, 1024, 8192, "add"), (1574, 512, 4096, "store"), (3000, 128, 2048, "store"),
+               (4096, 256, 2048, "axpy"), (8192, 128, 1024, "store"), (2000, 512, 640, "add")]
+
+
+def bench_choice(out):
+    """The kernels that a product of 129 to 256 rows, or one round of clusters of more, can go to, beside the one that it goes to; each
+    behind the norm that writes its activations, with weights that are not in L2."""
+    names = {0: "tiles", 1: "stream", 2: "pairs", 3: "wide", 4: "quads"}
+    lib, number = ops.lib(), {"store": 0, "add": 1, "silu_mul": 2, "axpy": 5}
+    cases = [(M, N, K, e) for N, K, e in sorted(CHOICE_ROWS) for M in (136, 192, 224, 256)] + CHOICE_MORE
+    for (M, N, K, epi) in cases:
+        e = number[epi]
+        x, w, a = (torch.randn(*s, device="cuda").bfloat16() for s in ((M, K), (K,), (M, K)))
+        bcols = 2 * N if epi == "silu_mul" else N
+        nc = n_copies(K * bcols * 2)
+        bs = [torch.randn(K, bcols, device="cuda", dtype=torch.bfloat16) * K ** -0.5 for _ in range(min(nc, 200))]
+        old = torch.randn(M, N, device="cuda").to(torch.float32 if epi == "axpy" else torch.bfloat16)
+        kw = dict(out=torch.zeros_like(old), residual=old if epi == "add" else None, epilogue=epi, static_b=True)
+        can = {1: M <= 256 and lib.blitz_gemm_decode_supported(M, N, K, 0, e), 2: M <= 256 and lib.blitz_gemm_pair_supported(M, N, K, 0, e),
+               3: lib.blitz_gemm_wide_supported(M, N, K, 0, e, 1), 4: lib.blitz_gemm_quad_supported(M, N, K, 0, e), 0: M > 256}
+        hint = {0: dict(decode_path=False, pair_path=False, wide_path=False), 1: dict(decode_path=True), 2: dict(pair_path=True), 3: dict(wide_path=True),
+                4: dict(quad_path=True)}
+
+        def both(i, **h):
+            ops.rms_norm(x, w, out=a)
+            ops.gemm(a, bs[i], **kw, **h)
+        us = {k: timeit(lambda i: both(i, **hint[k]), copies=len(bs)) * 1e6 for k in sorted(hint) if can[k]}
+        ops.check_status()
+        runs, least = lib.blitz_gemm_kernel(M, N, K, e, 1), min(us, key=us.get)
+        row = dict(kind="choice", M=M, N=N, K=K, epilogue=epi, us={names[k]: round(t, 2) for k, t in us.items()}, runs=names[runs], least=names[least],
+                   over_least=round(us[runs] / us[least], 3))
+        out.append(row)
+        print(json.dumps(row), flush=True)
+    over = sorted(r["over_least"] for r in out if r["kind"] == "choice")
+    print(f"{len(over)} products: {sum(over) / len(over):.3f} of the least time on average, {over[-1]:.3f} at worst")
+
+
 def bench_decode_attn(cases, out):
     hbm, _, src = peaks()
     for (B, ctx, qh, kvh, hd, page, splits) in cases:
@@ -146,7 +189,7 @@ def bench_prefill_attn(cases, out):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--quick", action="store_true")
-    ap.add_argument("--only", default="", help="run only one group: gemm, decode_attn, prefill_attn")
+    ap.add_argument("--only", default="", help="run only one group: gemm, choice, decode_attn, prefill_attn")
     ap.add_argument("--json", default="")
     args = ap.parse_args()
     out = []
@@ -161,6 +204,8 @@ def main():
         bench_gemm(shapes, out)
     cases = [(64, 1024, 32, 8, 128, 64, 1), (256, 1024, 32, 8, 128, 64, 1), (256, 1024, 32, 8, 128, 16, 1),
              (8, 8192, 32, 8, 128, 64, 8), (1, 16384, 32, 8, 128, 64, 32)]
+    if args.only in ("", "choice"):
+        bench_choice(out)
     if args.only in ("", "decode_attn"):
         bench_decode_attn(cases[:2] if args.quick else cases, out)
     if args.only in ("", "prefill_attn"):

@@ -111,6 +111,27 @@ static bool one_round_of_quads(int M, int N, int K, int epilogue) {
   return (int64_t)((M + 255) / 256) * ((N + 127) / 128) <= machine().quads && blitz_gemm_quad_supported(M, N, K, 0, epilogue);
 }
 
+// Of those 129 to 256 rows, the products that are too wide for one round of quads, leave half of the pairs idle in whole tiles, and are deep:
+// K cut into parts on CTA pairs (2) pays the exchange of sums through L2, 8 us more than the others, from K = 4608 on, and the more the
+// more rows the weight-streaming kernel (1) reads again with every tile.  Each costs a time per K block that grows with the CTAs that
+// load at once, and half tiles (3) that of the whole K.  Clusters of an odd number of CTAs do not fill the SMs beside a predecessor's last
+// blocks: with nearly as many of them as are resident the last ones start late.  Measured behind a norm with cold weights, us, 1 / 2 / 3:
+//   6144 x 8192 with a residual, 136, 192 and 224 rows 33.0 / 34.9 / 39.0, 38.9 / 35.3 / 38.8, 41.6 / 35.7 / 39.4
+//   6144 x 14336 48.1 / 48.1 / 60.8 at 160 rows, 52.1 / 48.6 / 61.8 at 224;  8192 x 14336 54.1 / 58.6 / 63.9 at 192, 63.9 / 59.4 / 64.7 at 256
+//   5632 x 14336 (44 clusters of three) 46.9 / 46.9 / 60.4 at 136 rows, with a residual 61.4 / 48.4 / 62.4 at 208, 81.8 / 49.5 / 63.2 at 256
+// Over 1320 products of 4232 to 9472 columns, K = 5120 to 20480, 130 to 256 rows: 1.003 of the fastest on average, 1.17 at worst (those clusters at 136 rows).
+static int deep_few_rows(int M, int tiles, int wide, int kb, bool add, const GemmMachine& m) {
+  int p = m.sms / tiles < 8 ? m.sms / tiles : 8;
+  while (p > 1 && tiles > m.streams[p]) --p;
+  if (p < 1) p = 1;
+  const int q = m.sms / 2 / wide;
+  float streaming = 0.032f * M + (kb + p - 1) / p * (0.035f + 0.0009f * M + 0.0017f * p * tiles) + (add ? 0.05f * M / p : 0.f);
+  if (p > 1 && (p & 1) && 16 * tiles > 15 * m.streams[p]) streaming *= 1.3f;
+  const float parts = 10.4f + (kb + q - 1) / q * (0.167f + 0.0027f * q * wide + 0.042f * q);
+  const float halves = 2.7f + kb * (0.186f + 0.0022f * wide + 0.0001f * M);
+  return parts < halves && parts < streaming ? 2 : streaming <= halves ? 1 : 3;
+}
+
 // 129 to 256 rows: the weight-streaming kernel (1), whole or half tiles of 256 x 256 on CTA pairs (3), those with K cut into parts (2), or
 // K in halves over clusters of four (4).  The first is as fast as its loads, 128 bytes per row and column of a K block and CTA, with as many parts of
 // K as clusters fit, and adds an exchange of the parts' sums; the third takes a quarter of a microsecond per K block of a round of half tiles, 0.4 of
@@ -125,14 +146,14 @@ static bool one_round_of_quads(int M, int N, int K, int epilogue) {
 // Gated units need both accumulators' weights at once: fewer stages, and beyond 192 rows room for fewer parts.  144, 192 and 256 rows:
 //   14336 x 4096 49.3 / 57.0 / 56.6, 54.3 / 57.5 / 57.7, 66.7 / 58.3 / 58.2;  8192 x 4096 36.0 / 35.9 / 34.8, 38.3 / 36.7 / 35.5, 62.1 / 37.4 / 36.2
 //   2816 x 2048 15.7 / 19.1 / 14.3, 17.5 / 19.3 / 14.5, 36.1 / 19.1 / 15.1
-// Over 40 shapes at 3 to 7 numbers of rows: within 1 % of the fastest on average; (2) for all of them: 28 % (without (4) among the others).
+// (bench/kernels_bench.py --only choice times all of them at 104 such products and sums up: 1.01 of the fastest on average.)
 int blitz_gemm_few_rows(int M, int N, int K, int epilogue) {
   const GemmMachine& m = machine();
   const int sms = m.sms, pairs = sms / 2;
   const int tiles = (N + 127) / 128, wide = (N + 255) / 256, kb = (K + 63) / 64;
   if (epilogue == 2 || epilogue == 7) return M <= 192 && tiles > pairs ? 1 : 3;
   const bool quads = one_round_of_quads(M, N, K, epilogue);
-  if (!quads && M > 224 && K >= 8192 && 2 * wide <= pairs && (int64_t)N * K >= 48 << 20) return 2;
+  if (!quads && 2 * wide <= pairs && kb > 71) return deep_few_rows(M, tiles, wide, kb, epilogue == 1, m);
   int parts = sms / tiles < 8 ? sms / tiles : 8;
   if (parts > kb) parts = kb;
   while (parts > 1 && tiles > m.streams[parts]) --parts;
