@@ -14,6 +14,7 @@
 #include "launch.cuh"
 #include "ptx.cuh"
 #include "scalar.cuh"
+#include "tmap.cuh"
 
 namespace blitz {
 
@@ -34,12 +35,14 @@ struct RopeStoreParams {
   int* status;
 };
 
-// (Wide accesses without a norm: 40 registers, six blocks an SM; a token's chain of loads, sines and stores is waited for by more of them.
-// 4096 tokens of 16 + 4 heads of 128, 64 dimensions rotated: 24.0 us with four, 20.2 so.)
+// Bound by a token's chain of loads, sines and stores, which other blocks of the SM hide.  Wide accesses without a norm come in two
+// builds: four blocks an SM of 56 to 64 registers, or six of 40, whose chain is longer.  Six pay when there are more tokens than four blocks
+// on every SM take at once.  Four / six, us, 32 + 8 heads of 128 in pairs: 16 tokens 2.50 / 2.61, 256 4.51 / 5.57, 600 7.1 / 6.3, 1000 8.4 / 8.4, 4096 26.4 / 22.9,
+// 8192 54.0 / 45.2;  16 + 4 heads of 128, halves, 64 dimensions rotated: 2.66 / 2.92, 3.59 / 4.93, 6.2 / 5.7, 7.2 / 7.5, 22.8 / 19.7, 43.2 / 36.3.
 enum RopeMode : int { kRopeAny = 0, kRopeWidePairs = 1, kRopeWideHalves = 2 };  // wide: eight elements per access
 
-template <typename T, int MODE, bool NORM>
-__global__ void __launch_bounds__(NORM && MODE == kRopeWideHalves ? 1024 : 256, NORM && MODE == kRopeWideHalves ? 1 : MODE == kRopeAny ? 5 : NORM ? 4 : 6) rope_store_kernel(const RopeStoreParams p) {
+template <typename T, int MODE, bool NORM, int BLOCKS = MODE == kRopeAny ? 5 : 4>
+__global__ void __launch_bounds__(NORM && MODE == kRopeWideHalves ? 1024 : 256, NORM && MODE == kRopeWideHalves ? 1 : BLOCKS) rope_store_kernel(const RopeStoreParams p) {
   ptx::griddep_launch_dependents();
   ptx::griddep_wait();
   extern __shared__ float s_ang[];  // [rot_dims / 2] cos, [rot_dims / 2] sin
@@ -344,6 +347,11 @@ int blitz_rope_store(void* q, const void* k, const void* v, const void* q_b, con
     using T = decltype(type);
     constexpr bool N = decltype(norm)::value;
     if (!wide) return launch_pdl(rope_store_kernel<T, kRopeAny, N>, grid, block, smem, stream, p);
+    if constexpr (!N) {
+      if ((int64_t)num_tokens * block.x > 1024 * (int64_t)device_sm_count())
+        return interleaved ? launch_pdl(rope_store_kernel<T, kRopeWidePairs, N, 6>, grid, block, smem, stream, p)
+                           : launch_pdl(rope_store_kernel<T, kRopeWideHalves, N, 6>, grid, block, smem, stream, p);
+    }
     return interleaved ? launch_pdl(rope_store_kernel<T, kRopeWidePairs, N>, grid, block, smem, stream, p)
                        : launch_pdl(rope_store_kernel<T, kRopeWideHalves, N>, grid, block, smem, stream, p);
   };
