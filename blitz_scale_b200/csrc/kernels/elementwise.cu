@@ -56,8 +56,8 @@ __device__ __forceinline__ uint4 scaled8(const uint4& v, const uint4& w, float s
 // 8192 rows.  (A warp per row without any barrier takes 28.6 us for those by itself, but a prompt's pass of 8192 tokens took the same
 // 95.7 ms with either.)
 template <typename T>
-__global__ void rms_norm_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ out, int hidden, float eps) {
-  ptx::griddep_launch_dependents();
+__global__ void rms_norm_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ out, int hidden, float eps, bool early) {
+  if (early) ptx::griddep_launch_dependents();
   ptx::griddep_wait();
   __shared__ float red[32];
   const int64_t base = static_cast<int64_t>(blockIdx.x) * hidden;
@@ -92,8 +92,8 @@ __global__ void rms_norm_kernel(const T* __restrict__ x, const T* __restrict__ w
 // of 4096 columns 2.05 / 2.45, of 8192 2.7 / 3.1; 256 rows of 4096 3.1 / 3.6, of 12288 6.7 / 5.4; 8192 rows of 8192 123 / 100.
 template <typename T, bool KEEP>
 __global__ void add_rms_norm_kernel(const T* __restrict__ x, T* __restrict__ residual, const T* __restrict__ w, T* __restrict__ out,
-                                    int hidden, float eps) {
-  ptx::griddep_launch_dependents();
+                                    int hidden, float eps, bool early) {
+  if (early) ptx::griddep_launch_dependents();
   ptx::griddep_wait();
   __shared__ float red[32];
   const int64_t base = static_cast<int64_t>(blockIdx.x) * hidden;
@@ -451,6 +451,11 @@ static inline int pick_threads(int nvec) {
   return t;
 }
 
+// Whether a norm lets its successor start ahead of its end.  Blocks of 1024 threads beyond the two that each SM holds do not: a chain of
+// 513 of them and a product on CTA pairs did not end in a replay of its graph, which fits blocks of a later norm that hold the SMs while
+// blocks of an earlier one still have to start.  (Narrower blocks, and as many as fit, never did that.)
+static inline bool norm_starts_successor(int num_tokens, int threads) { return threads < 1024 || num_tokens <= 2 * device_sm_count(); }
+
 }  // namespace blitz
 
 extern "C" {
@@ -472,8 +477,9 @@ int blitz_rms_norm(const void* x, const void* w, void* out, int num_tokens, int 
   if (num_tokens <= 0) return 0;
   if (hidden & 7) return -1;
   cudaError_t blitz_last = cudaSuccess;
-  BLITZ_DISPATCH_DTYPE(dtype, (blitz_last = launch_pdl(rms_norm_kernel<T>, dim3(num_tokens), dim3(pick_threads(hidden >> 3)), 0, stream,
-                                  (const T*)x, (const T*)w, (T*)out, hidden, eps)));
+  const int threads = pick_threads(hidden >> 3);
+  BLITZ_DISPATCH_DTYPE(dtype, (blitz_last = launch_pdl(rms_norm_kernel<T>, dim3(num_tokens), dim3(threads), 0, stream,
+                                  (const T*)x, (const T*)w, (T*)out, hidden, eps, norm_starts_successor(num_tokens, threads))));
   return (int)blitz_last;
 }
 
@@ -486,7 +492,7 @@ int blitz_add_rms_norm(const void* x, void* residual, const void* w, void* out, 
   const int threads = pick_threads(hidden >> 3);
   const bool keep = threads < 1024 || num_tokens <= device_sm_count();
   BLITZ_DISPATCH_DTYPE(dtype, (blitz_last = launch_pdl(keep ? add_rms_norm_kernel<T, true> : add_rms_norm_kernel<T, false>, dim3(num_tokens), dim3(threads), 0,
-                                  stream, (const T*)x, (T*)residual, (const T*)w, (T*)out, hidden, eps)));
+                                  stream, (const T*)x, (T*)residual, (const T*)w, (T*)out, hidden, eps, norm_starts_successor(num_tokens, threads))));
   return (int)blitz_last;
 }
 
