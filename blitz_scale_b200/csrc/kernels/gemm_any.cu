@@ -146,7 +146,7 @@ static int deep_few_rows(int M, int tiles, int wide, int kb, bool add, const Gem
 // Gated units need both accumulators' weights at once: fewer stages, and beyond 192 rows room for fewer parts.  144, 192 and 256 rows:
 //   14336 x 4096 49.3 / 57.0 / 56.6, 54.3 / 57.5 / 57.7, 66.7 / 58.3 / 58.2;  8192 x 4096 36.0 / 35.9 / 34.8, 38.3 / 36.7 / 35.5, 62.1 / 37.4 / 36.2
 //   2816 x 2048 15.7 / 19.1 / 14.3, 17.5 / 19.3 / 14.5, 36.1 / 19.1 / 15.1
-// (bench/kernels_bench.py --only choice times all of them at 104 such products and sums up: 1.01 of the fastest on average.)
+// (bench/kernels_bench.py --only choice times all of them at 104 such products: 1.01 of the fastest on average, 1.20 at worst.)
 int blitz_gemm_few_rows(int M, int N, int K, int epilogue) {
   const GemmMachine& m = machine();
   const int sms = m.sms, pairs = sms / 2;

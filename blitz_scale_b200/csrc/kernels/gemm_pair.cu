@@ -15,7 +15,7 @@
 // are counted on the even CTA's barrier, whose elected thread issues the instructions for the pair.
 //
 // Of the products that name no kernel, the rule in gemm_any.cu sends here only those of more than 224 rows that are deep and too wide for K in
-// halves (256 rows x 6144 columns of K = 8192, us: 40.5 weight-streaming, 35.7 here, 39.3 on whole tiles); others ask for parts or tiles.
+// halves (256 rows x 6144 columns of K = 8192, us: 40.5 weight-streaming, 35.7 here, 39.3 on whole tiles); others ask for parts or tiles.  Gated units come here only from callers that ask for this kernel.
 //
 // Scheduling.  Work is cut into units of (super tile, 64-wide K block); pair p takes the units
 // [p*upp, (p+1)*upp) in order, so all pairs finish together whatever the tile count (stream-K).  A pair whose
@@ -32,8 +32,7 @@
 // 128-byte-swizzled 32 x 64 boxes to a staging area and hand them to TMA stores: a thread-per-row epilogue would
 // issue one 16-byte store per lane into 32 different rows, which the load/store unit serialises.  Residual values
 // are requested before the wait for the accumulator.  The slabs of a tile are a rolled loop: the code runs once or twice a launch, behind
-// weights that have displaced it from every cache (unrolled / rolled, from the last accumulator to the end, us, 256 rows x 6144 and
-// 4096 x 4096, 4096 x 14336: 11.3 / 9.5, 12.3 / 10.5, 11.3 / 10; the products of a layer of Llama-3-8B with their norms 146 / 138).
+// weights that have displaced it from every cache (from the last accumulator to the end 9.5 to 10.5 us at 256 rows, unrolled 11.3 to 12.3).
 // Replaces cuBLAS at these sizes (src/util/cublas_wrapper.h:31-141 of the reference; call sites
 // src/layer/attn.h:137-215, src/layer/glu.h:109-136, src/layer/lm_head.h:89-98).
 //
