@@ -49,8 +49,9 @@ struct GlaParams {
   int* status;
 };
 
-// VEC: value columns a thread handles at once.
-template <typename T, int VEC, bool WKV>
+// VEC: value columns a thread handles at once.  KEEP: the state stays in shared memory over a row's tokens, and nothing is requested ahead:
+// the registers for that would halve the blocks on an SM (32 rows of 5 tokens, 32 heads of 128 x 64: 59 us, with them 87).
+template <typename T, int VEC, bool WKV, bool KEEP>
 __global__ void __launch_bounds__(kGlaThreads) gla_recurrent_kernel(const GlaParams p) {
   ptx::griddep_launch_dependents();
   ptx::griddep_wait();
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(kGlaThreads) gla_recurrent_kernel(const GlaPar
   if (t_end <= t_beg) return;
   float* gstate = p.state + (static_cast<int64_t>(slot) * p.heads + h) * K * V;
   bool fresh = p.pos[t_beg] == 0;
-  const bool keep = p.in_shared != 0;
+  constexpr bool keep = KEEP;
   if (keep) {
     for (int i = tid; i < K * V; i += kGlaThreads) s_state[i] = fresh ? 0.f : gstate[i];
     fresh = false;
@@ -92,10 +93,10 @@ __global__ void __launch_bounds__(kGlaThreads) gla_recurrent_kernel(const GlaPar
   const T* bonus = reinterpret_cast<const T*>(p.bonus) + h * K;
   // Rows of the state a thread has in flight: those of the first batch are requested before the decays are computed, a batch's
   // successor before it is worked on.  (48 rows of 8 heads of 128 x 256: 30 us with loads as they come, 23.6 so.)
-  constexpr int kBatch = VEC == 4 ? 8 : 1;
+  constexpr int kBatch = VEC == 4 && !KEEP ? 8 : 1;
   float4 ahead[kBatch];
   auto request = [&](int c0, int first, float4 (&to)[kBatch]) {
-    if (VEC != 4) return;
+    if (VEC != 4 || KEEP) return;
 #pragma unroll
     for (int i = 0; i < kBatch; ++i) {
       const int c = first + i * parts;
@@ -131,27 +132,34 @@ __global__ void __launch_bounds__(kGlaThreads) gla_recurrent_kernel(const GlaPar
       if (part < parts && c0 + col < nv) {
         if (VEC == 4) {
           const float4 vv = ldf4<T>(v + vg);
-          if (keep || c0 > 0) request(c0, part, ahead);
+          auto step = [&](int c, float4 s) {
+            const float a = s_alpha[c], kk = s_k[c], qq = s_q[c];
+            if (WKV) {
+              const float b = s_bonus[c];
+              o.x += qq * (s.x + b * vv.x); o.y += qq * (s.y + b * vv.y); o.z += qq * (s.z + b * vv.z); o.w += qq * (s.w + b * vv.w);
+            }
+            s.x = a * s.x + kk * vv.x; s.y = a * s.y + kk * vv.y; s.z = a * s.z + kk * vv.z; s.w = a * s.w + kk * vv.w;
+            *reinterpret_cast<float4*>(S + static_cast<int64_t>(c) * V + vg) = s;
+            if (!WKV) {
+              o.x += qq * s.x; o.y += qq * s.y; o.z += qq * s.z; o.w += qq * s.w;
+            }
+          };
+          if constexpr (KEEP) {
+#pragma unroll 4
+            for (int c = part; c < K; c += parts) step(c, *reinterpret_cast<const float4*>(S + static_cast<int64_t>(c) * V + vg));
+          } else {
+            if (c0 > 0) request(c0, part, ahead);
 #pragma unroll 1
-          for (int first = part; first < K; first += kBatch * parts) {
-            float4 here[kBatch];
+            for (int first = part; first < K; first += kBatch * parts) {
+              float4 here[kBatch];
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) here[i] = ahead[i];
-            if (first + kBatch * parts < K) request(c0, first + kBatch * parts, ahead);
+              for (int i = 0; i < kBatch; ++i) here[i] = ahead[i];
+              if (first + kBatch * parts < K) request(c0, first + kBatch * parts, ahead);
 #pragma unroll
-            for (int i = 0; i < kBatch; ++i) {
-              const int c = first + i * parts;
-              if (c >= K) break;
-              float4 s = here[i];
-              const float a = s_alpha[c], kk = s_k[c], qq = s_q[c];
-              if (WKV) {
-                const float b = s_bonus[c];
-                o.x += qq * (s.x + b * vv.x); o.y += qq * (s.y + b * vv.y); o.z += qq * (s.z + b * vv.z); o.w += qq * (s.w + b * vv.w);
-              }
-              s.x = a * s.x + kk * vv.x; s.y = a * s.y + kk * vv.y; s.z = a * s.z + kk * vv.z; s.w = a * s.w + kk * vv.w;
-              *reinterpret_cast<float4*>(S + static_cast<int64_t>(c) * V + vg) = s;
-              if (!WKV) {
-                o.x += qq * s.x; o.y += qq * s.y; o.z += qq * s.z; o.w += qq * s.w;
+              for (int i = 0; i < kBatch; ++i) {
+                const int c = first + i * parts;
+                if (c >= K) break;
+                step(c, here[i]);
               }
             }
           }
@@ -203,11 +211,12 @@ static cudaError_t launch_gla_recurrent(GlaParams p, bool multi, cudaStream_t st
   p.in_shared = multi && whole <= kLimit;
   const size_t smem = p.in_shared ? whole : base + park;
   if (smem > kLimit) return cudaErrorInvalidValue;
-  auto kern = gla_recurrent_kernel<T, VEC, WKV>;
-  static PerDeviceOnce once;
-  cudaError_t e = once.run([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit); });
-  if (e != cudaSuccess) return e;
-  return launch_pdl(kern, dim3(p.rows, p.heads), dim3(kGlaThreads), smem, stream, p);
+  auto go = [&](auto kern, PerDeviceOnce& once) {
+    const cudaError_t e = once.run([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit); });
+    return e != cudaSuccess ? e : launch_pdl(kern, dim3(p.rows, p.heads), dim3(kGlaThreads), smem, stream, p);
+  };
+  static PerDeviceOnce kept, streamed;
+  return p.in_shared ? go(gla_recurrent_kernel<T, VEC, WKV, true>, kept) : go(gla_recurrent_kernel<T, VEC, WKV, false>, streamed);
 }
 
 template <bool WKV>
