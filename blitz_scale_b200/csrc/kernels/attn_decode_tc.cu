@@ -606,8 +606,9 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
 
 // Combine split partials: out = sum_s w_s o_s / (sum_s w_s + e^sink), w_s = 2^(lse_s - max lse).  A lane looks after the weight of
 // every 32nd split, so that the loads of the partials do not wait for one another's weights (16 splits: 6.8 us behind the attention
-// with a serial loop, 3.6 us so), and the first eight splits' partials are on their way while the weights are (8 splits: 4.2 -> 2.6 us).
-template <typename T>
+// with a serial loop, 3.6 us so).  EARLY, at most eight splits: their partials are on their way while the weights are (8 splits: 4.2 -> 2.6 us;
+// with more the values held back lengthen the loop, 16 splits of one row of 32 heads: 1 us, 40: 4 us).
+template <typename T, bool EARLY>
 __global__ void attn_merge_tc_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
                                      T* __restrict__ out, int64_t out_stride, int q_heads, int hd, int num_splits,
                                      const T* __restrict__ sink, const T* __restrict__ gate, int64_t gate_stride, int sum_only) {
@@ -617,37 +618,41 @@ __global__ void attn_merge_tc_kernel(const float* __restrict__ part_o, const flo
   const int64_t base = (static_cast<int64_t>(b) * q_heads + head) * num_splits;
   const float snk = sink ? to_f<T>(sink[head]) * 1.4426950408889634f : -INFINITY;
   const int d = threadIdx.x;  // (a block has a thread per column)
-  // the partials of the first splits are requested together with the weights
   constexpr int kEarly = 8;
-  float early[kEarly];
+  float early[kEarly], first = -INFINITY;
+  float M = snk;
+  if constexpr (EARLY) {
 #pragma unroll
-  for (int i = 0; i < kEarly; ++i) early[i] = i < num_splits && d < hd ? part_o[(base + i) * hd + d] : 0.f;
-  const float first = lane < num_splits ? part_lse[base + lane] : -INFINITY;
-  float M = fmaxf(snk, first);
-  for (int s = lane + 32; s < num_splits; s += 32) M = fmaxf(M, part_lse[base + s]);
+    for (int i = 0; i < kEarly; ++i) early[i] = i < num_splits && d < hd ? part_o[(base + i) * hd + d] : 0.f;
+    if (lane < num_splits) first = part_lse[base + lane];
+    M = fmaxf(M, first);
+  } else {
+    for (int s = lane; s < num_splits; s += 32) M = fmaxf(M, part_lse[base + s]);
+  }
 #pragma unroll
   for (int d = 16; d; d >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, d));
   const float g = gate ? head_gate(gate + b * gate_stride + head) : 1.f;
   float acc = 0.f, wsum = 0.f;
   if (M > -INFINITY) {
-    for (int s0 = 0; s0 < num_splits; s0 += 32) {
-      const float mine = s0 + lane < num_splits ? exp2f((s0 == 0 ? first : part_lse[base + s0 + lane]) - M) : 0.f;
-      const int here = min(32, num_splits - s0);
-      int i = 0;
-      if (s0 == 0) {
+    if constexpr (EARLY) {
+      const float mine = lane < num_splits ? exp2f(first - M) : 0.f;
 #pragma unroll
-        for (; i < kEarly; ++i) {
-          if (i >= here) break;
-          const float w = __shfl_sync(0xffffffffu, mine, i);
-          wsum += w;
-          if (d < hd) acc += w * early[i];
-        }
-      }
-#pragma unroll 8
-      for (; i < here; ++i) {
+      for (int i = 0; i < kEarly; ++i) {
+        if (i >= num_splits) break;
         const float w = __shfl_sync(0xffffffffu, mine, i);
         wsum += w;
-        if (d < hd) acc += w * part_o[(base + s0 + i) * hd + d];
+        if (d < hd) acc += w * early[i];
+      }
+    } else {
+      for (int s0 = 0; s0 < num_splits; s0 += 32) {
+        const float mine = s0 + lane < num_splits ? exp2f(part_lse[base + s0 + lane] - M) : 0.f;
+        const int here = min(32, num_splits - s0);
+#pragma unroll 8
+        for (int i = 0; i < here; ++i) {
+          const float w = __shfl_sync(0xffffffffu, mine, i);
+          wsum += w;
+          if (d < hd) acc += w * part_o[(base + s0 + i) * hd + d];
+        }
       }
     }
     if (sink) wsum += exp2f(snk - M);
@@ -751,7 +756,7 @@ int blitz_attn_decode(const void* q, int64_t q_stride, const void* k_pool, const
   if (num_splits > 1) {
     auto merge = [&](auto type) {
       using T = decltype(type);
-      return (int)launch_pdl(attn_merge_tc_kernel<T>, dim3(batch, q_heads), dim3(vdim > 64 ? 128 : 64), 0, stream, p.part_o, p.part_lse,
+      return (int)launch_pdl(p.num_splits <= 8 ? attn_merge_tc_kernel<T, true> : attn_merge_tc_kernel<T, false>, dim3(batch, q_heads), dim3(vdim > 64 ? 128 : 64), 0, stream, p.part_o, p.part_lse,
                              (T*)out, out_stride, q_heads, vdim, num_splits, (const T*)sink, (const T*)gate, gate_stride, sigmoid);
     };
     rc = dtype == 1 ? merge(__nv_bfloat16{}) : merge(__half{});
@@ -870,10 +875,10 @@ extern "C" int blitz_attn_decode_noalloc(const void* q, int64_t q_stride, const 
   if (rc != 0 || num_splits == 1) return rc;
   dim3 grid(batch, q_heads);
   if (dtype == 1)
-    attn_merge_tc_kernel<__nv_bfloat16><<<grid, head_dim, 0, stream>>>(p.part_o, p.part_lse, (__nv_bfloat16*)out, out_stride,
+    attn_merge_tc_kernel<__nv_bfloat16, false><<<grid, head_dim, 0, stream>>>(p.part_o, p.part_lse, (__nv_bfloat16*)out, out_stride,
                                                                        q_heads, head_dim, num_splits, nullptr, nullptr, 0, 0);
   else
-    attn_merge_tc_kernel<__half><<<grid, head_dim, 0, stream>>>(p.part_o, p.part_lse, (__half*)out, out_stride, q_heads,
+    attn_merge_tc_kernel<__half, false><<<grid, head_dim, 0, stream>>>(p.part_o, p.part_lse, (__half*)out, out_stride, q_heads,
                                                                 head_dim, num_splits, nullptr, nullptr, 0, 0);
   return (int)cudaGetLastError();
 }
