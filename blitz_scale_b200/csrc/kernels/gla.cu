@@ -50,7 +50,7 @@ struct GlaParams {
 };
 
 // VEC: value columns a thread handles at once.  KEEP: the state stays in shared memory over a row's tokens, and nothing is requested ahead:
-// the registers for that would halve the blocks on an SM (32 rows of 5 tokens, 32 heads of 128 x 64: 59 us, with them 87).
+// the registers for that would halve the blocks on an SM (32 rows of 5 tokens, 32 heads of 128 x 64: 56 us, with them 87).
 template <typename T, int VEC, bool WKV, bool KEEP>
 __global__ void __launch_bounds__(kGlaThreads) gla_recurrent_kernel(const GlaParams p) {
   ptx::griddep_launch_dependents();
